@@ -1074,8 +1074,7 @@ int alebgk_body_loads(alebgk_ctx *c, int nbodies, const double *centre,
     if (c->maxBodyId >= nbodies)
         return fail(c, ALEBGK_EINVAL, "a particle's body id exceeds nbodies");
     CK(cudaSetDevice(c->cfg.device));
-    double *dc = nullptr;
-    CK(cudaMalloc(&dc, 4 * 64 * sizeof(double)));
+    double *dc = c->d.bodyIO;      // the context's body staging (its head holds 13 x 64 values)
     cudaError_t e = cudaMemcpyAsync(dc, centre, 24 * (size_t)nbodies, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(dc + 3 * 64, area, 8 * (size_t)nbodies, cudaMemcpyHostToDevice, c->stream);
@@ -1083,7 +1082,6 @@ int alebgk_body_loads(alebgk_ctx *c, int nbodies, const double *centre,
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(out, c->d.bodyOut, 48 * (size_t)nbodies, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(dc);
     if (e != cudaSuccess)
         return fail(c, ALEBGK_ECUDA, std::string("body loads: ") + cudaGetErrorString(e));
     return ALEBGK_OK;
