@@ -105,6 +105,14 @@ cudaError_t pinnedStaging(alebgk_ctx *c, size_t bytes)
     return e;
 }
 
+void freeMarch(alebgk_ctx *c)
+{
+    if (c->march.units) cudaFree(c->march.units);
+    if (c->march.coefT) cudaFree(c->march.coefT);
+    if (c->march.coefTy) cudaFree(c->march.coefTy);
+    c->march = MarchState();
+}
+
 void freeBuffers(alebgk_ctx *c)
 {
     DeviceBuffers &d = c->d;
@@ -119,10 +127,7 @@ void freeBuffers(alebgk_ctx *c)
     if (c->macSnap) { cudaFree(c->macSnap); c->macSnap = nullptr; }
     c->snapSteps = -1;
     c->hostSteps = 0;
-    if (c->march.units) cudaFree(c->march.units);
-    if (c->march.coefT) cudaFree(c->march.coefT);
-    if (c->march.coefTy) cudaFree(c->march.coefTy);
-    c->march = MarchState();
+    freeMarch(c);
     for (auto &g : c->graph)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     c->uploaded = false;
@@ -237,6 +242,70 @@ int alebgk_last_error(const alebgk_ctx *c, char *buf, size_t len)
 
 // The geometry part of alebgk_upload (tables, march plan, buffers); with
 // withState also the state (g and macros) from the cloud.
+// Sets up the lattice march where it applies (a complete 3-D lattice without
+// bodies): its plan, and its coefficient table laid out from the class table
+// that is already on the device.
+static int setupMarch(alebgk_ctx *c, const alebgk_cloud *cl, const CoeffTables &tb)
+{
+    freeMarch(c);
+    const StepParams &p = c->sp;
+    DeviceBuffers &d = c->d;
+    const int N = p.N;
+    const bool f64 = c->cfg.precision == 64;
+    const size_t es = f64 ? 8 : 4;
+    std::string err;
+    bool anyBody = false;
+    for (int i = 0; i < N && !anyBody; ++i) anyBody = cl->body_id[i] >= 0;
+    if (c->cfg.transport != 1 && !anyBody)
+    {
+        MarchPlan plan;
+        buildMarchPlan(cl->xyz, N, p.dim, cl->nnb, cl->nbr, ALEBGK_MAX_NEIGH, tb, plan);
+        if (plan.ok)
+        {
+            MarchState &m = c->march;
+            m.f64 = f64;
+            m.vpl = f64 ? 1 : c->tune.marchVpl;
+            // one list, the long y-march units first
+            std::vector<MarchUnit> all(plan.unitsY);
+            all.insert(all.end(), plan.units.begin(), plan.units.end());
+            m.nunits = (int)all.size();
+            m.nunitsY = (int)plan.unitsY.size();
+            m.Vpad = plan.Vpad; m.Nx = plan.Nx; m.Ny = plan.Ny; m.Nz = plan.Nz;
+            CK(cudaMalloc(&m.units, sizeof(MarchUnit) * m.nunits));
+            CK(cudaMemcpy(m.units, all.data(), sizeof(MarchUnit) * m.nunits,
+                          cudaMemcpyHostToDevice));
+            auto table = [&](void **dst, const std::vector<int> &slotOf) -> cudaError_t {
+                int *so = nullptr;
+                cudaError_t e = cudaMalloc(dst, slotOf.size() * (size_t)m.Vpad * es);
+                if (e == cudaSuccess) e = cudaMalloc(&so, slotOf.size() * 4);
+                if (e == cudaSuccess)
+                    e = cudaMemcpy(so, slotOf.data(), slotOf.size() * 4, cudaMemcpyHostToDevice);
+                if (e == cudaSuccess)
+                    e = launchMarchTable(d.coef, so, plan.ncls, tb.S, p.V, m.Vpad, f64, *dst,
+                                         c->stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+                if (so) cudaFree(so);
+                return e;
+            };
+            CK(table(&m.coefT, plan.slotOf));
+            if (m.nunitsY > 0) CK(table(&m.coefTy, plan.slotOfY));
+            for (int b = 0; b < 2; ++b)
+            {
+                if (!encodeMarchMap(m.tmap[b], d.f[b], p.V, m.Nx, m.Ny, m.Nz, p.ldf, false,
+                                    f64, m.vpl, &err))
+                    return fail(c, ALEBGK_ECUDA, err);
+                if (m.nunitsY > 0 &&
+                    !encodeMarchMap(m.tmapY[b], d.f[b], p.V, m.Nx, m.Ny, m.Nz, p.ldf, true,
+                                    f64, m.vpl, &err))
+                    return fail(c, ALEBGK_ECUDA, err);
+            }
+            CK(prepareMarch());
+            m.enabled = true;
+        }
+    }
+    return ALEBGK_OK;
+}
+
 static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool withState)
 {
     if (!c || !cl) return fail(c, ALEBGK_EINVAL, "null argument");
@@ -263,15 +332,9 @@ static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool wi
     in.maxNeigh = ALEBGK_MAX_NEIGH;
     CoeffTables tb, tl;
     std::string err;
-    // The tables are solved on the device, except where the lattice march
-    // may take the cloud: its plan re-lays the host tables.
-    const bool f64cloud = c->cfg.precision == 64;
-    bool anyBody = false;
-    for (int i = 0; i < N && !anyBody; ++i) anyBody = cl->body_id[i] >= 0;
-    const bool devTables =
-        (gCoeffBuilder == 0 || gCoeffBuilder == 2) &&
-        !(!f64cloud && c->cfg.transport != 1 && !anyBody &&
-          marchEligible(cl->xyz, N, p.dim, cl->nnb, cl->nbr, ALEBGK_MAX_NEIGH));
+    // The tables are solved on the device; the lattice march's own table is
+    // laid out from them.
+    const bool devTables = gCoeffBuilder == 0 || gCoeffBuilder == 2;
     CoeffInput inLin = in;
     inLin.mlsOrder = 1;
     DeviceBuffers &d = c->d;
@@ -418,50 +481,8 @@ static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool wi
         return fail(c, ALEBGK_EINVAL,
                     "the streamed particle kernel needs a 3-D cloud whose rows fit in "
                     "shared memory");
-    // Lattice-marching transport (FP32, complete 3-D lattice; such clouds
-    // always take the host tables, which the plan re-lays).
-    if (!f64 && c->cfg.transport != 1 && !devTables)
-    {
-        MarchPlan plan;
-        buildMarchPlan(cl->xyz, N, p.dim, cl->nnb, cl->nbr, ALEBGK_MAX_NEIGH, tb,
-                       nullptr, plan);
-        if (plan.ok)
-        {
-            MarchState &m = c->march;
-            m.vpl = c->tune.marchVpl;
-            // one list, the long y-march units first
-            std::vector<MarchUnit> all(plan.unitsY);
-            all.insert(all.end(), plan.units.begin(), plan.units.end());
-            m.nunits = (int)all.size();
-            m.nunitsY = (int)plan.unitsY.size();
-            m.Vpad = plan.Vpad; m.Nx = plan.Nx; m.Ny = plan.Ny; m.Nz = plan.Nz;
-            CK(cudaMalloc(&m.units, sizeof(MarchUnit) * m.nunits));
-            CK(cudaMemcpy(m.units, all.data(), sizeof(MarchUnit) * m.nunits,
-                          cudaMemcpyHostToDevice));
-            CK(cudaMalloc(&m.coefT, plan.coefT.size() * 4));
-            CK(cudaMemcpy(m.coefT, plan.coefT.data(), plan.coefT.size() * 4,
-                          cudaMemcpyHostToDevice));
-            if (m.nunitsY > 0)
-            {
-                CK(cudaMalloc(&m.coefTy, plan.coefTy.size() * 4));
-                CK(cudaMemcpy(m.coefTy, plan.coefTy.data(), plan.coefTy.size() * 4,
-                              cudaMemcpyHostToDevice));
-            }
-            for (int b = 0; b < 2; ++b)
-            {
-                if (!encodeMarchMap(m.tmap[b], d.f[b], p.V, m.Nx, m.Ny, m.Nz, p.ldf, false,
-                                    m.vpl, &err))
-                    return fail(c, ALEBGK_ECUDA, err);
-                if (m.nunitsY > 0 &&
-                    !encodeMarchMap(m.tmapY[b], d.f[b], p.V, m.Nx, m.Ny, m.Nz, p.ldf, true,
-                                    m.vpl, &err))
-                    return fail(c, ALEBGK_ECUDA, err);
-            }
-            CK(prepareMarch());
-            m.enabled = true;
-        }
-    }
-    if (c->cfg.transport == 2 && !c->march.enabled)
+    if (const int r = setupMarch(c, cl, tb)) return r;
+    if (c->cfg.transport == 2 && (!c->march.enabled || f64))
         return fail(c, ALEBGK_EINVAL,
                     "the lattice march needs FP32 and a complete 3-D lattice cloud");
     c->bodyIdHost.assign(cl->body_id, cl->body_id + N);
@@ -495,19 +516,15 @@ namespace {
 // step scalars and every per-particle buffer stay where they are; the
 // geometry arrays, stencil classes and slot lists (built on the device from
 // the uploaded geometry) and MLS tables (solved on the device) are written
-// over the old ones, and only buffers that must grow are reallocated.  Returns 1 (nothing done) where it does not apply: tables the
-// host builds, or a cloud the lattice march takes.
+// over the old ones, and only buffers that must grow are reallocated; a
+// lattice's march is set up again.  Returns 1 (nothing done) where it does
+// not apply: tables the host builds.
 int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
 {
     StepParams &p = c->sp;
     const int N = p.N;
-    if (gCoeffBuilder == 1 || c->march.enabled) return 1;
-    bool anyBody = false;
-    for (int i = 0; i < N && !anyBody; ++i) anyBody = cl->body_id[i] >= 0;
+    if (gCoeffBuilder == 1) return 1;
     const bool f64 = c->cfg.precision == 64;
-    if (!f64 && c->cfg.transport != 1 && !anyBody &&
-        marchEligible(cl->xyz, N, p.dim, cl->nnb, cl->nbr, ALEBGK_MAX_NEIGH))
-        return 1;
     if (const int r = checkNeighbours(c, cl, N)) return r;
     p.dt = dt;
     p.lam = dt / p.tau;
@@ -593,10 +610,12 @@ int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
                       cudaMemcpyHostToDevice));
     CK(putRowOrder(c, cl->boundary, N));
     CK(cudaStreamSynchronize(c->stream));
-    // The step graphs hold the slot stride and the table pointers: rebuilt
-    // when either changed.
+    const bool marched = c->march.enabled;
+    if (const int r = setupMarch(c, cl, tb)) return r;
+    // The step graphs hold the slot stride, the table pointers and the march's
+    // plan: rebuilt when any changed.
     const void *bufAfter[] = {d.coef, d.coefLin, d.slots, d.surfList, d.bodyIO};
-    bool same = std::memcmp(spBefore, &p, sizeof p) == 0;
+    bool same = std::memcmp(spBefore, &p, sizeof p) == 0 && !marched && !c->march.enabled;
     for (int k = 0; k < 5 && same; ++k) same = bufBefore[k] == bufAfter[k];
     if (!same)
         for (auto &g : c->graph)

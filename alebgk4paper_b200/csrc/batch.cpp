@@ -155,16 +155,17 @@ int alebgk_set_march_width(alebgk_ctx *c, int velocities_per_lane)
         return failc(c, ALEBGK_EINVAL, "march width: 1 or 2 velocities per lane");
     c->tune.marchVpl = velocities_per_lane;
     MarchState &m = c->march;
-    if (!m.enabled || m.vpl == velocities_per_lane) return ALEBGK_OK;
+    // (FP64 rows always march one velocity a lane.)
+    if (!m.enabled || m.f64 || m.vpl == velocities_per_lane) return ALEBGK_OK;
     m.vpl = velocities_per_lane;
     const StepParams &p = c->sp;
     std::string err;
     for (int b = 0; b < 2; ++b)
     {
-        if (!encodeMarchMap(m.tmap[b], c->d.f[b], p.V, m.Nx, m.Ny, m.Nz, p.ldf, false, m.vpl,
+        if (!encodeMarchMap(m.tmap[b], c->d.f[b], p.V, m.Nx, m.Ny, m.Nz, p.ldf, false, false, m.vpl,
                             &err) ||
             (m.nunitsY > 0 && !encodeMarchMap(m.tmapY[b], c->d.f[b], p.V, m.Nx, m.Ny, m.Nz,
-                                              p.ldf, true, m.vpl, &err)))
+                                              p.ldf, true, false, m.vpl, &err)))
             return failc(c, ALEBGK_ECUDA, err);
     }
     dropGraphs(c);

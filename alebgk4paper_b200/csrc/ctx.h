@@ -17,9 +17,10 @@ struct MarchState
 {
     bool enabled = false;
     int nunits = 0, nunitsY = 0, Vpad = 0, Nx = 0, Ny = 0, Nz = 0;
-    int vpl = 2;                              // velocities per lane (1 or 2)
+    int vpl = 2;                              // FP32: velocities per lane (1 or 2); FP64: 1
+    bool f64 = false;
     MarchUnit *units = nullptr;               // y-march units first, then z-march
-    float *coefT = nullptr, *coefTy = nullptr;
+    void *coefT = nullptr, *coefTy = nullptr; // [class][81][Vpad], FP32 or FP64
     alignas(64) unsigned char tmap[2][128];   // CUtensorMap per source buffer
     alignas(64) unsigned char tmapY[2][128];  // the same with the y-march box
 };
@@ -287,9 +288,13 @@ cudaError_t bodyLoadsNoAlloc(alebgk_ctx *c, int nbodies, const double *centre,
 cudaError_t launchResidual(alebgk_ctx *c, double *out, cudaStream_t st);
 cudaError_t launchConvertIn(alebgk_ctx *c, const double *src, int buf);
 cudaError_t launchConvertOut(alebgk_ctx *c, double *dst, int buf);
-cudaError_t launchMarch(alebgk_ctx *c, int from, float *outBuf, cudaStream_t st);
+cudaError_t launchMarch(alebgk_ctx *c, int from, void *outBuf, cudaStream_t st);
 cudaError_t prepareMarch();
+// The march's coefficient table [class][81][Vpad] from the class table coef
+// [class][S][V] and the template's slots (device arrays).
+cudaError_t launchMarchTable(const void *coef, const int *slotOf, int ncls, int S, int V, int Vpad,
+                             bool f64, void *out, cudaStream_t st);
 bool encodeMarchMap(void *tmapOut, void *f, int V, int Nx, int Ny, int Nz, int ldf,
-                    bool yMarch, int vpl, std::string *err);
+                    bool yMarch, bool f64, int vpl, std::string *err);
 
 }  // namespace alebgk

@@ -1,4 +1,4 @@
-// march.cu -- lattice-marching MLS transport for sm_100a (FP32).
+// march.cu -- lattice-marching MLS transport for sm_100a (FP32 and FP64).
 //
 // gt(x,y,z;k) = scale * sum_o C[class][o][k] * h(x+o;k) over the 81 lattice
 // offsets |o|^2 <= 6, for a cloud that is a complete lattice (march.h).
@@ -25,6 +25,12 @@
 // far ahead as the ring allows.  Every wait is bounded; a timeout sets the
 // step's error word instead of hanging.  Packed and scalar FMAs round alike (each half of
 // fma.rn.f32x2 is one fmaf), so both widths give the same bits.
+//
+// FP64 takes the kernel at one velocity a lane, in the registers and shared
+// memory of the two-velocity FP32 form: its bound is the FP64 pipe (4.8e9
+// FMAs at cavity3d Nx 40 Nv 10, 0.26 ms at 64 lanes an SM; HBM 0.16 ms).
+// Measured there: 2.58 ms by the coefficient gather (L1-bound, a coefficient
+// and a value loaded per FMA), 0.685 ms marched.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -43,9 +49,11 @@ constexpr int kPW = kMarchTileX + 4;      // staged plane: 12 x 8 particles
 constexpr int kPH = kMarchTileY + 4;
 constexpr int kRing = 6;                  // staged planes
 // Bytes of one staged plane at VPL velocities per lane.
-template <int VPL>
-__host__ __device__ constexpr uint32_t planeBytes() { return kPW * kPH * kMarchChunk * VPL * 4; }
-
+template <typename R, int VPL>
+__host__ __device__ constexpr uint32_t planeBytes()
+{
+    return kPW * kPH * kMarchChunk * VPL * sizeof(R);
+}
 
 __host__ __device__ constexpr int tidx(int dx, int dy, int dz)
 {
@@ -73,17 +81,26 @@ __device__ __forceinline__ void unroll(F &&f)
     unrollImpl(std::make_integer_sequence<int, N>{}, f);
 }
 
-// VPL velocities of one lane: a float, or a float2 updated by packed
-// fma.rn.f32x2 / mul.rn.f32x2 (sm_100a).
-template <int VPL> struct Lanes;
-template <> struct Lanes<1>
+// VPL velocities of one lane: a float, a float2 updated by packed
+// fma.rn.f32x2 / mul.rn.f32x2 (sm_100a), or a double.  float2 and double take
+// the same registers and shared memory, and each of their FMAs holds the FMA
+// pipe for two cycles a warp.
+template <typename R, int VPL> struct Lanes;
+template <> struct Lanes<float, 1>
 {
     typedef float T;
     static __device__ __forceinline__ T zero() { return 0.0f; }
     static __device__ __forceinline__ T fma(T a, T b, T c) { return fmaf(a, b, c); }
     static __device__ __forceinline__ T mul(T a, float s) { return a * s; }
 };
-template <> struct Lanes<2>
+template <> struct Lanes<double, 1>
+{
+    typedef double T;
+    static __device__ __forceinline__ T zero() { return 0.0; }
+    static __device__ __forceinline__ T fma(T a, T b, T c) { return ::fma(a, b, c); }
+    static __device__ __forceinline__ T mul(T a, double s) { return a * s; }
+};
+template <> struct Lanes<float, 2>
 {
     typedef float2 T;
     static __device__ __forceinline__ T zero() { return make_float2(0.0f, 0.0f); }
@@ -107,17 +124,17 @@ __device__ __forceinline__ void tmaLoadPlane(void *dst, const CUtensorMap *map, 
 
 }  // namespace
 
-template <int VPL>
-__global__ void __launch_bounds__(kMarchWarps * 32, 3 - VPL)
+template <typename R, int VPL>
+__global__ void __launch_bounds__(kMarchWarps * 32, VPL * (int)sizeof(R) == 4 ? 2 : 1)
 k_march(const __grid_constant__ CUtensorMap tmapZ, const __grid_constant__ CUtensorMap tmapY,
-        const MarchUnit *__restrict__ units, const float *__restrict__ coefTz,
-        const float *__restrict__ coefTy, float *__restrict__ out, int ldf, int Nx, int Ny,
+        const MarchUnit *__restrict__ units, const R *__restrict__ coefTz,
+        const R *__restrict__ coefTy, R *__restrict__ out, int ldf, int Nx, int Ny,
         int Nz, int V, int Vpad, StepScalars *sc)
 {
-    typedef Lanes<VPL> LN;
+    typedef Lanes<R, VPL> LN;
     typedef typename LN::T VT;
     constexpr int CW = kMarchChunk * VPL;        // velocities per CTA
-    constexpr uint32_t kPlaneBytes = planeBytes<VPL>();
+    constexpr uint32_t kPlaneBytes = planeBytes<R, VPL>();
     extern __shared__ __align__(128) unsigned char marchSmem[];
     typedef VT Plane[kPH][kPW][kMarchChunk];
     Plane *ring = reinterpret_cast<Plane *>(marchSmem);
@@ -134,7 +151,7 @@ k_march(const __grid_constant__ CUtensorMap tmapZ, const __grid_constant__ CUten
     // at one y, with the coefficients in that frame.
     const bool yMarch = u.yMarch != 0;
     const CUtensorMap *tmap = yMarch ? &tmapY : &tmapZ;
-    const float *coefT = yMarch ? coefTy : coefTz;
+    const R *coefT = yMarch ? coefTy : coefTz;
     const int colStride = ldf;
     const int rowStride = yMarch ? ldf * Nx * Ny : ldf * Nx;
     const int planeStride = yMarch ? ldf * Nx : ldf * Nx * Ny;
@@ -194,13 +211,13 @@ k_march(const __grid_constant__ CUtensorMap tmapZ, const __grid_constant__ CUten
     for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int r = 0; r < 5; ++r) acc[c][r] = LN::zero();
-    const float scale = (float)sc->scale;
+    const R scale = (R)sc->scale;
     // Output column c of the warp's block at plane z:
     // outBase + z planeStride + (c & 1) colStride + (c >> 1) rowStride.
     // With VPL = 2 and an odd V the last pair of a row may end one past V:
     // that float lies in the row padding (ldf rounds V up to a multiple of
     // four), which nothing reads.
-    float *outBase = out + (long long)(ux0 + bx) * colStride + (long long)(uy0 + by) * rowStride + k;
+    R *outBase = out + (long long)(ux0 + bx) * colStride + (long long)(uy0 + by) * rowStride + k;
     const int smask = (k < V) ? mask : 0;
     bool dead = false;
 
@@ -239,8 +256,8 @@ k_march(const __grid_constant__ CUtensorMap tmapZ, const __grid_constant__ CUten
             unroll<EB>([&](auto B) {
                 constexpr int dx = (xMajor ? decltype(A)::value : decltype(B)::value) - 2;
                 constexpr int dy = (xMajor ? decltype(B)::value : decltype(A)::value) - 2;
-                unroll<5>([&](auto R) {
-                    constexpr int r = decltype(R)::value;
+                unroll<5>([&](auto Q) {
+                    constexpr int r = decltype(Q)::value;
                     constexpr int dz = 2 - r;
                     if (!gated || inSeg(r))
                     {
@@ -256,7 +273,7 @@ k_march(const __grid_constant__ CUtensorMap tmapZ, const __grid_constant__ CUten
         });
     };
     // Queue slot 0 (output plane zi - 2) is complete: store it, shift.
-    auto storeShift = [&](auto SHAPE, float *o, bool store) {
+    auto storeShift = [&](auto SHAPE, R *o, bool store) {
         constexpr int shp = decltype(SHAPE)::value;
         if (store)
         {
@@ -305,7 +322,7 @@ k_march(const __grid_constant__ CUtensorMap tmapZ, const __grid_constant__ CUten
     auto marchLong = [&](auto SHAPE) {
         int s = 0;
         uint32_t par = 0;
-        float *o = outBase + (long long)(za - 4) * planeStride;   // plane zi - 2 at n = 0
+        R *o = outBase + (long long)(za - 4) * planeStride;   // plane zi - 2 at n = 0
         for (int n = 0; n < nin; ++n)
         {
             mbarWait(&full[s], par, dead);
@@ -325,7 +342,7 @@ k_march(const __grid_constant__ CUtensorMap tmapZ, const __grid_constant__ CUten
         const unsigned L = (unsigned)(zb - za);
         int s = 0;
         uint32_t par = 0;
-        float *o = outBase + (long long)(za - 4) * planeStride;
+        R *o = outBase + (long long)(za - 4) * planeStride;
         for (int n = 0; n < nin; ++n)
         {
             const int m = n - moff;
@@ -369,7 +386,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   CUtensorMapFloatOOBfill);
 
 bool encodeMarchMap(void *tmapOut, void *f, int V, int Nx, int Ny, int Nz, int ldf,
-                    bool yMarch, int vpl, std::string *err)
+                    bool yMarch, bool f64, int vpl, std::string *err)
 {
     static EncodeTiledFn fn = nullptr;
     if (!fn)
@@ -386,8 +403,8 @@ bool encodeMarchMap(void *tmapOut, void *f, int V, int Nx, int Ny, int Nz, int l
         fn = reinterpret_cast<EncodeTiledFn>(p);
     }
     const cuuint64_t dims[4] = {(cuuint64_t)V, (cuuint64_t)Nx, (cuuint64_t)Ny, (cuuint64_t)Nz};
-    const cuuint64_t strides[3] = {(cuuint64_t)ldf * 4, (cuuint64_t)ldf * 4 * Nx,
-                                   (cuuint64_t)ldf * 4 * Nx * Ny};
+    const cuuint64_t es = f64 ? 8 : 4;
+    const cuuint64_t strides[3] = {ldf * es, ldf * es * Nx, ldf * es * Nx * Ny};
     // z-march: a 12 x 8 (x, y) tile at one z; y-march: a 12 x 8 (x, z) tile
     // at one y.  Both land in shared memory as [8][12][32 vpl velocities].
     const cuuint32_t cw = (cuuint32_t)(kMarchChunk * vpl);
@@ -395,8 +412,8 @@ bool encodeMarchMap(void *tmapOut, void *f, int V, int Nx, int Ny, int Nz, int l
     const cuuint32_t boxY[4] = {cw, kPW, 1, kPH};
     const cuuint32_t *box = yMarch ? boxY : boxZ;
     const cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = fn(reinterpret_cast<CUtensorMap *>(tmapOut), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                    f, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    CUresult r = fn(reinterpret_cast<CUtensorMap *>(tmapOut),
+                    f64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, f, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
@@ -409,32 +426,71 @@ bool encodeMarchMap(void *tmapOut, void *f, int V, int Nx, int Ny, int Nz, int l
 
 cudaError_t prepareMarch()
 {
-    cudaError_t e = cudaFuncSetAttribute(k_march<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kRing * planeBytes<1>()));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_march<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(kRing * planeBytes<2>()));
+    auto set = [](const void *fn, uint32_t plane) {
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(kRing * plane));
+    };
+    cudaError_t e = set((const void *)k_march<float, 1>, planeBytes<float, 1>());
+    if (e == cudaSuccess) e = set((const void *)k_march<float, 2>, planeBytes<float, 2>());
+    if (e == cudaSuccess) e = set((const void *)k_march<double, 1>, planeBytes<double, 1>());
     return e;
 }
 
-cudaError_t launchMarch(alebgk_ctx *c, int from, float *outBuf, cudaStream_t st)
+namespace {
+
+template <typename R>
+__global__ void k_march_table(const R *__restrict__ coef, const int *__restrict__ slotOf, int S,
+                              int V, int Vpad, R *__restrict__ out)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= Vpad) return;
+    const size_t row = (size_t)blockIdx.z * kTmplOffsets + blockIdx.y;   // class, offset
+    const int s = slotOf[row];
+    out[row * Vpad + k] = (s >= 0 && k < V) ? coef[((size_t)blockIdx.z * S + s) * V + k] : R(0);
+}
+
+template <typename R, int VPL>
+void launchMarchT(const alebgk_ctx *c, int from, void *outBuf, cudaStream_t st)
 {
     const StepParams &p = c->sp;
     const MarchState &ms = c->march;
     const CUtensorMap *tz = reinterpret_cast<const CUtensorMap *>(ms.tmap[from]);
     const CUtensorMap *ty = reinterpret_cast<const CUtensorMap *>(ms.nunitsY ? ms.tmapY[from]
                                                                               : ms.tmap[from]);
-    const float *cy = ms.coefTy ? ms.coefTy : ms.coefT;
-    if (ms.vpl == 2)
-        k_march<2><<<dim3(ms.Vpad / (2 * kMarchChunk), ms.nunits), kMarchWarps * 32,
-                     kRing * planeBytes<2>(), st>>>(*tz, *ty, ms.units, ms.coefT, cy, outBuf,
-                                                    p.ldf, ms.Nx, ms.Ny, ms.Nz, p.V, ms.Vpad,
-                                                    c->d.sc);
-    else
-        k_march<1><<<dim3(ms.Vpad / kMarchChunk, ms.nunits), kMarchWarps * 32,
-                     kRing * planeBytes<1>(), st>>>(*tz, *ty, ms.units, ms.coefT, cy, outBuf,
-                                                    p.ldf, ms.Nx, ms.Ny, ms.Nz, p.V, ms.Vpad,
-                                                    c->d.sc);
+    const R *cz = static_cast<const R *>(ms.coefT);
+    const R *cy = ms.coefTy ? static_cast<const R *>(ms.coefTy) : cz;
+    k_march<R, VPL><<<dim3((p.V + VPL * kMarchChunk - 1) / (VPL * kMarchChunk), ms.nunits),
+                      kMarchWarps * 32, kRing * planeBytes<R, VPL>(), st>>>(
+        *tz, *ty, ms.units, cz, cy, static_cast<R *>(outBuf), p.ldf, ms.Nx, ms.Ny, ms.Nz, p.V,
+        ms.Vpad, c->d.sc);
+}
+
+}  // namespace
+
+cudaError_t launchMarchTable(const void *coef, const int *slotOf, int ncls, int S, int V, int Vpad,
+                             bool f64, void *out, cudaStream_t st)
+{
+    // at most 65535 classes per launch (the grid's z limit)
+    for (int c0 = 0; c0 < ncls; c0 += 65535)
+    {
+        const dim3 grid((Vpad + 255) / 256, kTmplOffsets, ncls - c0 < 65535 ? ncls - c0 : 65535);
+        const size_t src = (size_t)c0 * S * V, dst = (size_t)c0 * kTmplOffsets * Vpad;
+        const int *so = slotOf + (size_t)c0 * kTmplOffsets;
+        if (f64)
+            k_march_table<double><<<grid, 256, 0, st>>>(static_cast<const double *>(coef) + src, so,
+                                                        S, V, Vpad, static_cast<double *>(out) + dst);
+        else
+            k_march_table<float><<<grid, 256, 0, st>>>(static_cast<const float *>(coef) + src, so, S,
+                                                       V, Vpad, static_cast<float *>(out) + dst);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launchMarch(alebgk_ctx *c, int from, void *outBuf, cudaStream_t st)
+{
+    if (c->march.f64) launchMarchT<double, 1>(c, from, outBuf, st);
+    else if (c->march.vpl == 2) launchMarchT<float, 2>(c, from, outBuf, st);
+    else launchMarchT<float, 1>(c, from, outBuf, st);
     return cudaGetLastError();
 }
 

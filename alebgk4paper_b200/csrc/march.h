@@ -47,20 +47,14 @@ struct MarchPlan
     int ncls = 0, Vpad = 0;
     std::vector<MarchUnit> units;    // marching through z
     std::vector<MarchUnit> unitsY;   // thin z-planes, marching through y
-    std::vector<float> coefT;        // [class][81][Vpad]
-    std::vector<float> coefTy;       // the same in the y-march frame
-    std::vector<float> coefTLin;     // same, linear MLS
+    // [class][81]: the slot of the class's table that holds each template
+    // offset (-1: none), and the same in the y-march frame.
+    std::vector<int> slotOf, slotOfY;
 };
 
 // Detects the lattice and builds the plan; plan.ok is false when the cloud
 // is not a complete lattice with two-step stencils.
-// Whether a cloud is a complete lattice in generation order with every
-// neighbour within the march's 81-offset template (the test of buildMarchPlan).
-bool marchEligible(const double *xyz, int N, int dim, const int *nnb, const int *nbr,
-                   int maxNeigh);
-
 void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb,
-                    const int *nbr, int maxNeigh, const CoeffTables &tb,
-                    const CoeffTables *tl, MarchPlan &plan);
+                    const int *nbr, int maxNeigh, const CoeffTables &tb, MarchPlan &plan);
 
 }  // namespace alebgk

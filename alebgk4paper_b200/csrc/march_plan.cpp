@@ -3,6 +3,7 @@
 #include "march.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <map>
 
@@ -10,16 +11,18 @@ namespace alebgk {
 
 int templateIndex(int dx, int dy, int dz)
 {
-    int n = 0;
-    for (int z = -2; z <= 2; ++z)
-        for (int y = -2; y <= 2; ++y)
-            for (int x = -2; x <= 2; ++x)
-            {
-                if (x * x + y * y + z * z > 6) continue;
-                if (x == dx && y == dy && z == dz) return n;
-                ++n;
-            }
-    return -1;
+    // (a table: every neighbour of every particle is looked up)
+    static const std::array<int, 125> table = [] {
+        std::array<int, 125> t{};
+        int n = 0;
+        for (int z = -2; z <= 2; ++z)
+            for (int y = -2; y <= 2; ++y)
+                for (int x = -2; x <= 2; ++x)
+                    t[(z + 2) * 25 + (y + 2) * 5 + x + 2] = x * x + y * y + z * z > 6 ? -1 : n++;
+        return t;
+    }();
+    if (dx < -2 || dx > 2 || dy < -2 || dy > 2 || dz < -2 || dz > 2) return -1;
+    return table[(dz + 2) * 25 + (dy + 2) * 5 + dx + 2];
 }
 
 namespace {
@@ -48,38 +51,8 @@ int axisRanks(const double *xyz, int N, int axis, std::vector<int> &rank)
 
 }  // namespace
 
-bool marchEligible(const double *xyz, int N, int dim, const int *nnb, const int *nbr,
-                   int maxNeigh)
-{
-    if (dim != 3 || N < 8) return false;
-    std::vector<int> rx, ry, rz;
-    const int nx = axisRanks(xyz, N, 0, rx);
-    const int ny = axisRanks(xyz, N, 1, ry);
-    const int nz = axisRanks(xyz, N, 2, rz);
-    if ((long long)nx * ny * nz != N || nx < 2 || ny < 2 || nz < 2) return false;
-    const bool zdesc = rz[0] > rz[(size_t)nx * ny];
-    for (int i = 0; i < N; ++i)
-    {
-        const int ix = i % nx, iy = (i / nx) % ny, iz = i / (nx * ny);
-        const int ez = zdesc ? nz - 1 - iz : iz;
-        if (rx[i] != ix || ry[i] != iy || rz[i] != ez) return false;
-    }
-    for (int i = 0; i < N; ++i)
-    {
-        const int xi = i % nx, yi = (i / nx) % ny, zi = i / (nx * ny);
-        for (int s = 0; s < nnb[i]; ++s)
-        {
-            const int j = nbr[(size_t)i * maxNeigh + s];
-            if (templateIndex(j % nx - xi, (j / nx) % ny - yi, j / (nx * ny) - zi) < 0)
-                return false;
-        }
-    }
-    return true;
-}
-
 void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb, const int *nbr,
-                    int maxNeigh, const CoeffTables &tb, const CoeffTables *tl,
-                    MarchPlan &plan)
+                    int maxNeigh, const CoeffTables &tb, MarchPlan &plan)
 {
     plan = MarchPlan();
     if (dim != 3 || N < 8) return;
@@ -113,37 +86,25 @@ void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb, const int
         }
     }
 
-    // Canonical tables [class][81][Vpad].
+    // Template offset -> slot of each class, from its representative.
     const int V = tb.V, ncls = tb.ncls, S = tb.S;
     // Rows padded to whole chunks of the widest march (two velocities per lane).
     const int Vpad = (V + 2 * kMarchChunk - 1) / (2 * kMarchChunk) * (2 * kMarchChunk);
     plan.Nx = nx; plan.Ny = ny; plan.Nz = nz; plan.ncls = ncls; plan.Vpad = Vpad;
-    plan.coefT.assign((size_t)ncls * kTmplOffsets * Vpad, 0.0f);
-    if (tl) plan.coefTLin.assign((size_t)ncls * kTmplOffsets * Vpad, 0.0f);
-    // FP32 images of the class tables (roundCoefFP32), re-laid by offset.
-    std::vector<float> img((size_t)S * V), imgLin(tl ? (size_t)S * V : 0);
+    plan.slotOf.assign((size_t)ncls * kTmplOffsets, -1);
     for (int c = 0; c < ncls; ++c)
     {
         const int r = tb.rep[c];
         int xr, yr, zr;
         coord(r, xr, yr, zr);
-        const int *sl = &tb.slots[(size_t)r * S];
-        roundCoefFP32(&tb.coef[(size_t)c * S * V], img.data(), S, V);
-        if (tl) roundCoefFP32(&tl->coef[(size_t)c * S * V], imgLin.data(), S, V);
-        for (int s = 0; s < tb.nslot[r]; ++s)
+        const bool dev = !tb.repSlots.empty();
+        const int *sl = dev ? &tb.repSlots[(size_t)c * S] : &tb.slots[(size_t)r * S];
+        const int ns = dev ? tb.repNslot[c] : tb.nslot[r];
+        for (int s = 0; s < ns; ++s)
         {
             int xj, yj, zj;
             coord(sl[s], xj, yj, zj);
-            const int o = templateIndex(xj - xr, yj - yr, zj - zr);
-            const float *src = &img[(size_t)s * V];
-            float *dst = &plan.coefT[((size_t)c * kTmplOffsets + o) * Vpad];
-            for (int k = 0; k < V; ++k) dst[k] = src[k];
-            if (tl)
-            {
-                const float *sl2 = &imgLin[(size_t)s * V];
-                float *d2 = &plan.coefTLin[((size_t)c * kTmplOffsets + o) * Vpad];
-                for (int k = 0; k < V; ++k) d2[k] = sl2[k];
-            }
+            plan.slotOf[(size_t)c * kTmplOffsets + templateIndex(xj - xr, yj - yr, zj - zr)] = s;
         }
     }
 
@@ -281,21 +242,20 @@ void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb, const int
                 emit(plan.unitsY, x0, z0, ya, yb, subs);
             }
     }
-    // Coefficients in the y-march frame (x, lattice z, lattice y): the
-    // kernel's offset (ox, oy, oz) is the lattice offset (ox, oz, oy).
+    // The y-march frame is (x, lattice z, lattice y): the kernel's offset
+    // (ox, oy, oz) is the lattice offset (ox, oz, oy).
     if (!plan.unitsY.empty())
     {
-        plan.coefTy.assign(plan.coefT.size(), 0.0f);
+        plan.slotOfY.resize(plan.slotOf.size());
         for (int c = 0; c < ncls; ++c)
             for (int oz = -2; oz <= 2; ++oz)
                 for (int oy = -2; oy <= 2; ++oy)
                     for (int ox = -2; ox <= 2; ++ox)
                     {
                         const int tk = templateIndex(ox, oy, oz);
-                        if (tk < 0) continue;
-                        const int tl = templateIndex(ox, oz, oy);
-                        std::copy_n(&plan.coefT[((size_t)c * kTmplOffsets + tl) * Vpad], Vpad,
-                                    &plan.coefTy[((size_t)c * kTmplOffsets + tk) * Vpad]);
+                        if (tk >= 0)
+                            plan.slotOfY[(size_t)c * kTmplOffsets + tk] =
+                                plan.slotOf[(size_t)c * kTmplOffsets + templateIndex(ox, oz, oy)];
                     }
     }
     plan.ok = ncls < (1 << 17);

@@ -2247,14 +2247,14 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
         k_step_begin<<<nadOn ? nadBlocks : 1, kNT, 0, st>>>(
             d.sc, 1, macA, d.boundary, d.nslot, d.slots, p.S, p.N, nadOn ? d.nad : nullptr);
     mark();
-    const bool march = sizeof(T) == 4 && c->march.enabled;
+    const bool march = c->march.enabled;
     // Transport fused into the particle kernel (transport threads 0), except
     // when stages are timed: then it runs as its own kernel, with the same
     // sums, so that its time is seen.
     const bool fused = !march && !c->pStream && c->tune.transportThreads == 0 && !ev;
     if (march)
     {
-        cudaError_t e = launchMarch(c, from, reinterpret_cast<float *>(fb), st);
+        cudaError_t e = launchMarch(c, from, fb, st);
         if (e != cudaSuccess) return e;
     }
     else if (!fused)
@@ -3080,11 +3080,11 @@ static cudaError_t slabSegT(alebgk_ctx *c, int from, int seg, cudaStream_t st)
         const int nadBlocks = min((p.N + kNT / 32 - 1) / (kNT / 32), 1184);
         k_step_begin<<<nadOn ? nadBlocks : 1, kNT, 0, st>>>(
             d.sc, 1, macA, d.boundary, d.nslot, d.slots, p.S, p.N, nadOn ? d.nad : nullptr);
-        const bool march = sizeof(T) == 4 && c->march.enabled;
+        const bool march = c->march.enabled;
         const bool fused = !march && !c->pStream && c->tune.transportThreads == 0;
         if (march)
         {
-            cudaError_t e = launchMarch(c, from, reinterpret_cast<float *>(fb), st);
+            cudaError_t e = launchMarch(c, from, fb, st);
             if (e != cudaSuccess) return e;
         }
         else if (!fused)

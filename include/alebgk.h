@@ -65,8 +65,8 @@ typedef struct alebgk_config
     int periodic[3];  /* per-axis periodicity (minimum-image stencils)        */
     double L[3];      /* periodic lengths                                     */
     int transport;    /* 0 auto (lattice march when the cloud is a complete
-                         lattice and precision is 32, else coefficient
-                         gather), 1 always gather, 2 require the march       */
+                         lattice without bodies, else coefficient gather),
+                         1 always gather, 2 require the march (FP32 only)    */
     int particle;     /* 0 auto (streamed rows for a 3-D cloud whose rows fit,
                          in FP32 as three row kernels; else one warp per
                          particle), 1 always the general kernel, 2 require
