@@ -10,8 +10,6 @@
 // loop orders one for one: foot point, per-slot weight and basis, the
 // normal-equation matrix summed slot by slot, elimination with unit
 // right-hand sides, and the coefficients w_s * (row 0 of the inverse . b_s).
-// The stencil classes themselves (a hash of each particle's neighbour
-// offsets) are still built on the host.
 #include <cuda_runtime.h>
 
 #include <vector>
@@ -44,84 +42,192 @@ __device__ __forceinline__ double weightSqD(double r2, double h)
     return w * w;
 }
 
-__device__ __forceinline__ int basisD(double dx, double dy, double dz, int ndim, double h,
-                                      double *b, int order)
+// Basis of size P (3, 6: 2-D linear, quadratic; 4, 10: 3-D) at the offset
+// scaled by the support.
+template <int P>
+__device__ __forceinline__ void basisOf(double sx, double sy, double sz, double *b)
 {
-    double sx = dx / h, sy = dy / h, sz = dz / h;
     b[0] = 1.0; b[1] = sx; b[2] = sy;
-    if (ndim == 2)
+    if (P == 6)
     {
-        if (order >= 2)
-        {
-            b[3] = sx * sx; b[4] = sx * sy; b[5] = sy * sy;
-            return 6;
-        }
-        return 3;
+        b[3] = sx * sx; b[4] = sx * sy; b[5] = sy * sy;
     }
-    b[3] = sz;
-    if (order >= 2)
+    if (P == 4 || P == 10) b[3] = sz;
+    if (P == 10)
     {
         b[4] = sx * sx; b[5] = sy * sy; b[6] = sz * sz;
         b[7] = sx * sy; b[8] = sx * sz; b[9] = sy * sz;
-        return 10;
     }
-    return 4;
 }
 
-__device__ int solveSkipGED(double *A, double *B, int n, int nrhs)
+// One (class, node): the coefficients of its slots into cc, with the basis
+// size fixed at compile time so that the normal matrix lives in registers
+// from its first term to the last back substitution.  The elimination
+// (partial pivots, |pivot| < 1e-30 skipped, as solveSkipGE) keeps its
+// multipliers below the diagonal and its pivot rows in one word; the unit
+// right-hand sides, of which only the first unknown is needed, then go
+// through it one by one.  Same operations on the same values as the host's.
+template <typename T, int P>
+__device__ __forceinline__ void classNode(const ClassArgs &a, int c, int n, double xf, double yf,
+                                          double zf, const double *__restrict__ sp,
+                                          T *__restrict__ cc, int k, int *degen)
 {
-    int skipped = 0;
-    for (int col = 0; col < n; ++col)
+    constexpr bool d3 = P == 4 || P == 10;
+    const int V = a.V;
+    // weight and scaled offset of slot s; false outside the support
+    auto slotAt = [&](int s, double &ws, double &sx, double &sy, double &sz) {
+        double dx = sp[3 * s] - xf, dy = sp[3 * s + 1] - yf;
+        double dz = d3 ? sp[3 * s + 2] - zf : 0.0;
+        if (a.periodic[0]) dx = minImageD(dx, a.L[0]);
+        if (a.periodic[1]) dy = minImageD(dy, a.L[1]);
+        if (d3 && a.periodic[2]) dz = minImageD(dz, a.L[2]);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        ws = weightSqD(r2, a.h);
+        if (ws < 1.0e-30) return false;
+        sx = dx / a.h;
+        sy = dy / a.h;
+        sz = dz / a.h;
+        return true;
+    };
+    double A[P][P];
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+#pragma unroll
+        for (int j = 0; j < P; ++j) A[i][j] = 0.0;
+    bool any = false;
+#pragma unroll 1
+    for (int s = 1; s < n; ++s)
     {
-        int piv = col;
-        double mx = fabs(A[col * n + col]);
-        for (int row = col + 1; row < n; ++row)
-            if (fabs(A[row * n + col]) > mx)
-            {
-                mx = fabs(A[row * n + col]);
-                piv = row;
-            }
-        if (piv != col)
+        double ws, sx, sy, sz, b[P];
+        if (!slotAt(s, ws, sx, sy, sz)) continue;
+        basisOf<P>(sx, sy, sz, b);
+#pragma unroll
+        for (int i = 0; i < P; ++i)
         {
-            for (int j = 0; j < n; ++j)
+            const double wb = ws * b[i];
+#pragma unroll
+            for (int j = 0; j < P; ++j) A[i][j] += wb * b[j];
+        }
+        any = true;
+    }
+    if (!any) { cc[k] = (T)1.0; return; }
+    unsigned long long piv = 0;      // pivot row of column q in bits [4 q, 4 q + 4)
+    unsigned good = 0;               // columns with a pivot
+#pragma unroll
+    for (int col = 0; col < P; ++col)
+    {
+        int pr = col;
+        double mx = fabs(A[col][col]);
+#pragma unroll
+        for (int row = col + 1; row < P; ++row)
+            if (fabs(A[row][col]) > mx)
             {
-                double t = A[col * n + j]; A[col * n + j] = A[piv * n + j]; A[piv * n + j] = t;
+                mx = fabs(A[row][col]);
+                pr = row;
             }
-            for (int j = 0; j < nrhs; ++j)
+        piv |= (unsigned long long)pr << (4 * col);
+#pragma unroll
+        for (int row = col + 1; row < P; ++row)
+        {
+            const bool sw = pr == row;
+#pragma unroll
+            for (int j = col; j < P; ++j)
             {
-                double t = B[col * nrhs + j]; B[col * nrhs + j] = B[piv * nrhs + j];
-                B[piv * nrhs + j] = t;
+                const double t = A[col][j];
+                A[col][j] = sw ? A[row][j] : t;
+                A[row][j] = sw ? t : A[row][j];
             }
         }
-        double d = A[col * n + col];
-        if (fabs(d) < 1.0e-30) { ++skipped; continue; }
-        for (int row = col + 1; row < n; ++row)
+        const double d = A[col][col];
+        if (!(fabs(d) < 1.0e-30))
         {
-            double f = A[row * n + col] / d;
-            for (int j = col; j < n; ++j) A[row * n + j] -= f * A[col * n + j];
-            for (int j = 0; j < nrhs; ++j) B[row * nrhs + j] -= f * B[col * nrhs + j];
+            good |= 1u << col;
+#pragma unroll
+            for (int row = col + 1; row < P; ++row)
+            {
+                const double f = A[row][col] / d;
+#pragma unroll
+                for (int j = col + 1; j < P; ++j) A[row][j] -= f * A[col][j];
+                A[row][col] = f;     // the multiplier; nothing reads the column again
+            }
         }
     }
-    for (int i = n - 1; i >= 0; --i)
+    if (good != (1u << P) - 1) atomicAdd(degen + c, 1);
+    double B0[P];
+#pragma unroll
+    for (int m = 0; m < P; ++m)
     {
-        bool ok = fabs(A[i * n + i]) > 1.0e-30;
-        for (int r = 0; r < nrhs; ++r)
+        double x[P];
+#pragma unroll
+        for (int i = 0; i < P; ++i) x[i] = i == m ? 1.0 : 0.0;
+#pragma unroll
+        for (int col = 0; col < P; ++col)
         {
-            double s = B[i * nrhs + r];
-            for (int j = i + 1; j < n; ++j) s -= A[i * n + j] * B[j * nrhs + r];
-            B[i * nrhs + r] = ok ? s / A[i * n + i] : 0.0;
+            const int pr = (int)(piv >> (4 * col)) & 15;
+#pragma unroll
+            for (int row = col + 1; row < P; ++row)
+            {
+                const bool sw = pr == row;
+                const double t = x[col];
+                x[col] = sw ? x[row] : t;
+                x[row] = sw ? t : x[row];
+            }
+            if (good >> col & 1u)
+#pragma unroll
+                for (int row = col + 1; row < P; ++row) x[row] -= A[row][col] * x[col];
+        }
+#pragma unroll
+        for (int i = P - 1; i >= 0; --i)
+        {
+            double s = x[i];
+#pragma unroll
+            for (int j = i + 1; j < P; ++j) s -= A[i][j] * x[j];
+            x[i] = fabs(A[i][i]) > 1.0e-30 ? s / A[i][i] : 0.0;
+        }
+        B0[m] = x[0];
+    }
+    // FP32 tables: the largest coefficient takes the rounding of the node's
+    // sum, as roundCoefFP32 does on the host (same order, same operations).
+    double s64 = 0.0, s32 = 0.0, big = -1.0;
+    int smax = 0;
+#pragma unroll 1
+    for (int s = 1; s < n; ++s)
+    {
+        double ws, sx, sy, sz, b[P];
+        if (!slotAt(s, ws, sx, sy, sz)) continue;
+        basisOf<P>(sx, sy, sz, b);
+        double acc = 0.0;
+#pragma unroll
+        for (int m = 0; m < P; ++m) acc += B0[m] * b[m];
+        const double w = ws * acc;
+        cc[(size_t)s * V + k] = (T)w;
+        if (sizeof(T) == 4)
+        {
+            s64 += w;
+            s32 += (double)(T)w;
+            if (fabs(w) > big) { big = fabs(w); smax = s; }
         }
     }
-    return skipped;
+    if (sizeof(T) == 4 && big > 0.0)
+    {
+        const size_t q = (size_t)smax * V + k;
+        cc[q] = (T)((double)cc[q] + (s64 - s32));
+    }
 }
 
 // Per class: rep position (3), mesh velocity (3), wall state (7), then the
-// positions of slots 1..nsl-1 (3 each) at [c][S][3].
+// positions of slots 1..nsl-1 (3 each) at [c][S][3].  A block is of one
+// class, so its threads take one basis size.
+// Bound: FP64 issue (about 280 operations a slot in the support and 4 000 for
+// the elimination, uncontracted).  Measured, cavity3d-cube Nx 40 Nv 10
+// (1 099 classes x 1 000 nodes, FP32 tables): quadratic 14.2 ms with both
+// matrices in local memory, read and written for every slot; 3.1 ms in
+// registers (255, two blocks an SM).  Linear 1.92 -> 1.87 ms.
 template <typename T>
-__global__ void k_class_tables(ClassArgs a, int order0, const int *__restrict__ boundary,
-                               const int *__restrict__ nsl, const double *__restrict__ rep,
-                               const double *__restrict__ slotPos, T *__restrict__ table,
-                               int *__restrict__ degen)
+__global__ void __launch_bounds__(128, 2)
+k_class_tables(ClassArgs a, int order0, const int *__restrict__ boundary,
+               const int *__restrict__ nsl, const double *__restrict__ rep,
+               const double *__restrict__ slotPos, T *__restrict__ table, int *__restrict__ degen)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = blockIdx.y;
@@ -148,64 +254,13 @@ __global__ void k_class_tables(ClassArgs a, int order0, const int *__restrict__ 
     const double zf = rp[2] - (vz - rp[5]) * a.dt;
     const int n = nsl[c];
     const double *sp = slotPos + (size_t)c * a.S * 3;
-    auto offset = [&](int s, double &dx, double &dy, double &dz) {
-        dx = sp[3 * s] - xf;
-        dy = sp[3 * s + 1] - yf;
-        dz = (ndim == 3) ? sp[3 * s + 2] - zf : 0.0;
-        if (a.periodic[0]) dx = minImageD(dx, a.L[0]);
-        if (a.periodic[1]) dy = minImageD(dy, a.L[1]);
-        if (ndim == 3 && a.periodic[2]) dz = minImageD(dz, a.L[2]);
-    };
-    int P = 0;
-    double A[100];
-    for (int q = 0; q < 100; ++q) A[q] = 0.0;
-    bool any = false;
-    double b[10];
-    for (int s = 1; s < n; ++s)
+    if (ndim == 3)
     {
-        double dx, dy, dz;
-        offset(s, dx, dy, dz);
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const double ws = weightSqD(r2, a.h);
-        if (ws < 1.0e-30) continue;
-        P = basisD(dx, dy, dz, ndim, a.h, b, order);
-        for (int p1 = 0; p1 < P; ++p1)
-            for (int p2 = 0; p2 < P; ++p2) A[p1 * P + p2] += ws * b[p1] * b[p2];
-        any = true;
+        if (order >= 2) classNode<T, 10>(a, c, n, xf, yf, zf, sp, cc, k, degen);
+        else classNode<T, 4>(a, c, n, xf, yf, zf, sp, cc, k, degen);
     }
-    if (!any) { cc[k] = (T)1.0; return; }
-    double B[100];
-    for (int q = 0; q < 100; ++q) B[q] = 0.0;
-    for (int m = 0; m < P; ++m) B[m * P + m] = 1.0;
-    if (solveSkipGED(A, B, P, P) > 0) atomicAdd(degen + c, 1);
-    // FP32 tables: the largest coefficient takes the rounding of the node's
-    // sum, as roundCoefFP32 does on the host (same order, same operations).
-    double s64 = 0.0, s32 = 0.0, big = -1.0;
-    int smax = 0;
-    for (int s = 1; s < n; ++s)
-    {
-        double dx, dy, dz;
-        offset(s, dx, dy, dz);
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const double ws = weightSqD(r2, a.h);
-        if (ws < 1.0e-30) continue;
-        basisD(dx, dy, dz, ndim, a.h, b, order);
-        double acc = 0.0;
-        for (int m = 0; m < P; ++m) acc += B[m] * b[m];
-        const double c = ws * acc;
-        cc[(size_t)s * V + k] = (T)c;
-        if (sizeof(T) == 4)
-        {
-            s64 += c;
-            s32 += (double)(T)c;
-            if (fabs(c) > big) { big = fabs(c); smax = s; }
-        }
-    }
-    if (sizeof(T) == 4 && big > 0.0)
-    {
-        const size_t q = (size_t)smax * V + k;
-        cc[q] = (T)((double)cc[q] + (s64 - s32));
-    }
+    else if (order >= 2) classNode<T, 6>(a, c, n, xf, yf, zf, sp, cc, k, degen);
+    else classNode<T, 3>(a, c, n, xf, yf, zf, sp, cc, k, degen);
 }
 
 }  // namespace
