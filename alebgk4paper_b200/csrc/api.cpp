@@ -120,7 +120,8 @@ void freeBuffers(alebgk_ctx *c)
                     d.boundary, d.bodyId, d.cls, d.nslot, d.slots, d.macro[0],
                     d.macro[1], d.mood, d.flag, d.flagList, d.degList, d.massPos, d.massEnd, d.minG, d.nad, d.redPartial,
                     d.dpx, d.bodyTmp, d.bodyOut, d.stage, d.surfList, d.bodyIO, d.rankAll, d.sc,
-                    d.rowOrder};
+                    d.rowOrder, d.tiles, d.tileRest, d.tileCount, d.tileFlag,
+                    d.tileCovered};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     d = DeviceBuffers();
@@ -306,6 +307,26 @@ static int setupMarch(alebgk_ctx *c, const alebgk_cloud *cl, const CoeffTables &
     return ALEBGK_OK;
 }
 
+// The gather transport's tiles of a 3-D cloud that does not march, unless the
+// plain gather is asked for.
+static int setupTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb)
+{
+    DeviceBuffers &d = c->d;
+    const size_t N = c->sp.N;
+    c->tiled = c->sp.dim == 3 && !c->march.enabled && c->cfg.transport == 0;
+    if (!c->tiled) return ALEBGK_OK;
+    if (!d.tiles)
+    {
+        CK(dalloc(&d.tiles, tileInts((int)N)));
+        CK(dalloc(&d.tileRest, N));
+        CK(dalloc(&d.tileCount, 2));
+        CK(dalloc(&d.tileFlag, N));
+        CK(dalloc(&d.tileCovered, N));
+    }
+    CK(buildTiles(c, in, tb));
+    return ALEBGK_OK;
+}
+
 static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool withState)
 {
     if (!c || !cl) return fail(c, ALEBGK_EINVAL, "null argument");
@@ -482,6 +503,7 @@ static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool wi
                     "the streamed particle kernel needs a 3-D cloud whose rows fit in "
                     "shared memory");
     if (const int r = setupMarch(c, cl, tb)) return r;
+    if (const int r = setupTiles(c, in, tb)) return r;
     if (c->cfg.transport == 2 && (!c->march.enabled || f64))
         return fail(c, ALEBGK_EINVAL,
                     "the lattice march needs FP32 and a complete 3-D lattice cloud");
@@ -612,10 +634,13 @@ int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
     CK(cudaStreamSynchronize(c->stream));
     const bool marched = c->march.enabled;
     if (const int r = setupMarch(c, cl, tb)) return r;
-    // The step graphs hold the slot stride, the table pointers and the march's
+    const bool tiledBefore = c->tiled;
+    if (const int r = setupTiles(c, in, tb)) return r;
+    // The step graphs hold the slot stride, the table pointers, the march's
     // plan: rebuilt when any changed.
     const void *bufAfter[] = {d.coef, d.coefLin, d.slots, d.surfList, d.bodyIO};
-    bool same = std::memcmp(spBefore, &p, sizeof p) == 0 && !marched && !c->march.enabled;
+    bool same = std::memcmp(spBefore, &p, sizeof p) == 0 && !marched && !c->march.enabled &&
+                tiledBefore == c->tiled;
     for (int k = 0; k < 5 && same; ++k) same = bufBefore[k] == bufAfter[k];
     if (!same)
         for (auto &g : c->graph)

@@ -74,6 +74,10 @@ struct DeviceBuffers
     int *surfList = nullptr;           // body-surface particles (boundary, bodyId >= 0)
     int *rowOrder = nullptr;           // the row kernel's visiting order: interior
                                        // particles, then wall particles
+    // Tiles of the gather transport (tiles.cu): tiles, particles outside them,
+    // the counts of both, and the plan's two per-particle arrays.
+    int *tiles = nullptr, *tileRest = nullptr, *tileCount = nullptr;
+    int *tileFlag = nullptr, *tileCovered = nullptr;
     double *bodyIO = nullptr;          // body-step staging: kBodyIOHead + 13 per surface particle
     double *rankAll = nullptr;         // multi-process slab: every rank's 4 combine words
     int rankAllCap = 0;                // ranks rankAll holds
@@ -134,6 +138,7 @@ struct alebgk_ctx
     int cur = 0;                 // buffer holding the current h and macros
     bool uploaded = false;
     int ncls = 0;
+    bool tiled = false;          // the gather transport runs by tiles (tiles.cu)
     int degenerateParticles = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     // Launch shapes of the general kernels (alebgk_set_launch / autotune).
@@ -169,6 +174,14 @@ struct alebgk_ctx
 };
 
 namespace alebgk {
+
+// Tiles of the gather transport (tiles.cu): the plan of the uploaded cloud,
+// the int words of the tile list of N particles, and the transport of the tiles.
+struct CoeffInput;
+struct CoeffTables;
+cudaError_t buildTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb);
+size_t tileInts(int N);
+cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st);
 
 // Launch wrappers (step.cu).
 cudaError_t prepareKernels(alebgk_ctx *c);

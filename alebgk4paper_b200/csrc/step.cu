@@ -228,11 +228,12 @@ __device__ __forceinline__ void k_transport_body(const T *__restrict__ f, T *__r
             const T *__restrict__ coef, const int *__restrict__ cls,
             const int *__restrict__ nslot, const int *__restrict__ slots,
             int S, int N, int V, int L, int ldf, const StepScalars *__restrict__ sc, int chunk,
-            int tile)
+            int tile, const int *__restrict__ list, const int *__restrict__ count)
 {
     const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int i = tile * nw + warp;
-    if (i >= N) return;
+    int i = tile * nw + warp;
+    if (i >= (list ? __ldg(count) : N)) return;
+    if (list) i = __ldg(list + i);
     const T scale = T(sc->scale);
     const int nch = transportChunks(V);
     if (L == 2)
@@ -243,15 +244,18 @@ __device__ __forceinline__ void k_transport_body(const T *__restrict__ f, T *__r
                            threadIdx.x & 31);
 }
 
-// Grid (velocity chunks, particle tiles of blockDim.x / 32).
+// Grid (velocity chunks, particle tiles of blockDim.x / 32); with a list,
+// its count particles instead of all N.
 template <typename T>
 __global__ void __launch_bounds__(kNT)
 k_transport(const T *__restrict__ f, T *__restrict__ g,
             const T *__restrict__ coef, const int *__restrict__ cls,
             const int *__restrict__ nslot, const int *__restrict__ slots,
-            int S, int N, int V, int L, int ldf, const StepScalars *__restrict__ sc)
+            int S, int N, int V, int L, int ldf, const StepScalars *__restrict__ sc,
+            const int *__restrict__ list, const int *__restrict__ count)
 {
-    k_transport_body(f, g, coef, cls, nslot, slots, S, N, V, L, ldf, sc, blockIdx.x, blockIdx.y);
+    k_transport_body(f, g, coef, cls, nslot, slots, S, N, V, L, ldf, sc, blockIdx.x, blockIdx.y,
+                     list, count);
 }
 
 // Walks the nodes k = lane, lane + 32, ... of a particle row and keeps the
@@ -2200,6 +2204,29 @@ static void launchParticleStream(alebgk_ctx *c, const ParticleArgs<T> &pa, const
     k_particle_stream<T><<<c->pStreamBlocks, kNT, c->pStreamSmem, st>>>(pa, p, c->pStreamWpb);
 }
 
+// The gather transport as its own kernel: by tiles and the particles outside
+// them where the cloud has tiles, else every particle alone.
+template <typename T>
+static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
+{
+    const StepParams &p = c->sp;
+    DeviceBuffers &d = c->d;
+    const T *fa = static_cast<const T *>(d.f[from]);
+    T *fb = static_cast<T *>(d.f[1 - from]);
+    const int tt = c->tune.transportThreads > 0 ? c->tune.transportThreads : kNT;
+    const dim3 gt(transportChunks(p.V), (p.N + tt / 32 - 1) / (tt / 32));
+    if (c->tiled)
+    {
+        const cudaError_t e = launchTiles(c, fa, fb, st);
+        if (e != cudaSuccess) return e;
+    }
+    k_transport<T><<<gt, tt, 0, st>>>(fa, fb, static_cast<const T *>(d.coef), d.cls, d.nslot,
+                                      d.slots, p.S, p.N, p.V, p.L, p.ldf, d.sc,
+                                      c->tiled ? d.tileRest : nullptr,
+                                      c->tiled ? d.tileCount + 1 : nullptr);
+    return cudaGetLastError();
+}
+
 // Launches one step.  With ev != nullptr an event is recorded before each
 // launch and after the last one (ev[0..ALEBGK_NSTAGES]), in launch order:
 // step_begin, transport, particle, redo, sigma, fixup, mass_sum, scale_mood,
@@ -2259,11 +2286,8 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
     }
     else if (!fused)
     {
-        const int tt = c->tune.transportThreads > 0 ? c->tune.transportThreads : kNT;
-        dim3 gt(transportChunks(p.V), (p.N + tt / 32 - 1) / (tt / 32));
-        k_transport<T><<<gt, tt, 0, st>>>(fa, fb, static_cast<const T *>(d.coef),
-                                           d.cls, d.nslot, d.slots, p.S, p.N, p.V, p.L,
-                                           p.ldf, d.sc);
+        const cudaError_t e = launchGather<T>(c, from, st);
+        if (e != cudaSuccess) return e;
     }
     mark();
     if (fork) cudaStreamWaitEvent(st, c->evJoin, 0);
@@ -3089,11 +3113,8 @@ static cudaError_t slabSegT(alebgk_ctx *c, int from, int seg, cudaStream_t st)
         }
         else if (!fused)
         {
-            const int tt = c->tune.transportThreads > 0 ? c->tune.transportThreads : kNT;
-            dim3 gt(transportChunks(p.V), (p.N + tt / 32 - 1) / (tt / 32));
-            k_transport<T><<<gt, tt, 0, st>>>(fa, fb, static_cast<const T *>(d.coef), d.cls,
-                                               d.nslot, d.slots, p.S, p.N, p.V, p.L, p.ldf,
-                                               d.sc);
+            const cudaError_t e = launchGather<T>(c, from, st);
+            if (e != cudaSuccess) return e;
         }
         const int wmax = particleWarpsPerBlock(p, sizeof(T));
         const int wpb = (c->tune.particleWarps > 0 && c->tune.particleWarps < wmax)

@@ -1,0 +1,385 @@
+// tiles.cu -- coefficient-gather transport of a 3-D cloud that is a lattice
+// for the most part (a cavity with bodies in it): the particles inside it go
+// in tiles of 4 x 2 lattice neighbours, the rest through the plain gather.
+//
+// A tile is eight particles of one full stencil class (80 neighbours at the
+// lattice offsets |o|^2 <= 6) whose neighbours, by their own slot lists, lie
+// in rows of consecutive particle indices: row (dz, y), y = -2..3, holds the
+// x = -2..5 around the tile.  The plan checks every slot of every member on
+// the device, so holes, surfaces and cut rows need no rules: a tile that does
+// not hold leaves its particles to the gather.
+//
+// Transport: one warp per tile and chunk of velocities.  Each neighbour value
+// is loaded once for the tile and each coefficient once per row pair, 180 +
+// 160 loads for the 640 FMAs of eight particles (the gather loads a value and
+// a coefficient for every FMA and is bound by L1 throughput).  Every particle
+// sums its slots in slot order, as the gather does; the full class has no
+// coefficient of its own value.
+// Measured, cavity3d-cube Nx 40 Nv 10 FP32: transport 1.53 ms by the gather
+// alone, 0.756 ms with tiles; the particles outside them (walls, the layers
+// beside them, around the body) take about half of that.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <utility>
+#include <vector>
+
+#include "coeffs.h"
+#include "ctx.h"
+
+namespace alebgk {
+
+namespace {
+
+// A tile: class, its two first members, then the index of x = 0 of each row
+// (dz + 2) * 6 + y + 2 (rows outside every member's stencil unused).
+constexpr int kTileInts = 33;
+
+__host__ __device__ constexpr int off3(int dx, int dy, int dz)
+{
+    int n = 0;
+    for (int z = -2; z <= 2; ++z)
+        for (int y = -2; y <= 2; ++y)
+            for (int x = -2; x <= 2; ++x)
+            {
+                if (x * x + y * y + z * z > 6) continue;
+                if (x == dx && y == dy && z == dz) return n;
+                ++n;
+            }
+    return -1;
+}
+// Slot of an offset in a full class: the self first, then template order.
+__host__ __device__ constexpr int slot3(int dx, int dy, int dz)
+{
+    const int o = off3(dx, dy, dz), self = off3(0, 0, 0);
+    return o < 0 ? -1 : (o == self ? 0 : (o < self ? o + 1 : o));
+}
+static_assert(slot3(1, 1, 2) == 80 && slot3(-1, -1, -2) == 1, "80 neighbours");
+
+struct Tmpl3
+{
+    signed char d[81][3];     // offset of each slot
+    signed char slot[125];    // slot of (dz + 2) * 25 + (dy + 2) * 5 + dx + 2
+};
+
+Tmpl3 makeTmpl3()
+{
+    Tmpl3 t{};
+    for (int z = -2; z <= 2; ++z)
+        for (int y = -2; y <= 2; ++y)
+            for (int x = -2; x <= 2; ++x)
+            {
+                const int s = slot3(x, y, z);
+                t.slot[(z + 2) * 25 + (y + 2) * 5 + x + 2] = (signed char)s;
+                if (s >= 0) { t.d[s][0] = (signed char)x; t.d[s][1] = (signed char)y; t.d[s][2] = (signed char)z; }
+            }
+    return t;
+}
+
+struct TileGrid
+{
+    double x0, y0, hx, hy;
+};
+
+__device__ __forceinline__ int rowSlot(const Tmpl3 &t, int dy, int dz)
+{
+    if (dy < -2 || dy > 2) return -1;
+    return t.slot[(dz + 2) * 25 + (dy + 2) * 5 + 2];
+}
+
+// Index of x = 0 of row (dz, y) of the tile with first members i and j.
+__device__ __forceinline__ int tileRow(const Tmpl3 &t, const int *slots, int S, int i, int j, int y,
+                                       int dz)
+{
+    const int s = rowSlot(t, y, dz);
+    if (s >= 0) return slots[(size_t)i * S + s];
+    const int q = rowSlot(t, y - 1, dz);
+    return q >= 0 ? slots[(size_t)j * S + q] : -1;
+}
+
+// One warp per particle: whether a tile starts there; marks its members.
+__global__ void k_tile_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__restrict__ pos,
+                            const int *__restrict__ cls, const int *__restrict__ slots,
+                            const int *__restrict__ full, int *__restrict__ flag,
+                            int *__restrict__ covered)
+{
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= N) return;
+    const int c = cls[i];
+    bool ok = full[c] != 0 && i + 3 < N;
+    int j = 0;
+    if (ok)
+    {
+        const long long ix = llround((pos[3 * (size_t)i] - g.x0) / g.hx);
+        const long long iy = llround((pos[3 * (size_t)i + 1] - g.y0) / g.hy);
+        ok = ((ix + 2) & 3) == 0 && (iy & 1) == 0;
+    }
+    if (ok)
+    {
+        j = slots[(size_t)i * S + t.slot[2 * 25 + 3 * 5 + 2]];      // (0, 1, 0)
+        ok = j + 3 < N;
+        for (int m = 0; m < 4 && ok; ++m) ok = cls[i + m] == c && cls[j + m] == c;
+    }
+    if (ok)
+        for (int q = lane; q < 8 * 80; q += 32)
+        {
+            const int m = q / 80, s = 1 + q % 80, b = m >> 2, x = m & 3;
+            const int mem = b ? j + x : i + x;
+            const int y = t.d[s][1] + b, dz = t.d[s][2];
+            const int base = y == 0 && dz == 0 ? i : (y == 1 && dz == 0 ? j
+                                                                        : tileRow(t, slots, S, i, j, y, dz));
+            ok = ok && slots[(size_t)mem * S + s] == base + x + t.d[s][0];
+        }
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) flag[i] = ok;
+    if (ok && lane < 8) covered[lane >> 2 ? j + (lane & 3) : i + (lane & 3)] = 1;
+}
+
+// One block: places of the tiles and of the particles outside them, in
+// particle order, and their counts.
+__global__ void __launch_bounds__(1024)
+k_tile_scan(int N, int *flag, int *covered, int *count)
+{
+    __shared__ int sh[2][1024];
+    const int t = threadIdx.x, per = (N + 1023) / 1024;
+    const int a = min(t * per, N), b = min(a + per, N);
+    int nt = 0, nr = 0;
+    for (int i = a; i < b; ++i)
+    {
+        nt += flag[i];
+        nr += !covered[i];
+    }
+    sh[0][t] = nt;
+    sh[1][t] = nr;
+    __syncthreads();
+    for (int o = 1; o < 1024; o <<= 1)
+    {
+        const int x = t >= o ? sh[0][t - o] : 0, y = t >= o ? sh[1][t - o] : 0;
+        __syncthreads();
+        sh[0][t] += x;
+        sh[1][t] += y;
+        __syncthreads();
+    }
+    int pt = sh[0][t] - nt, pr = sh[1][t] - nr;
+    for (int i = a; i < b; ++i)
+    {
+        flag[i] = flag[i] ? pt++ : -1;
+        covered[i] = covered[i] ? -1 : pr++;
+    }
+    if (t == 1023)
+    {
+        count[0] = sh[0][1023];
+        count[1] = sh[1][1023];
+    }
+}
+
+__global__ void k_tile_write(Tmpl3 t, int N, int S, const int *__restrict__ cls,
+                             const int *__restrict__ slots, const int *__restrict__ flag,
+                             const int *__restrict__ covered, int *__restrict__ tiles,
+                             int *__restrict__ rest)
+{
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= N) return;
+    if (lane == 0 && covered[i] >= 0) rest[covered[i]] = i;
+    if (flag[i] < 0) return;
+    int *o = tiles + (size_t)flag[i] * kTileInts;
+    const int j = slots[(size_t)i * S + t.slot[2 * 25 + 3 * 5 + 2]];
+    if (lane < 30)
+    {
+        const int dz = lane / 6 - 2, y = lane % 6 - 2;
+        o[3 + lane] = dz == 0 && y == 0 ? i : (dz == 0 && y == 1 ? j : tileRow(t, slots, S, i, j, y, dz));
+    }
+    if (lane == 0)
+    {
+        o[0] = cls[i];
+        o[1] = i;
+        o[2] = j;
+    }
+}
+
+template <int... I, typename F>
+__device__ __forceinline__ void unroll3Impl(std::integer_sequence<int, I...>, F &&f)
+{
+    (f(std::integral_constant<int, I>{}), ...);
+}
+template <int M, typename F>
+__device__ __forceinline__ void unroll3(F &&f)
+{
+    unroll3Impl(std::make_integer_sequence<int, M>{}, f);
+}
+
+// The velocities of one lane: two of FP32 (packed FMAs), or one.
+template <typename T, int VPL> struct Vel;
+template <> struct Vel<float, 2>
+{
+    typedef float2 V;
+    static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return __ffma2_rn(a, b, c); }
+    static __device__ __forceinline__ V mul(V a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
+};
+template <typename T> struct Vel<T, 1>
+{
+    typedef T V;
+    static __device__ __forceinline__ V zero() { return T(0); }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return ::fma(a, b, c); }
+    static __device__ __forceinline__ V mul(V a, T s) { return a * s; }
+};
+
+// Grid (velocity chunks, blocks of eight tiles).
+template <typename T, int VPL>
+__global__ void __launch_bounds__(256, 2)
+k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restrict__ coef,
+                  const int *__restrict__ tiles, const int *__restrict__ count, int S, int V, int ldf,
+                  const StepScalars *__restrict__ sc)
+{
+    typedef Vel<T, VPL> L;
+    typedef typename L::V VT;
+    const int tile = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (tile >= __ldg(count)) return;
+    const int k = (blockIdx.x * 32 + lane) * VPL;
+    if (k >= V) return;
+    const int *tl = tiles + (size_t)tile * kTileInts;
+    const T *cc = coef + (size_t)__ldg(tl) * S * V + k;
+    const T *fk = f + k;
+    auto coefAt = [&](int s) { return __ldg(reinterpret_cast<const VT *>(cc + (size_t)s * V)); };
+    VT acc[2][4];
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[b][x] = L::zero();
+    unroll3<30>([&](auto R) {
+        constexpr int r = decltype(R)::value, dz = r / 6 - 2, y = r % 6 - 2;
+        // member row 0 meets this row at offset dy = y, member row 1 at y - 1
+        constexpr bool m0 = slot3(0, y, dz) >= 0, m1 = slot3(0, y - 1, dz) >= 0;
+        if constexpr (m0 || m1)
+        {
+            const T *row = fk + (size_t)__ldg(tl + 3 + r) * ldf;
+            VT v[8];
+            unroll3<8>([&](auto X) {
+                constexpr int x = decltype(X)::value - 2, z = decltype(R)::value / 6 - 2;
+                constexpr int w = decltype(R)::value % 6 - 2;
+                if constexpr ((x > -2 && x < 5) || slot3(2, w, z) >= 0 || slot3(2, w - 1, z) >= 0)
+                    v[x + 2] = __ldg(reinterpret_cast<const VT *>(row + (long long)x * ldf));
+            });
+            unroll3<10>([&](auto D) {
+                constexpr int bb = decltype(D)::value / 5, dx = decltype(D)::value % 5 - 2;
+                constexpr int s = slot3(dx, decltype(R)::value % 6 - 2 - bb,
+                                        decltype(R)::value / 6 - 2);
+                if constexpr (s > 0)
+                {
+                    const VT c = coefAt(s);
+                    unroll3<4>([&](auto M) {
+                        constexpr int m = decltype(M)::value;
+                        constexpr int bm = decltype(D)::value / 5, at = m + decltype(D)::value % 5;
+                        acc[bm][m] = L::fma(c, v[at], acc[bm][m]);
+                    });
+                }
+            });
+        }
+    });
+    const T scale = T(sc->scale);
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+    {
+        T *o = g + (size_t)__ldg(tl + 1 + b) * ldf + k;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+            *reinterpret_cast<VT *>(o + (size_t)x * ldf) = L::mul(acc[b][x], scale);
+    }
+}
+
+}  // namespace
+
+// Classes whose slots are the whole template in order (full classes), by
+// their representatives; the lattice spacing comes from the first of them.
+static bool fullClasses(const CoeffInput &in, const CoeffTables &tb, std::vector<int> &full,
+                        TileGrid &g)
+{
+    static const Tmpl3 t = makeTmpl3();
+    full.assign(tb.ncls, 0);
+    bool any = false;
+    if (tb.S < 81) return false;
+    for (int c = 0; c < tb.ncls; ++c)
+    {
+        const int r = tb.rep[c];
+        const bool packed = tb.slots.empty();
+        const int ns = packed ? tb.repNslot[c] : tb.nslot[r];
+        if (ns != 81 || in.boundary[r]) continue;
+        const int *sl = packed ? &tb.repSlots[(size_t)c * tb.S] : &tb.slots[(size_t)r * tb.S];
+        const double *p = in.xyz + 3 * (size_t)r;
+        const double *px = in.xyz + 3 * (size_t)sl[slot3(1, 0, 0)];
+        const double *py = in.xyz + 3 * (size_t)sl[slot3(0, 1, 0)];
+        const double *pz = in.xyz + 3 * (size_t)sl[slot3(0, 0, 1)];
+        const double h[3] = {px[0] - p[0], py[1] - p[1], pz[2] - p[2]};
+        bool ok = h[0] > 0 && h[1] > 0 && h[2] > 0;
+        for (int s = 1; s < 81 && ok; ++s)
+        {
+            const double *q = in.xyz + 3 * (size_t)sl[s];
+            for (int a = 0; a < 3 && ok; ++a)
+                ok = std::fabs((q[a] - p[a]) / h[a] - t.d[s][a]) < 1e-6;
+        }
+        if (!ok) continue;
+        full[c] = 1;
+        if (!any) g = TileGrid{in.xyz[0], in.xyz[1], h[0], h[1]};
+        any = true;
+    }
+    return any;
+}
+
+// Plans the tiles of the uploaded cloud (classes and slot lists on the
+// device); c->d.tileCount holds their number and that of the rest.
+cudaError_t buildTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb)
+{
+    static const Tmpl3 t = makeTmpl3();
+    DeviceBuffers &d = c->d;
+    const int N = c->sp.N;
+    std::vector<int> full;
+    TileGrid g{0, 0, 1, 1};
+    fullClasses(in, tb, full, g);
+    int *dFull = nullptr;
+    cudaError_t e = cudaMalloc(&dFull, 4 * std::max<size_t>(full.size(), 1));
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(dFull, full.data(), 4 * full.size(), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d.tileCovered, 0, 4 * (size_t)N, c->stream);
+    if (e == cudaSuccess)
+    {
+        const int blocks = (int)(((long long)N * 32 + 255) / 256);
+        k_tile_mark<<<blocks, 256, 0, c->stream>>>(t, g, N, tb.S, d.pos, d.cls, d.slots, dFull,
+                                                   d.tileFlag, d.tileCovered);
+        k_tile_scan<<<1, 1024, 0, c->stream>>>(N, d.tileFlag, d.tileCovered, d.tileCount);
+        k_tile_write<<<blocks, 256, 0, c->stream>>>(t, N, tb.S, d.cls, d.slots, d.tileFlag,
+                                                    d.tileCovered, d.tiles, d.tileRest);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (dFull) cudaFree(dFull);
+    return e;
+}
+
+size_t tileInts(int N) { return (size_t)(N / 8 + 1) * kTileInts; }
+
+cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st)
+{
+    const StepParams &p = c->sp;
+    const DeviceBuffers &d = c->d;
+    // as many blocks as there could be tiles: the plan's counts stay on the
+    // device, and a refresh of the geometry changes no launch
+    const int by = (p.N / 8 + 7) / 8;
+    if (by == 0) return cudaSuccess;
+    if (c->cfg.precision == 64)
+        k_transport_tiles<double, 1><<<dim3((p.V + 31) / 32, by), 256, 0, st>>>(
+            static_cast<const double *>(f), static_cast<double *>(g),
+            static_cast<const double *>(d.coef), d.tiles, d.tileCount, p.S, p.V, p.ldf, d.sc);
+    else if (p.V % 2 == 0)
+        k_transport_tiles<float, 2><<<dim3((p.V + 63) / 64, by), 256, 0, st>>>(
+            static_cast<const float *>(f), static_cast<float *>(g),
+            static_cast<const float *>(d.coef), d.tiles, d.tileCount, p.S, p.V, p.ldf, d.sc);
+    else
+        k_transport_tiles<float, 1><<<dim3((p.V + 31) / 32, by), 256, 0, st>>>(
+            static_cast<const float *>(f), static_cast<float *>(g),
+            static_cast<const float *>(d.coef), d.tiles, d.tileCount, p.S, p.V, p.ldf, d.sc);
+    return cudaGetLastError();
+}
+
+}  // namespace alebgk

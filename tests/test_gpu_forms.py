@@ -1,0 +1,38 @@
+"""The forms that a step and the network choose by size against the general ones, at the edges of their ranges."""
+import numpy as np
+import pytest
+
+import alebgk4paper_b200 as ab
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.parametrize("Nx,Nv", [(3, 4), (7, 5), (9, 8), (12, 10), (17, 6)])
+def test_fp64_march_equals_gather(gpu, Nx, Nv):
+    """Tiles and segments with remainders, an odd row length, a lattice smaller than a tile.  Both sum the same
+    80 products in another order: eps64 times the stencil's sum of |c| (at most 5) times sqrt(80), each step."""
+    c = ab.Case("cavity3d", Nx, Nv, -1.0, 2)
+    a, b = ab.Solver(c, precision=64), ab.Solver(c, precision=64, transport=1)
+    assert a.counters()["transport_kernel"] == 2 and b.counters()["transport_kernel"] == 1
+    a.cudaStep(3), b.cudaStep(3)
+    (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
+    assert _rel(ga, gb) < 3 * 5 * 9 * 1.2e-16
+    assert _rel(ma[:, 0], mb[:, 0]) < 3 * 5 * 9 * 1.2e-16
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("name,Nx,Nv", [("cavity3d-cube", 12, 5), ("cavity3d-cube", 17, 6), ("cavity3d-sphere", 21, 4),
+                                        ("cavity3d-cube", 24, 8)])
+def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
+    """Odd rows (one velocity a lane), partial chunks, lattices with partial tiles, bodies in the middle: every
+    particle sums its slots in the same order, so the states are the same bits."""
+    c = ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True)
+    a, b = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision, transport=1)
+    a.cudaStep(3), b.cudaStep(3)
+    (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
+    np.testing.assert_array_equal(ga, gb)
+    np.testing.assert_array_equal(ma, mb)
