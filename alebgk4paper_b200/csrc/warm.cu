@@ -19,6 +19,7 @@
 // to BF16 between layers.  Training keeps FP32 master weights and Adam state.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -33,7 +34,9 @@ namespace alebgk {
 
 namespace {
 
-constexpr int kTile = 128;     // points per tile = MMA M = threads per block
+constexpr int kTile = 128;     // points per tile = MMA M
+constexpr int kGroup = 256;    // threads per tile: two per point (each half of the columns)
+constexpr int kFwdGroups = 3;  // most tiles in flight in a forward block
 constexpr int kIn = 64;        // features
 constexpr int kHid = 128;      // hidden width
 constexpr int kOut = 16;       // output rows of W4 (9 used)
@@ -79,28 +82,45 @@ struct LossWeights
 };
 
 // ---------------------------------------------------------------------------
-// Features of one point: (x, y) in [0, 1]^2, a = scaled log density,
-// b = scaled lid Mach number.
+// Half of the features of one point: (x, y) in [0, 1]^2, a = scaled log
+// density, b = scaled lid Mach number.  Feature j: 2x - 1, 2y - 1, a, b, then
+// for k = 1..12 sin/cos(k pi x), sin/cos(k pi y), then zeros; half h holds
+// features 32 h .. 32 h + 31.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void features(float4 q, float *f)
+__device__ __forceinline__ void featuresHalf(float4 q, int half, float *f)
 {
-    f[0] = 2.f * q.x - 1.f;
-    f[1] = 2.f * q.y - 1.f;
-    f[2] = q.z;
-    f[3] = q.w;
+    const int k0 = half * (kIn / 8);
 #pragma unroll
-    for (int k = 1; k <= kFourier; ++k)
+    for (int j = 0; j < kIn / 8; ++j)
     {
-        float sx, cx, sy, cy;
-        sincospif((float)k * q.x, &sx, &cx);
-        sincospif((float)k * q.y, &sy, &cy);
-        f[4 * k + 0] = sx;
-        f[4 * k + 1] = cx;
-        f[4 * k + 2] = sy;
-        f[4 * k + 3] = cy;
+        const int k = k0 + j;
+        float sx = 0.f, cx = 0.f, sy = 0.f, cy = 0.f;
+        if (k == 0)
+        {
+            sx = 2.f * q.x - 1.f;
+            cx = 2.f * q.y - 1.f;
+            sy = q.z;
+            cy = q.w;
+        }
+        else if (k <= kFourier)
+        {
+            sincospif((float)k * q.x, &sx, &cx);
+            sincospif((float)k * q.y, &sy, &cy);
+        }
+        f[4 * j + 0] = sx;
+        f[4 * j + 1] = cx;
+        f[4 * j + 2] = sy;
+        f[4 * j + 3] = cy;
     }
-#pragma unroll
-    for (int j = 4 + 4 * kFourier; j < kIn; ++j) f[j] = 0.f;
+}
+
+// tanh x = 1 - 2 / (1 + e^2x) in FP32 with the fast exponential and divide:
+// absolute error below 3e-7, against the 2e-3 relative of the BF16 rounding
+// that follows every use.  tanhf, with its two branches, was half of the
+// forward kernel's instructions.
+__device__ __forceinline__ float tanhFast(float x)
+{
+    return 1.f - __fdividef(2.f, 1.f + __expf(2.f * x));
 }
 
 // Writes 16 consecutive values (k0 .. k0+15, k0 a multiple of 16) of row r of
@@ -121,18 +141,37 @@ __device__ __forceinline__ void storeBf16(uint8_t *p, float x)
     *reinterpret_cast<uint16_t *>(p) = (uint16_t)(packBf16(x, 0.f) & 0xFFFFu);
 }
 
-// Bounded wait, then a block-wide vote so that every thread takes the same
+// Barrier and vote among the threads of one tile's group.
+__device__ __forceinline__ void groupSync(int g)
+{
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(g + 1), "r"(kGroup) : "memory");
+}
+
+__device__ __forceinline__ bool groupOr(int g, bool v)
+{
+    int out;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n"
+        " barrier.cta.red.or.pred q, %2, %3, p;\n selp.b32 %0, 1, 0, q;\n}\n"
+        : "=r"(out)
+        : "r"(v ? 1 : 0), "r"(g + 1), "r"(kGroup)
+        : "memory");
+    return out != 0;
+}
+
+// Bounded wait, then a vote of the group so that every thread takes the same
 // branch when a wait gives up.
-__device__ __forceinline__ bool waitAll(uint64_t *bar, uint32_t parity, bool &dead)
+__device__ __forceinline__ bool waitAll(uint64_t *bar, uint32_t parity, bool &dead, int g = 0)
 {
     mbarWait(bar, parity, dead);
-    dead = __syncthreads_or(dead ? 1 : 0) != 0;
+    dead = groupOr(g, dead);
     return !dead;
 }
 
 __device__ __forceinline__ void setErr(int *err, int bit)
 {
-    if (err) atomicOr(err, bit);
+    // (host memory that the device maps: written on an error only)
+    if (err) *(volatile int *)err = bit;
 }
 
 // Issues the MMAs of one layer product D = A * B^T over K, one thread.
@@ -144,16 +183,30 @@ __device__ __forceinline__ void mmaChain(uint32_t d, uint32_t a, int aRows, uint
 }
 
 // ---------------------------------------------------------------------------
-// Forward.  One CTA of 128 threads per tile (persistent over tiles); thread t
-// owns point t of the tile = row t of every activation and TMEM lane t.
-// With yImg, also writes each tile's Y_l^T images for the backward pass.
+// Forward.  A block holds the weights and one to kFwdGroups groups of 256
+// threads, each with a tile of its own (activation image, 128 columns of
+// tensor memory), persistent over tiles; threads t and t + 128 of a group own
+// point t of the tile = row t of every activation and TMEM lane t, half of
+// the columns each.  With yImg, also writes each tile's Y_l^T images for the
+// backward pass.
+// Bound: a tile is a chain of five MMAs, each with an epilogue (tanh, BF16,
+// shared memory) of far more issue slots than the MMA's time, so what counts
+// is epilogue instructions and that one tile's MMA and barriers run under
+// the others' epilogues.  Measured, one call for 73 728 points (576 tiles):
+// 84 us with one tile a block, 128 threads a tile and tanhf; 52 us in this
+// form, 31 us of which are the call and one tile's chain (100 points take
+// them too).  Error of the outputs against FP64: 5.6e-3 in both, that of the
+// BF16 operands.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kFwdAct = kWImgBytes;                 // activation image, 32 KB
-constexpr uint32_t kFwdBias = kFwdAct + 32768;           // 528 floats
-constexpr uint32_t kFwdBar = kFwdBias + 2176;            // 2 mbarriers + TMEM slot
-constexpr uint32_t kFwdSmem = kFwdBar + 64 + 1024;       // + alignment slack
+constexpr uint32_t kFwdAct = kWImgBytes;                 // activation images, 32 KB each
+constexpr uint32_t fwdBias(int groups) { return kFwdAct + 32768u * groups; }   // 528 floats
+constexpr uint32_t fwdSmem(int groups)
+{
+    return fwdBias(groups) + 2176 + 64 + 1024;           // mbarriers, TMEM slot, alignment slack
+}
+static_assert(fwdSmem(kFwdGroups) <= 227 * 1024, "the groups' images fit");
 
-__global__ void __launch_bounds__(kTile, 1)
+__global__ void __launch_bounds__(kGroup * kFwdGroups, 1)
 k_mlp_forward(const uint8_t *__restrict__ wImg, const float *__restrict__ params,
               const float4 *__restrict__ pts, const int *__restrict__ idx, int n,
               float *__restrict__ out, uint8_t *__restrict__ yImg, int *err)
@@ -161,95 +214,122 @@ k_mlp_forward(const uint8_t *__restrict__ wImg, const float *__restrict__ params
     extern __shared__ uint8_t smemRaw[];
     uint8_t *sm = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
-    uint8_t *act = sm + kFwdAct;
-    float *bias = reinterpret_cast<float *>(sm + kFwdBias);
-    uint64_t *barW = reinterpret_cast<uint64_t *>(sm + kFwdBar);
-    uint64_t *barM = barW + 1;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(barW + 2);
-    const int t = threadIdx.x, warp = t >> 5;
+    const int groups = blockDim.x / kGroup, g = threadIdx.x / kGroup;
+    const int t = threadIdx.x & (kTile - 1), half = (threadIdx.x / kTile) & 1;
+    const int warp = threadIdx.x >> 5;
+    const bool lead = (threadIdx.x & (kGroup - 1)) == 0;
+    uint8_t *act = sm + kFwdAct + 32768u * g;
+    float *bias = reinterpret_cast<float *>(sm + kFwdAct + 32768u * groups);
+    uint64_t *barW = reinterpret_cast<uint64_t *>(sm + kFwdAct + 32768u * groups + 2176);
+    uint64_t *barM = barW + 1 + g;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(barW + 1 + kFwdGroups);
+    const uint32_t tcols = groups == 1 ? 128 : (groups == 2 ? 256 : 512);
     bool dead = false;
 
-    if (t == 0)
+    if (threadIdx.x == 0)
     {
-        mbarInit(barW, 1);
-        mbarInit(barM, 1);
+        for (int i = 0; i < 1 + groups; ++i) mbarInit(barW + i, 1);
         mbarInitFence();
     }
-    if (warp == 0) tmemAlloc(tslot, 128);
-    for (int j = t; j < 4 * kHid + kOut; j += kTile) bias[j] = params[kWEnd + j];
+    if (warp == 0) tmemAlloc(tslot, tcols);
+    for (int j = threadIdx.x; j < 4 * kHid + kOut; j += blockDim.x) bias[j] = params[kWEnd + j];
     tmemFenceBefore();
     __syncthreads();
-    if (t == 0)
+    if (threadIdx.x == 0)
     {
         mbarExpectTx(barW, kWImgBytes);
         for (uint32_t o = 0; o < kWImgBytes; o += 16384)
             bulkLoad(sm + o, wImg + o, min(16384u, kWImgBytes - o), barW);
     }
-    waitAll(barW, 0, dead);
     tmemFenceAfter();
-    const uint32_t tmem = *tslot;
-    const uint32_t tlane = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t tbase = *tslot, tmem = tbase + 128u * g;
+    const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t actS = smemAddr(act), wS = smemAddr(sm);
     uint32_t phase = 0;
+    bool loaded = false;
 
     const int ntiles = (n + kTile - 1) / kTile;
-    for (int tile = blockIdx.x; tile < ntiles && !dead; tile += gridDim.x)
+    for (int tile = blockIdx.x + gridDim.x * g; tile < ntiles && !dead;
+         tile += gridDim.x * groups)
     {
         const int p = tile * kTile + t;
         const bool valid = p < n;
         uint8_t *yt = yImg ? yImg + (size_t)tile * kYTileBytes : nullptr;
         {
-            float f[kIn];
+            float f[kIn / 2];
             if (valid)
-                features(pts[idx ? idx[p] : p], f);
+                featuresHalf(pts[idx ? idx[p] : p], half, f);
             else
-                for (int j = 0; j < kIn; ++j) f[j] = 0.f;
 #pragma unroll
-            for (int k0 = 0; k0 < kIn; k0 += 16) storeRow16(act, kTile, t, k0, f + k0);
+                for (int j = 0; j < kIn / 2; ++j) f[j] = 0.f;
+            const int j0 = half * (kIn / 2);
+#pragma unroll
+            for (int k0 = 0; k0 < kIn / 2; k0 += 16) storeRow16(act, kTile, t, j0 + k0, f + k0);
             if (yt)
             {
 #pragma unroll
-                for (int j = 0; j < kIn; ++j)
-                    storeBf16(yt + yImgOff(0) + swzOffset(j, t, kIn), f[j]);
+                for (int j = 0; j < kIn / 2; ++j)
+                    storeBf16(yt + yImgOff(0) + swzOffset(j0 + j, t, kIn), f[j]);
             }
         }
         fenceProxyAsync();
         tmemFenceBefore();
-        __syncthreads();
+        groupSync(g);
+        if (!loaded)
+        {
+            // the weights, loaded under the first tile's features
+            if (!waitAll(barW, 0, dead, g)) break;
+            loaded = true;
+        }
 #pragma unroll 1
         for (int l = 0; l < 5; ++l)
         {
             const int K = layerIn(l), N = layerOut(l);
-            if (t == 0)
+            if (lead)
             {
                 tmemFenceAfter();
                 mmaChain(tmem, actS, kTile, wS + wImgOff(l), N, K, ummaIdescBf16(kTile, N));
                 ummaCommit(barM);
             }
-            if (!waitAll(barM, phase, dead)) break;
+            if (!waitAll(barM, phase, dead, g)) break;
             phase ^= 1;
             tmemFenceAfter();
-            for (int c0 = 0; c0 < N; c0 += 16)
+            if (l < 4)
             {
-                float v[16];
-                tmemLoad16(tlane + c0, v);
-                const float *bl = bias + l * kHid + c0;
-                if (l < 4)
+#pragma unroll 1
+                for (int c0 = half * (kHid / 2); c0 < (half + 1) * (kHid / 2); c0 += 32)
                 {
+                    float v[32];
+                    tmemLoad32(tlane + c0, v);
+                    const float4 *bl = reinterpret_cast<const float4 *>(bias + l * kHid + c0);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = tanhf(v[i] + bl[i]);
+                    for (int i = 0; i < 8; ++i)
+                    {
+                        const float4 b4 = bl[i];
+                        v[4 * i + 0] = tanhFast(v[4 * i + 0] + b4.x);
+                        v[4 * i + 1] = tanhFast(v[4 * i + 1] + b4.y);
+                        v[4 * i + 2] = tanhFast(v[4 * i + 2] + b4.z);
+                        v[4 * i + 3] = tanhFast(v[4 * i + 3] + b4.w);
+                    }
                     storeRow16(act, kTile, t, c0, v);
+                    storeRow16(act, kTile, t, c0 + 16, v + 16);
                     if (yt)
                     {
                         uint8_t *yl = yt + yImgOff(l + 1);
 #pragma unroll
-                        for (int i = 0; i < 16; ++i)
+                        for (int i = 0; i < 32; ++i)
                             storeBf16(yl + swzOffset(c0 + i, t, kHid), v[i]);
                     }
                 }
-                else if (valid)
+            }
+            else if (half == 0)
+            {
+                float v[16];
+                tmemLoad16(tlane, v);
+                const float *bl = bias + l * kHid;
+                if (valid)
                 {
-                    float4 *o = reinterpret_cast<float4 *>(out + (size_t)p * kOut + c0);
+                    float4 *o = reinterpret_cast<float4 *>(out + (size_t)p * kOut);
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         o[i] = make_float4(v[4 * i] + bl[4 * i], v[4 * i + 1] + bl[4 * i + 1],
@@ -259,16 +339,24 @@ k_mlp_forward(const uint8_t *__restrict__ wImg, const float *__restrict__ params
             }
             fenceProxyAsync();
             tmemFenceBefore();
-            __syncthreads();
+            groupSync(g);
         }
     }
-    if (dead && t == 0) setErr(err, 1);
+    if (dead && lead) setErr(err, 1);
+    // No thread leaves while the weights are still arriving (a group without
+    // a tile has not waited for them; a second bounded wait after a timeout).
+    if (threadIdx.x == 0 && (!loaded || dead))
+    {
+        bool d2 = false;
+        mbarWait(barW, 0, d2);
+        if (d2) setErr(err, 1);
+    }
     tmemFenceBefore();
     __syncthreads();
     if (warp == 0)
     {
         tmemFenceAfter();
-        tmemDealloc(tmem, 128);
+        tmemDealloc(tbase, tcols);
     }
 }
 
@@ -289,7 +377,7 @@ constexpr uint32_t kBwdDZT = 163840;    // 32 KB: rows = out, K = points
 constexpr uint32_t kBwdBar = 196608;    // 5 mbarriers + TMEM slot + loss scratch
 constexpr uint32_t kBwdSmem = kBwdBar + 128 + 1024;
 
-__global__ void __launch_bounds__(kTile, 1)
+__global__ void __launch_bounds__(kGroup, 1)
 k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yImg,
                const float *__restrict__ out, const float *__restrict__ tgt,
                const int *__restrict__ idx, int n, LossWeights lw, float *__restrict__ part,
@@ -304,10 +392,12 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
     uint64_t *barM = barWT + 4;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(barWT + 5);
     float *red = reinterpret_cast<float *>(barWT + 6);               // 4 floats
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x & (kTile - 1), half = threadIdx.x / kTile;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool lead = threadIdx.x == 0;
     bool dead = false;
 
-    if (t == 0)
+    if (lead)
     {
         for (int i = 0; i < 5; ++i) mbarInit(barWT + i, 1);
         mbarInitFence();
@@ -317,7 +407,7 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
     __syncthreads();
     tmemFenceAfter();
     const uint32_t tmem = *tslot;
-    const uint32_t tlane = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t dzS = smemAddr(dz), dztS = smemAddr(dzt);
     uint32_t phM = 0, phWT[2] = {0, 0}, phY[2] = {0, 0};
     const float invN = 1.f / (float)n;
@@ -336,14 +426,15 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
     {
         const uint8_t *yt = yImg + (size_t)tile * kYTileBytes;
         float *pr = part + (size_t)tile * kPartStride;
-        if (t == 0)
+        if (lead)
         {
             loadY(yt, 4, 0);
             loadWT(4, 0);
             loadY(yt, 3, 1);
             loadWT(3, 1);
         }
-        // dZ4 = dLoss/dO and the tile's loss.
+        // dZ4 = dLoss/dO and the tile's loss (one thread per point).
+        if (half == 0)
         {
             const int p = tile * kTile + t;
             float d[kOut], loss = 0.f;
@@ -370,7 +461,7 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
         fenceProxyAsync();
         tmemFenceBefore();
         __syncthreads();
-        if (t == 0) pr[kLossSlot] = (red[0] + red[1]) + (red[2] + red[3]);
+        if (lead) pr[kLossSlot] = (red[0] + red[1]) + (red[2] + red[3]);
 
 #pragma unroll 1
         for (int l = 4; l >= 0; --l)
@@ -386,7 +477,7 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
                 if (!waitAll(barWT + b, phWT[b], dead)) break;
                 phWT[b] ^= 1;
             }
-            if (t == 0)
+            if (lead)
             {
                 tmemFenceAfter();
                 if (l == 4)   // dW4^T [in x out] = Y4^T dZ4: A = Y4^T, B = dZ4^T
@@ -400,11 +491,12 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
             if (!waitAll(barM, phM, dead)) break;
             phM ^= 1;
             tmemFenceAfter();
-            if (t == 0 && l - 2 >= 1) loadWT(l - 2, b);
+            if (lead && l - 2 >= 1) loadWT(l - 2, b);
             // db_l from the BF16 dZ_l the MMAs used.
-            if (t < outW)
+            if (half == 0 && t < outW)
             {
                 float s = 0.f;
+#pragma unroll 4
                 for (int k0 = 0; k0 < kTile; k0 += 8)
                 {
                     const uint4 w = *reinterpret_cast<const uint4 *>(dzt + swzOffset(t, k0, outW));
@@ -418,12 +510,13 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
             {
                 float v[16];
                 tmemLoad16(tlane + 128, v);
+                if (half == 1)
 #pragma unroll
-                for (int o = 0; o < kOut; ++o) pr[wOff(4) + o * kHid + t] = v[o];
+                    for (int o = 0; o < kOut; ++o) pr[wOff(4) + o * kHid + t] = v[o];
             }
             else
             {
-                for (int c0 = 0; c0 < in; c0 += 16)
+                for (int c0 = half * (in / 2); c0 < (half + 1) * (in / 2); c0 += 16)
                 {
                     float v[16];
                     tmemLoad16(tlane + 128 + c0, v);
@@ -438,7 +531,7 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
             {
                 const uint8_t *ys = sm + kBwdY + b * 32768;
                 float dzRow[16];
-                for (int c0 = 0; c0 < kHid; c0 += 16)
+                for (int c0 = half * (kHid / 2); c0 < (half + 1) * (kHid / 2); c0 += 16)
                 {
                     tmemLoad16(tlane + c0, dzRow);
 #pragma unroll
@@ -457,11 +550,11 @@ k_mlp_backward(const uint8_t *__restrict__ wtImg, const uint8_t *__restrict__ yI
             fenceProxyAsync();
             tmemFenceBefore();
             __syncthreads();
-            if (t == 0 && l - 2 >= 0) loadY(yt, l - 2, b);
+            if (lead && l - 2 >= 0) loadY(yt, l - 2, b);
         }
         __syncthreads();
     }
-    if (dead && t == 0) setErr(err, 2);
+    if (dead && lead) setErr(err, 2);
     tmemFenceBefore();
     __syncthreads();
     if (warp == 0)
@@ -506,7 +599,9 @@ __global__ void k_mlp_update(const float *__restrict__ part, int ntiles, float *
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > kNParams) return;
+    // (in tile order; sixteen loads in flight)
     float g = 0.f;
+#pragma unroll 16
     for (int tl = 0; tl < ntiles; ++tl) g += part[(size_t)tl * kPartStride + i];
     if (i == kLossSlot)
     {
@@ -726,7 +821,7 @@ struct alebgk_net
     uint8_t *wImg = nullptr, *wtImg = nullptr;
     uint8_t *yImg = nullptr;
     float *part = nullptr, *out = nullptr;
-    int *err = nullptr;
+    int *err = nullptr, *errHost = nullptr;   // pinned host word and its device address
     size_t tilesCap = 0;
     long long adamSteps = 0;
     std::string msg;
@@ -765,10 +860,8 @@ int ensureTiles(alebgk_net *n, size_t tiles)
 
 int checkErr(alebgk_net *n)
 {
-    int h = 0;
-    NCK(cudaMemcpyAsync(&h, n->err, sizeof(int), cudaMemcpyDeviceToHost, n->stream));
     NCK(cudaStreamSynchronize(n->stream));
-    if (h) return netFail(n, ALEBGK_ECUDA, "a tensor-core pipeline wait timed out");
+    if (*n->errHost) return netFail(n, ALEBGK_ECUDA, "a tensor-core pipeline wait timed out");
     return ALEBGK_OK;
 }
 
@@ -790,14 +883,16 @@ int runBatch(alebgk_net *n, const float *pts, const float *tgt, const int *idx, 
         if (rc) return rc;
     }
     const int grid = gridFor(n, tiles);
-    k_mlp_forward<<<grid, kTile, kFwdSmem, n->stream>>>(
+    // Forward: a group per tile while the blocks have tiles for them.
+    const int groups = std::min(kFwdGroups, (tiles + grid - 1) / grid);
+    k_mlp_forward<<<grid, kGroup * groups, fwdSmem(groups), n->stream>>>(
         n->wImg, n->params, reinterpret_cast<const float4 *>(pts), idx, count,
         train ? n->out : outDev, train ? n->yImg : nullptr, n->err);
     NCK(cudaGetLastError());
     if (!train) return ALEBGK_OK;
     LossWeights lw;
     for (int c = 0; c < kOutUsed; ++c) lw.w[c] = chanW ? chanW[c] : 1.f;
-    k_mlp_backward<<<grid, kTile, kBwdSmem, n->stream>>>(n->wtImg, n->yImg, n->out, tgt, idx,
+    k_mlp_backward<<<grid, kGroup, kBwdSmem, n->stream>>>(n->wtImg, n->yImg, n->out, tgt, idx,
                                                         count, lw, n->part, n->err);
     NCK(cudaGetLastError());
     return ALEBGK_OK;
@@ -824,16 +919,21 @@ int alebgk_net_create(int device, alebgk_net **out)
     if (e == cudaSuccess) e = cudaMalloc(&n->loss, sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&n->wImg, kWImgBytes);
     if (e == cudaSuccess) e = cudaMalloc(&n->wtImg, kWTImgBytes);
-    if (e == cudaSuccess) e = cudaMalloc(&n->err, sizeof(int));
+    if (e == cudaSuccess)
+        e = cudaHostAlloc(reinterpret_cast<void **>(&n->errHost), sizeof(int), cudaHostAllocMapped);
+    if (e == cudaSuccess)
+    {
+        *n->errHost = 0;
+        e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&n->err), n->errHost, 0);
+    }
     if (e == cudaSuccess) e = cudaMemset(n->params, 0, kPartStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(n->m, 0, kPartStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(n->v, 0, kPartStride * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(n->wImg, 0, kWImgBytes);
     if (e == cudaSuccess) e = cudaMemset(n->wtImg, 0, kWTImgBytes);
-    if (e == cudaSuccess) e = cudaMemset(n->err, 0, sizeof(int));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kFwdSmem);
+                                 (int)fwdSmem(kFwdGroups));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kBwdSmem);
@@ -853,8 +953,9 @@ void alebgk_net_destroy(alebgk_net *n)
     if (n->stream) cudaStreamSynchronize(n->stream);
     for (void *p : {(void *)n->params, (void *)n->m, (void *)n->v, (void *)n->grad,
                     (void *)n->loss, (void *)n->wImg, (void *)n->wtImg, (void *)n->yImg,
-                    (void *)n->part, (void *)n->out, (void *)n->err})
+                    (void *)n->part, (void *)n->out})
         if (p) cudaFree(p);
+    if (n->errHost) cudaFreeHost(n->errHost);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
 }

@@ -36,3 +36,16 @@ def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
     (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
     np.testing.assert_array_equal(ga, gb)
     np.testing.assert_array_equal(ma, mb)
+
+
+def test_forward_rows_do_not_depend_on_the_call(gpu):
+    """One to three tiles in flight a block, full and ragged last tiles: a point's outputs are the same bits."""
+    from alebgk4paper_b200 import warmstart as ws
+    rng = np.random.default_rng(3)
+    net = ws.WarmStartNet(ws.init_params(1))
+    q = rng.uniform(0, 1, (3 * 148 * 128 + 300, 4)).astype(np.float32)
+    full = net.forward(q).cpu().numpy()
+    assert np.isfinite(full).all()
+    for n in (1, 127, 128, 129, 148 * 128, 148 * 128 + 1, 2 * 148 * 128 + 77, len(q) - 1):
+        np.testing.assert_array_equal(net.forward(q[:n]).cpu().numpy(), full[:n])
+    net.close()
