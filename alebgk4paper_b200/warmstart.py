@@ -28,6 +28,7 @@ import ctypes
 import json
 import math
 import time
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 
@@ -211,10 +212,34 @@ class WarmStartNet:
         rng = np.random.default_rng(seed)
         w = np.ones(N_USED, np.float32) if chan_w is None else np.asarray(chan_w, np.float32)
         wp = w.ctypes.data_as(_abi.c_float_p)
+        # An epoch's permutation takes the host longer (about 9 ns a row) than
+        # its steps take the device, so the next one is drawn on a thread of
+        # its own meanwhile; only as many as the steps need.
+        left = -(-steps // max(1, n // batch)) if n else 0
+
+        def draw():
+            return rng.permutation(n).astype(np.int32)
+
+        with ThreadPoolExecutor(1) as pool:
+            ahead = pool.submit(draw) if left > 0 else None
+            log = self._fit_steps(x, y, n, steps, batch, lr, lr_final, log_every, wp, pool, draw,
+                                  ahead, left)
+        self._ok(self.lib.alebgk_net_sync(self.h))
+        return log
+
+    def _fit_steps(self, x, y, n, steps, batch, lr, lr_final, log_every, wp, pool, draw, ahead,
+                   left):
+        t = self.torch
         perm, pos, log = None, n, []
         for s in range(steps):
             if pos + batch > n:
-                perm = self._dev(rng.permutation(n).astype(np.int32), t.int32)
+                perm, left = ahead.result(), left - 1
+                ahead = pool.submit(draw) if left > 0 else None
+                # the steps read the indices on the network's own stream: the
+                # last epoch's are freed only once they are done
+                if s:
+                    self._ok(self.lib.alebgk_net_sync(self.h))
+                perm = self._dev(perm, t.int32)
                 pos = 0
             ix = perm[pos:pos + batch]
             pos += batch
@@ -226,7 +251,6 @@ class WarmStartNet:
                 float(cur), 0.9, 0.999, 1e-8, ctypes.byref(loss) if want else None))
             if want:
                 log.append((s, loss.value / ix.shape[0]))
-        self._ok(self.lib.alebgk_net_sync(self.h))
         return log
 
     def close(self):
