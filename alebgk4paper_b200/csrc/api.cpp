@@ -50,9 +50,14 @@ cudaError_t putRowOrder(alebgk_ctx *c, const int *boundary, int N)
 {
     std::vector<int> order;
     order.reserve(N);
+    c->interiorRows = 0;
     for (int pass = 0; pass < 2; ++pass)
         for (int i = 0; i < N; ++i)
-            if ((boundary[i] != 0) == (pass == 1)) order.push_back(i);
+            if ((boundary[i] != 0) == (pass == 1))
+            {
+                order.push_back(i);
+                if (pass == 0) c->interiorRows = (int)order.size();
+            }
     return cudaMemcpy(c->d.rowOrder, order.data(), 4 * (size_t)N, cudaMemcpyHostToDevice);
 }
 
@@ -567,6 +572,7 @@ int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
     // the graphs stay valid and are kept.
     unsigned char spBefore[sizeof(StepParams)];
     std::memcpy(spBefore, &p, sizeof p);
+    const int interiorBefore = c->interiorRows;
     const void *bufBefore[] = {d.coef, d.coefLin, d.slots, d.surfList, d.bodyIO};
     // Geometry first: the class keys are computed from the device copy.
     CK(cudaMemcpy(d.pos, cl->xyz, 24 * (size_t)N, cudaMemcpyHostToDevice));
@@ -637,9 +643,10 @@ int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
     const bool tiledBefore = c->tiled;
     if (const int r = setupTiles(c, in, tb)) return r;
     // The step graphs hold the slot stride, the table pointers, the march's
-    // plan: rebuilt when any changed.
+    // plan and the count of interior rows: rebuilt when any changed.
     const void *bufAfter[] = {d.coef, d.coefLin, d.slots, d.surfList, d.bodyIO};
     bool same = std::memcmp(spBefore, &p, sizeof p) == 0 && !marched && !c->march.enabled &&
+                interiorBefore == c->interiorRows &&
                 tiledBefore == c->tiled;
     for (int k = 0; k < 5 && same; ++k) same = bufBefore[k] == bufAfter[k];
     if (!same)
@@ -1073,7 +1080,10 @@ int alebgk_get_counters(alebgk_ctx *c, alebgk_counters *out)
     out->mass_before = s.sigma * s.massNew;
     out->error_word = s.err;
     out->transport_kernel = c->march.enabled ? 2 : 1;
-    out->particle_kernel = c->pStream ? (c->pRows ? 3 : 2) : 1;
+    // 3: the register rows of the FP32 grids up to Nv 10; the other forms of
+    // the row stage count as the streamed one
+    out->particle_kernel =
+        c->pStream ? (c->pRows && c->cfg.precision != 64 && c->sp.Nv <= 10 ? 3 : 2) : 1;
     return ALEBGK_OK;
 }
 

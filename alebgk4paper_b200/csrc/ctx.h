@@ -155,6 +155,12 @@ struct alebgk_ctx
     // Register-row form of the streamed stages (FP32, Nv <= 10): on, blocks.
     bool pRows = false;
     int pRowsBlocks = 0;
+    // Groups of rows (the other 3-D clouds); interior rows lead rowOrder.
+    bool pGroup = false;
+    int interiorRows = 0;
+    // Whether the particle stage runs by rows, on its own transported rows
+    // and with the NAD ranges of k_step_begin.
+    bool rowStage() const { return pStream || pGroup; }
     std::string err;
     std::vector<int> bodyIdHost;
     int maxBodyId = -1;          // largest entry of bodyIdHost (-1: no body particle)

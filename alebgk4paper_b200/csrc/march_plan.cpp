@@ -74,6 +74,8 @@ void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb, const int
     auto coord = [&](int i, int &x, int &y, int &z) {
         x = i % nx; y = (i / nx) % ny; z = i / (nx * ny);
     };
+    int outside = 0;
+#pragma omp parallel for schedule(static) reduction(| : outside)
     for (int i = 0; i < N; ++i)
     {
         int xi, yi, zi;
@@ -82,9 +84,10 @@ void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb, const int
         {
             int xj, yj, zj;
             coord(nbr[(size_t)i * maxNeigh + s], xj, yj, zj);
-            if (templateIndex(xj - xi, yj - yi, zj - zi) < 0) return;
+            outside |= templateIndex(xj - xi, yj - yi, zj - zi) < 0;
         }
     }
+    if (outside) return;
 
     // Template offset -> slot of each class, from its representative.
     const int V = tb.V, ncls = tb.ncls, S = tb.S;

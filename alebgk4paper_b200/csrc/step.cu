@@ -706,6 +706,31 @@ __device__ __forceinline__ void warpSumMany(double (&v)[K], int lane)
     }
 }
 
+// Sums the eight values v over the warp: the return value is the total of
+// value q = (bits 4, 3, 2 of the lane), complete on the lanes whose bits 1
+// and 0 are zero (and on the others of the group).
+__device__ __forceinline__ double warpSum8(const double (&v)[8], int lane)
+{
+    double w[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) w[q] = v[q];
+#pragma unroll
+    for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1)
+    {
+        const bool up = (lane & bit) != 0;
+#pragma unroll
+        for (int q = 0; q < half; ++q)
+        {
+            const double keep = up ? w[q + half] : w[q];
+            const double give = up ? w[q] : w[q + half];
+            w[q] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+    }
+    w[0] += __shfl_xor_sync(0xffffffffu, w[0], 2);
+    w[0] += __shfl_xor_sync(0xffffffffu, w[0], 1);
+    return w[0];
+}
+
 // NAD neighbour density range of every interior particle
 // (MLSTransport.cpp:325-379) from the previous step's macros, one warp per
 // particle; the streamed particle kernel reads it instead of gathering.
@@ -1075,14 +1100,14 @@ k_particle_stream(ParticleArgs<T> a, StepParams p, int wpb)
 }
 
 // ---------------------------------------------------------------------------
-// The same stages for a 3-D single-layer FP32 cloud with Nv = NV <= 10, the
-// row held in registers: one warp per row (a persistent grid walks the
+// The same stages for a 3-D single-layer cloud with Nv = NV of an instance,
+// the row held in registers: one warp per row (a persistent grid walks the
 // rows).  A row of NV^3 velocities is NV^2 lines of NV contiguous values
 // (fixed ky, kz; kx = 0..NV-1); lane l holds lines l, l + 32, ... .  One
 // load of the row serves the whole stage:
-//   - positivity sums and the moments of the positive part, in FP32 per lane
-//     (the kx loop runs over compile-time velocity registers, the line's vy,
-//     vz apply once per line), combined over the warp in FP64;
+//   - positivity sums and the moments of the positive part, in the storage
+//     type per lane (the kx loop runs over compile-time velocity registers,
+//     the line's vy, vz apply once per line), combined over the warp in FP64;
 //   - the decisions and the Maxwellian's parameters, on every lane alike;
 //   - the per-axis Maxwellian factors, one (axis, node) per lane in FP64,
 //     and their per-axis moment sums by one warp reduction;
@@ -1095,14 +1120,32 @@ k_particle_stream(ParticleArgs<T> a, StepParams p, int wpb)
 // negative values sum to less than 1e-30 in magnitude (Positivity), below the
 // rounding of the FP64 moments, and rows of no positive mass are deferred to
 // k_fixup as before.
+// Bound: a row's FP64 chain (reductions, exponentials, divisions) and the HBM
+// traffic of the row in and out.  Measured, particle stage: FP32 Nx 40 Nv 10
+// 172 us (HBM 79); FP32 Nx 27 Nv 12 111 us, 175 by the streamed rows; FP64 Nx
+// 40 Nv 10 336 us (HBM 159), 470 streamed and 425 in groups of rows.  The
+// register file ends it: FP64 at Nv 12, FP32 at Nv 14.
 // ---------------------------------------------------------------------------
 constexpr int kRowsThreads = 128;   // four warps per block of the register-row stage
 
+// Two consecutive values of a row.
+template <typename T> struct Pair2;
+template <> struct Pair2<float>
+{
+    typedef float2 V;
+    static __device__ __forceinline__ V make(float a, float b) { return make_float2(a, b); }
+};
+template <> struct Pair2<double>
+{
+    typedef double2 V;
+    static __device__ __forceinline__ V make(double a, double b) { return make_double2(a, b); }
+};
+
 // Lane l's lines l, l + 32, ... of a row of NV^3 values (zeros past the
 // row's NV^2 lines).
-template <int NV>
-__device__ __forceinline__ void loadRowLines(const float *row, int lane,
-                                             float (&x)[(NV * NV + 31) / 32][NV])
+template <typename T, int NV>
+__device__ __forceinline__ void loadRowLines(const T *row, int lane,
+                                             T (&x)[(NV * NV + 31) / 32][NV])
 {
     constexpr int LINES = NV * NV, LPL = (LINES + 31) / 32;
 #pragma unroll
@@ -1111,13 +1154,13 @@ __device__ __forceinline__ void loadRowLines(const float *row, int lane,
         const int L = lane + 32 * j;
         if (L < LINES)
         {
-            const float *ln = row + L * NV;
+            const T *ln = row + L * NV;
             if constexpr (NV % 2 == 0)
             {
 #pragma unroll
                 for (int q = 0; q < NV; q += 2)
                 {
-                    const float2 v2 = *reinterpret_cast<const float2 *>(ln + q);
+                    const auto v2 = *reinterpret_cast<const typename Pair2<T>::V *>(ln + q);
                     x[j][q] = v2.x;
                     x[j][q + 1] = v2.y;
                 }
@@ -1131,29 +1174,48 @@ __device__ __forceinline__ void loadRowLines(const float *row, int lane,
         else
         {
 #pragma unroll
-            for (int q = 0; q < NV; ++q) x[j][q] = 0.0f;
+            for (int q = 0; q < NV; ++q) x[j][q] = T(0);
         }
     }
 }
 
-template <int NV>
-__global__ void __launch_bounds__(kRowsThreads, 4)
-k_particle_rows(ParticleArgs<float> a, StepParams p)
+// Blocks an SM: the registers that the row takes.
+template <typename T, int NV>
+constexpr int rowsBlocks() { return NV <= 8 || (NV <= 10 && sizeof(T) == 4) ? 4 : (sizeof(T) == 4 || NV <= 10 ? 3 : 2); }
+
+// Dynamic shared memory: two staged rows per warp.
+template <typename T>
+static size_t rowsSmem(int Nv)
+{
+    const int V = Nv * Nv * Nv, pad = 16 / (int)sizeof(T);
+    return sizeof(T) * (size_t)((V + pad - 1) / pad * pad) * 2 * (kRowsThreads / 32);
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(kRowsThreads, rowsBlocks<T, NV>())
+k_particle_rows(ParticleArgs<T> a, StepParams p)
 {
     constexpr int LINES = NV * NV;
     constexpr int LPL = (LINES + 31) / 32;       // lines per lane
     constexpr int V = NV * NV * NV;
-    static_assert(NV <= 10 && 3 * NV <= 32, "rows of at most 10^3 velocities");
+    constexpr int AXR = (3 * NV + 31) / 32;      // axis nodes per lane
+    static_assert(AXR <= 2, "at most 64 axis nodes");
     __shared__ double wtab[kRowsThreads / 32][3][kMaxNv];  // diffuse-wall tables
     __shared__ double velD[kMaxNv];
-    __shared__ float velF[kMaxNv];
+    __shared__ T velT[kMaxNv];
     __shared__ int idxT[V];
+    // Factors of longer grids, by axis node (up to 10 nodes they go by shuffle).
+    __shared__ T efS[kRowsThreads / 32][AXR > 1 ? 3 * NV : 1];
     // Two staged rows per warp: the row being processed (the wall rows' flux
     // balance reads it from here) and the next one, arriving by one bulk copy.
-    constexpr int LDF = (V + 3) / 4 * 4;
-    __shared__ __align__(16) float rowBuf[kRowsThreads / 32][2][LDF];
+    constexpr int PAD = 16 / (int)sizeof(T);
+    constexpr int LDF = (V + PAD - 1) / PAD * PAD;
+    extern __shared__ __align__(16) unsigned char rowsSmemRaw[];
     __shared__ __align__(8) uint64_t rowBar[kRowsThreads / 32][2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T *rowBuf[2];
+    rowBuf[0] = reinterpret_cast<T *>(rowsSmemRaw) + (size_t)(2 * warp) * LDF;
+    rowBuf[1] = rowBuf[0] + LDF;
     if (lane == 0)
     {
         mbarInit(&rowBar[warp][0], 1);
@@ -1168,18 +1230,15 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
     for (int q = threadIdx.x; q < NV; q += blockDim.x)
     {
         velD[q] = fma((double)q, p.dv, p.vmin);
-        velF[q] = (float)velD[q];
+        velT[q] = (T)velD[q];
     }
     __syncthreads();
-    float vx[NV];
+    T vx[NV];
 #pragma unroll
-    for (int q = 0; q < NV; ++q) vx[q] = velF[q];
-    // this lane's axis node of the per-axis factors
-    const int myAxis = lane / NV, myNode = lane - (lane / NV) * NV;
-    const double myV = lane < 3 * NV ? velD[myNode] : 0.0;
+    for (int q = 0; q < NV; ++q) vx[q] = velT[q];
     const double dvN = p.dvN, c1 = p.c1;
     const int W = gridDim.x * (blockDim.x >> 5);
-    constexpr uint32_t kRowBytes = 4u * LDF;
+    constexpr uint32_t kRowBytes = (uint32_t)sizeof(T) * LDF;
     // The warp's rows: t, t + W, ...; the index, wall flag and screen range
     // of the next row are loaded one row ahead, and the next row itself is
     // staged into the other rowBuf by one bulk copy while the current row is
@@ -1193,7 +1252,7 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
     if (lane == 0 && t < p.N)
     {
         mbarExpectTx(&rowBar[warp][0], kRowBytes);
-        bulkLoad(&rowBuf[warp][0][0], a.g + (size_t)inext * p.ldf, kRowBytes, &rowBar[warp][0]);
+        bulkLoad(rowBuf[0], a.g + (size_t)inext * p.ldf, kRowBytes, &rowBar[warp][0]);
     }
     bool dead = false;
     for (uint32_t it = 0; t < p.N; t += W, ++it)
@@ -1208,8 +1267,8 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
         nadN = (more && p.limiter == 2) ? reinterpret_cast<const double2 *>(a.nad)[inext]
                                         : make_double2(INFINITY, -INFINITY);
         inext2 = t + 2 * W < p.N ? a.rowOrder[t + 2 * W] : 0;
-        float *row = a.g + (size_t)i * p.ldf;
-        float x[LPL][NV];
+        T *row = a.g + (size_t)i * p.ldf;
+        T x[LPL][NV];
         const int b = it & 1;
         const uint32_t par = (it >> 1) & 1u;
         mbarWait(&rowBar[warp][b], par, dead);
@@ -1226,37 +1285,38 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
             __syncwarp();
             return;
         }
-        loadRowLines<NV>(&rowBuf[warp][b][0], lane, x);
+        T *cur = b ? rowBuf[1] : rowBuf[0];
+        loadRowLines<T, NV>(cur, lane, x);
         __syncwarp();
         if (lane == 0 && more)
         {
             fenceProxyAsync();     // the warp's reads of the other buffer are done
             mbarExpectTx(&rowBar[warp][b ^ 1], kRowBytes);
-            bulkLoad(&rowBuf[warp][b ^ 1][0], a.g + (size_t)inext * p.ldf, kRowBytes,
+            bulkLoad(b ? rowBuf[0] : rowBuf[1], a.g + (size_t)inext * p.ldf, kRowBytes,
                      &rowBar[warp][b ^ 1]);
         }
-        float s0 = 0.f, sn = 0.f, sx = 0.f, sy = 0.f, sz = 0.f, se = 0.f;
+        T s0 = T(0), sn = T(0), sx = T(0), sy = T(0), sz = T(0), se = T(0);
 #pragma unroll
         for (int j = 0; j < LPL; ++j)
         {
             const int L = lane + 32 * j;
-            float ls = 0.f, lx = 0.f, le = 0.f;
+            T ls = T(0), lx = T(0), le = T(0);
 #pragma unroll
             for (int q = 0; q < NV; ++q)
             {
-                const float xp = fmaxf(x[j][q], 0.0f);
+                const T xp = fmax(x[j][q], T(0));
                 ls += xp;
-                sn += fminf(x[j][q], 0.0f);
-                lx = fmaf(vx[q], xp, lx);
-                le = fmaf(vx[q] * vx[q], xp, le);
+                sn += x[j][q] - xp;      // the negative part; not finite if x is not
+                lx = fma(vx[q], xp, lx);
+                le = fma(vx[q] * vx[q], xp, le);
             }
             if (L < LINES)
             {
-                const float vy = velF[L % NV], vz = velF[L / NV];
+                const T vy = velT[L % NV], vz = velT[L / NV];
                 s0 += ls;
                 sx += lx;
-                sy = fmaf(vy, ls, sy);
-                sz = fmaf(vz, ls, sz);
+                sy = fma(vy, ls, sy);
+                sz = fma(vz, ls, sz);
                 se += le + (vy * vy + vz * vz) * ls;
             }
         }
@@ -1274,7 +1334,7 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
                 if (pv.fix) atomicAdd(&a.sc->nfix, 1);
                 a.massPos[i] = m * dvN;
             }
-            finishWallStream(a, p, i, (const float *)&rowBuf[warp][b][0], idxT, velD, pv,
+            finishWallStream(a, p, i, (const T *)cur, idxT, velD, pv,
                              wtab[warp], lane);
             __syncwarp();
             continue;
@@ -1319,51 +1379,69 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
         // Per-axis factors: lane d NV + q holds axis d, node q; their
         // per-axis sums of velocity^0,1,2 by one reduction (eight values,
         // then the ninth).
-        double e = 0.0;
-        if (lane < 3 * NV)
-        {
-            const double u = myAxis == 0 ? ux : (myAxis == 1 ? uy : uz);
-            e = (myAxis == 0 ? lamA : 1.0) * exp(-(myV - u) * (myV - u) / twoRT);
-        }
-        double S8[8];
+        double S8[8], S22p = 0.0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < 8; ++j) S8[j] = 0.0;
+        T ef[AXR];
+#pragma unroll
+        for (int w = 0; w < AXR; ++w)
         {
-            const int d = j / 3, pw = j - 3 * d;
-            S8[j] = (lane < 3 * NV && myAxis == d)
-                        ? (pw == 0 ? e : (pw == 1 ? myV * e : myV * myV * e)) : 0.0;
+            const int an = lane + 32 * w;            // axis node: axis an / NV
+            const int axis = an / NV;
+            const bool on = an < 3 * NV;
+            const double va = on ? velD[an - axis * NV] : 0.0;
+            double e = 0.0;
+            if (on)
+            {
+                const double u = axis == 0 ? ux : (axis == 1 ? uy : uz);
+                e = (axis == 0 ? lamA : 1.0) * exp(-(va - u) * (va - u) / twoRT);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                const int d = j / 3, pw = j - 3 * d;
+                S8[j] += (on && axis == d) ? (pw == 0 ? e : (pw == 1 ? va * e : va * va * e)) : 0.0;
+            }
+            S22p += on && axis == 2 ? va * va * e : 0.0;
+            ef[w] = (T)(an < NV ? c1 * e : e);
+            if constexpr (AXR > 1)
+                if (on) efS[warp][an] = ef[w];
         }
         warpSumMany<8>(S8, lane);
-        const double S22 = warpSum(lane < 3 * NV && myAxis == 2 ? myV * myV * e : 0.0);
-        const float ef = (float)(lane < NV ? c1 * e : e);
-        float ex[NV];
+        const double S22 = warpSum(S22p);
+        if constexpr (AXR > 1) __syncwarp();
+        auto factor = [&](int an) -> T {
+            if constexpr (AXR > 1) return efS[warp][an];
+            else return __shfl_sync(0xffffffffu, ef[0], an);
+        };
+        T ex[NV];
 #pragma unroll
-        for (int q = 0; q < NV; ++q) ex[q] = __shfl_sync(0xffffffffu, ef, q);
-        const float am = (float)(c1 * (pv.fix ? pv.s : 1.0));
-        const float lo = pv.fix ? 0.0f : -INFINITY;
-        float mn = INFINITY;
+        for (int q = 0; q < NV; ++q) ex[q] = factor(q);
+        const T am = (T)(c1 * (pv.fix ? pv.s : 1.0));
+        const T lo = pv.fix ? T(0) : T(-INFINITY);
+        T mn = T(INFINITY);
 #pragma unroll
         for (int j = 0; j < LPL; ++j)
         {
             const int L = lane + 32 * j;
             const int Lc = L < LINES ? L : 0;
-            const float eyz = __shfl_sync(0xffffffffu, ef, NV + Lc % NV) *
-                              __shfl_sync(0xffffffffu, ef, 2 * NV + Lc / NV);
+            const T eyz = factor(NV + Lc % NV) * factor(2 * NV + Lc / NV);
             if (L < LINES)
             {
-                float h[NV];
+                T h[NV];
 #pragma unroll
                 for (int q = 0; q < NV; ++q)
                 {
-                    h[q] = fmaf(am, fmaxf(x[j][q], lo), ex[q] * eyz);
-                    mn = fminf(mn, h[q]);
+                    h[q] = fma(am, fmax(x[j][q], lo), ex[q] * eyz);
+                    mn = fmin(mn, h[q]);
                 }
-                float *ln = row + L * NV;
+                T *ln = row + L * NV;
                 if constexpr (NV % 2 == 0)
                 {
 #pragma unroll
                     for (int q = 0; q < NV; q += 2)
-                        *reinterpret_cast<float2 *>(ln + q) = make_float2(h[q], h[q + 1]);
+                        *reinterpret_cast<typename Pair2<T>::V *>(ln + q) =
+                            Pair2<T>::make(h[q], h[q + 1]);
                 }
                 else
                 {
@@ -1372,6 +1450,7 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
                 }
             }
         }
+        if constexpr (AXR > 1) __syncwarp();
         const double mnd = warpMin((double)mn);
         if (lane == 0)
         {
@@ -1399,21 +1478,25 @@ k_particle_rows(ParticleArgs<float> a, StepParams p)
     }
 }
 
-// Launch of the register-row stage for the cloud's Nv (nullptr when no
-// instance covers it).
-typedef void (*RowsKernel)(ParticleArgs<float>, StepParams);
-static RowsKernel rowsKernel(int Nv)
+// The register-row kernel of the cloud's Nv (nullptr when no instance covers
+// it).
+template <typename T>
+static auto rowsKernel(int Nv) -> void (*)(ParticleArgs<T>, StepParams)
 {
     switch (Nv)
     {
-    case 4: return k_particle_rows<4>;
-    case 5: return k_particle_rows<5>;
-    case 6: return k_particle_rows<6>;
-    case 8: return k_particle_rows<8>;
-    case 10: return k_particle_rows<10>;
+    case 4: return k_particle_rows<T, 4>;
+    case 5: return k_particle_rows<T, 5>;
+    case 6: return k_particle_rows<T, 6>;
+    case 8: return k_particle_rows<T, 8>;
+    case 10: return k_particle_rows<T, 10>;
+    case 12: return k_particle_rows<T, 12>;
+    case 14: if constexpr (sizeof(T) == 4) return k_particle_rows<T, 14>;
     default: return nullptr;
     }
 }
+
+#include "particle3d.cuh"
 
 // ---------------------------------------------------------------------------
 // Linear MLS redo of the flagged particles (Solver/Solver.cpp:641-646:
@@ -2187,19 +2270,23 @@ static int particleWarpsPerBlock(const StepParams &p, size_t es)
     return w < 1 ? 1 : (w > kNT / 32 ? kNT / 32 : w);
 }
 
-// The streamed particle stage of a 3-D single-layer cloud: batched (FP32)
-// or one warp per particle.
+// The particle stage of a 3-D single-layer cloud by rows: register rows
+// (FP32, Nv of an instance), groups of rows, or streamed rows of a warp.
 template <typename T>
 static void launchParticleStream(alebgk_ctx *c, const ParticleArgs<T> &pa, const StepParams &p,
                                  cudaStream_t st)
 {
-    if constexpr (sizeof(T) == 4)
+    if (c->pRows)
     {
-        if (c->pRows)
-        {
-            rowsKernel(p.Nv)<<<c->pRowsBlocks, kRowsThreads, 0, st>>>(pa, p);
-            return;
-        }
+        rowsKernel<T>(p.Nv)<<<c->pRowsBlocks, kRowsThreads, rowsSmem<T>(p.Nv), st>>>(pa, p);
+        return;
+    }
+    if (c->pGroup)
+    {
+        const int rows = groupRows(p, sizeof(T)), ni = c->interiorRows;
+        k_particle_group<T><<<(ni + rows - 1) / rows + (p.N - ni + rows - 1) / rows, kNT,
+                            (size_t)rows * p.ldf * sizeof(T), st>>>(pa, p, rows, ni);
+        return;
     }
     k_particle_stream<T><<<c->pStreamBlocks, kNT, c->pStreamSmem, st>>>(pa, p, c->pStreamWpb);
 }
@@ -2254,7 +2341,7 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
     const int pBlocks = (p.N + kNT / 32 - 1) / (kNT / 32);
     const int listBlocks = min(p.N, 296);
     mark();
-    const bool nadOn = c->pStream && p.limiter == 2;
+    const bool nadOn = c->rowStage() && p.limiter == 2;
     const int nadBlocks = min((p.N + kNT / 32 - 1) / (kNT / 32), 1184);
     // The NAD ranges depend only on the previous step's macros: in a step
     // graph they run on a side stream beside the transport; when stages are
@@ -2278,7 +2365,7 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
     // Transport fused into the particle kernel (transport threads 0), except
     // when stages are timed: then it runs as its own kernel, with the same
     // sums, so that its time is seen.
-    const bool fused = !march && !c->pStream && c->tune.transportThreads == 0 && !ev;
+    const bool fused = !march && !c->rowStage() && c->tune.transportThreads == 0 && !ev;
     if (march)
     {
         cudaError_t e = launchMarch(c, from, fb, st);
@@ -2296,7 +2383,7 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
     const int wpb = (c->tune.particleWarps > 0 && c->tune.particleWarps < wmax)
                         ? c->tune.particleWarps : wmax;
     const int ppBlocks = (p.N + wpb - 1) / wpb;
-    if (c->pStream)
+    if (c->rowStage())
         launchParticleStream<T>(c, pa, p, st);
     else if (fused)
     {
@@ -2358,7 +2445,7 @@ static cudaError_t prepareT(alebgk_ctx *c)
 
     // Streamed particle kernel: 3-D single layer, two rows per warp, at
     // least four warps per block in 200 KB of shared memory.
-    c->pStream = false;
+    c->pStream = c->pGroup = false;
     if (e == cudaSuccess && p.dim == 3 && p.L == 1 && p.Nv <= 255 && c->cfg.particle != 1)
     {
         int w = kNT / 32;
@@ -2382,24 +2469,40 @@ static cudaError_t prepareT(alebgk_ctx *c)
                 c->pStreamBlocks = need < sms * occ ? need : sms * occ;
             }
         }
-        // The register-row form of the same stages (FP32, Nv of an
-        // instance): the default, unless the shared-memory form is asked for.
+        // The register-row form of the same stages (Nv of an instance): the
+        // default, unless the shared-memory form is asked for.
         c->pRows = false;
-        // (Its staged rows are (V + 3) / 4 * 4 floats, the FP32 row stride.)
-        const RowsKernel rk = rowsKernel(p.Nv);
-        if (e == cudaSuccess && c->pStream && sizeof(T) == 4 && c->cfg.particle != 3 && rk &&
-            p.dim == 3 && p.ldf == (p.V + 3) / 4 * 4)
+        // (Its staged rows are whole 16-byte units, the row stride.)
+        const auto rk = rowsKernel<T>(p.Nv);
+        const int pad = 16 / (int)sizeof(T);
+        if (e == cudaSuccess && c->pStream && c->cfg.particle != 3 && rk && p.dim == 3 &&
+            p.ldf == (p.V + pad - 1) / pad * pad)
         {
+            const size_t smem = rowsSmem<T>(p.Nv);
+            set((const void *)rk, smem);
             int occ = 0, sms = 0;
-            e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e == cudaSuccess)
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rk, kRowsThreads, 0);
+                e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e == cudaSuccess)
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rk, kRowsThreads, smem);
             if (e == cudaSuccess && occ > 0)
             {
                 const int need = (p.N + kRowsThreads / 32 - 1) / (kRowsThreads / 32);
                 c->pRows = true;
                 c->pRowsBlocks = std::min(need, sms * occ);
             }
+        }
+        // Groups of rows: FP64 clouds, and FP32 rows too long for the
+        // streamed form, where they fit, unless the general or the streamed
+        // form is asked for.  (FP64 Nx 40 Nv 10: 470 us streamed, 425 in
+        // groups; FP32 rows that stream have nothing to gain, Nx 27 Nv 12 175
+        // and 168 us.)
+        const int rows = groupRows(p, sizeof(T));
+        if (e == cudaSuccess && !c->pRows && (sizeof(T) == 8 || !c->pStream) &&
+            c->cfg.particle != 3 && rows > 0)
+        {
+            set((const void *)k_particle_group<T>, (size_t)rows * p.ldf * sizeof(T));
+            c->pGroup = e == cudaSuccess;
         }
     }
     return e;
@@ -2952,7 +3055,7 @@ cudaError_t buildBatchLaunch(alebgk_ctx *const *cs, int n, double *const *resid,
     for (int i = 0; i < n; ++i)
     {
         alebgk_ctx *c = cs[i];
-        if (c->cfg.precision != c0->cfg.precision || c->sp.L != c0->sp.L || c->pStream ||
+        if (c->cfg.precision != c0->cfg.precision || c->sp.L != c0->sp.L || c->rowStage() ||
             c->march.enabled || c->cfg.device != c0->cfg.device)
             return cudaErrorNotSupported;
     }
@@ -3100,12 +3203,12 @@ static cudaError_t slabSegT(alebgk_ctx *c, int from, int seg, cudaStream_t st)
     const size_t rowBytes = (size_t)p.L * p.V * sizeof(T);
     if (seg == 0)
     {
-        const bool nadOn = c->pStream && p.limiter == 2;
+        const bool nadOn = c->rowStage() && p.limiter == 2;
         const int nadBlocks = min((p.N + kNT / 32 - 1) / (kNT / 32), 1184);
         k_step_begin<<<nadOn ? nadBlocks : 1, kNT, 0, st>>>(
             d.sc, 1, macA, d.boundary, d.nslot, d.slots, p.S, p.N, nadOn ? d.nad : nullptr);
         const bool march = c->march.enabled;
-        const bool fused = !march && !c->pStream && c->tune.transportThreads == 0;
+        const bool fused = !march && !c->rowStage() && c->tune.transportThreads == 0;
         if (march)
         {
             cudaError_t e = launchMarch(c, from, fb, st);
@@ -3120,7 +3223,7 @@ static cudaError_t slabSegT(alebgk_ctx *c, int from, int seg, cudaStream_t st)
         const int wpb = (c->tune.particleWarps > 0 && c->tune.particleWarps < wmax)
                             ? c->tune.particleWarps : wmax;
         const int ppBlocks = (p.N + wpb - 1) / wpb;
-        if (c->pStream)
+        if (c->rowStage())
             launchParticleStream<T>(c, pa, p, st);
         else if (fused && p.L == 2)
             k_particle<T, 2, true><<<ppBlocks, kNT, wpb * rowBytes, st>>>(pa, p, wpb);

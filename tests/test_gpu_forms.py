@@ -38,6 +38,26 @@ def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
     np.testing.assert_array_equal(ma, mb)
 
 
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("Nx,Nv", [(6, 7), (6, 9), (7, 12), (5, 14), (5, 16), (4, 20), (4, 27)])
+def test_row_groups_equal_general_particle_kernel(gpu, Nx, Nv, precision):
+    """Groups of four, two and one rows, the last group of a kind partly filled, rows below and above one round of
+    the block, rows with the FP64 collision.  FP32: three roundings a value and step in the collision."""
+    c = ab.Case("cavity3d", Nx, Nv, -1.0, 2)
+    c.g *= 1.0 + 0.01 * np.cos(np.arange(c.N))[:, None]
+    c.macro[:, 0] = c.g.sum(1) * c.params["dv"] ** 3
+    a = ab.Solver(c, precision=precision, transport=1)
+    b = ab.Solver(c, precision=precision, transport=1, particle=1)
+    a.cudaStep(2), b.cudaStep(2)
+    (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
+    tol = 1e-13 if precision == 64 else 2 * 5 * 3 * 6e-8
+    assert _rel(ga, gb) < tol
+    assert _rel(ma[:, 0], mb[:, 0]) < tol and _rel(ma[:, 4], mb[:, 4]) < tol
+    ca, cb = a.counters(), b.counters()
+    assert ca["transport_flags"] == cb["transport_flags"]
+    assert ca["positivity_fixes"] == cb["positivity_fixes"]
+
+
 def test_forward_rows_do_not_depend_on_the_call(gpu):
     """One to three tiles in flight a block, full and ragged last tiles: a point's outputs are the same bits."""
     from alebgk4paper_b200 import warmstart as ws
