@@ -15,6 +15,8 @@
 //   k_scale_mood      sigma on the macros, moodCheck
 //   k_recollide       second collision when moodCheck failed (else exits)
 //   k_mass_end        end-of-step mass after a second collision (else exits)
+// In a step graph k_fixup runs in k_sigma's last block (k_sigma_fix) and
+// k_mass_end in k_recollide's (k_late).
 // k_batch_* run the same stage bodies for a batch of clouds, one launch per
 // stage over all of them (a block finds its cloud from block offsets).
 // The stored state h is the true distribution divided by StepScalars::scale.
@@ -1876,6 +1878,99 @@ k_mass_end(const double *__restrict__ massEnd, int N, double *partial, StepScala
 }
 
 // ---------------------------------------------------------------------------
+// The rare-path launches of a step graph, merged.  A step ends in a chain of
+// short kernels that cost their launch (about 2 us each, beside sums of a few
+// arrays of N values): k_fixup and k_mass_end find nothing to do in nearly
+// every step, so their work goes to the last block of the kernel before them
+// (a ticket, as in gridSumLast).  Same operations and orders, same bits.
+//   k_sigma_fix   k_sigma, then k_fixup by its last block (lists of the few
+//                 rows without positive mass; with tau(rho, T) every row is
+//                 listed and k_fixup keeps its own launch)
+//   k_late        k_recollide, then k_mass_end by its last block
+// Measured, a step alone: cavity2d Nx 20 Nv 16 FP64 50.6 -> 49.2 us, cavity3d
+// Nx 27 Nv 12 FP32 778 -> 771 us for two.  Merging the whole chain into the
+// redo's last block was slower: 296 blocks' fences in every step, and sums on one SM (96 cavities:
+// 18.9 ms a 10 steps against 16.2).
+// ---------------------------------------------------------------------------
+template <typename T>
+__device__ __noinline__ void lateFixup(const ParticleArgs<T> &a, const StepParams &p)
+{
+    k_fixup_body<T>(a, p, 0, 1);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads)
+k_sigma_fix(ParticleArgs<T> a, StepParams p, double *partial)
+{
+    static_assert(kRedThreads == kNT, "one block size");
+    __shared__ bool mine;
+    StepScalars *sc = a.sc;
+    double m = 0.0;
+    if (threadIdx.x == 0) mine = false;
+    if (gridSumLast(a.massPos, p.N, partial, sc, &m))
+    {
+        sc->massNew = m;
+        sc->sigma = (m > 1.0e-30) ? sc->massOld / m : 1.0;
+        mine = sc->ndeg > 0;
+    }
+    __syncthreads();
+    if (mine) lateFixup<T>(a, p);
+}
+
+// The sum of a[0..N) by one block, in the order of gridSumLast over
+// kRedBlocks blocks; every thread receives it.
+__device__ double blockGridSum(const double *a, int N, double *sh)
+{
+    constexpr int stride = kRedBlocks * kRedThreads;
+    double total = 0.0;
+    for (int b = 0; b < kRedBlocks; ++b)
+    {
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        int i = b * kRedThreads + threadIdx.x;
+        for (; i + 3 * stride < N; i += 4 * stride)
+        {
+            s0 += __ldcg(a + i);
+            s1 += __ldcg(a + i + stride);
+            s2 += __ldcg(a + i + 2 * stride);
+            s3 += __ldcg(a + i + 3 * stride);
+        }
+        for (; i < N; i += stride) s0 += __ldcg(a + i);
+        double v[1] = {(s0 + s1) + (s2 + s3)};
+        blockSums<1>(v, sh);
+        total += v[0];
+    }
+    return total;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kNT)
+k_late(T *__restrict__ g, StepParams p, const int *__restrict__ boundary,
+       double *__restrict__ macNew, double *massEnd, StepScalars *sc)
+{
+    static_assert(kRedThreads == kNT, "one block size");
+    if (sc->moodfail == 0) return;
+    __shared__ double sh[32];
+    __shared__ bool last;
+    k_recollide_body(g, p, boundary, macNew, massEnd, sc, blockIdx.x, gridDim.x);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        last = atomicAdd(&sc->redCount, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    const double m = blockGridSum(massEnd, p.N, sh);
+    if (threadIdx.x == 0)
+    {
+        sc->redCount = 0;
+        sc->massEnd = sc->sigma * m;
+        sc->massOld = sc->massEnd;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Slab groups.  The global sums of the step (Conservation.cpp:48-109, the
 // moodCheck flag of Conservation.cpp:16-38) become, per slab, a sum over the
 // owned range into slabPart[q], then one combine over all slabs in slab
@@ -2396,14 +2491,26 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
     if (p.L == 2) k_redo<T, 2><<<listBlocks, kNT, rowBytes, st>>>(pa, p);
     else k_redo<T, 1><<<listBlocks, kNT, rowBytes, st>>>(pa, p);
     mark();
-    k_sigma<<<kRedBlocks, kRedThreads, 0, st>>>(d.massPos, p.N, d.redPartial, d.sc);
-    mark();
-    k_fixup<T><<<min(pBlocks, 296), kNT, 0, st>>>(pa, p);
+    const bool merged = !ev;      // (timed stages need launches of their own)
+    if (merged && !p.tauVar)
+        k_sigma_fix<T><<<kRedBlocks, kRedThreads, 0, st>>>(pa, p, d.redPartial);
+    else
+    {
+        k_sigma<<<kRedBlocks, kRedThreads, 0, st>>>(d.massPos, p.N, d.redPartial, d.sc);
+        mark();
+        k_fixup<T><<<min(pBlocks, 296), kNT, 0, st>>>(pa, p);
+    }
     mark();
     k_mass_sum<<<kRedBlocks, kRedThreads, 0, st>>>(d.massEnd, p.N, d.redPartial, d.sc);
     mark();
     k_scale_mood<<<(p.N + 255) / 256, 256, 0, st>>>(p, d.boundary, macB, d.minG, d.mood, d.sc);
     mark();
+    if (merged)
+    {
+        if (p.limiter == 2)
+            k_late<T><<<min(pBlocks, 592), kNT, 0, st>>>(fb, p, d.boundary, macB, d.massEnd, d.sc);
+        return cudaGetLastError();
+    }
     if (p.limiter == 2)
         k_recollide<T><<<min(pBlocks, 592), kNT, 0, st>>>(fb, p, d.boundary, macB, d.massEnd,
                                                          d.sc);

@@ -1,8 +1,11 @@
 """The forms that a step and the network choose by size against the general ones, at the edges of their ranges."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import alebgk4paper_b200 as ab
+from alebgk4paper_b200 import _abi
 
 pytestmark = pytest.mark.gpu
 
@@ -56,6 +59,26 @@ def test_row_groups_equal_general_particle_kernel(gpu, Nx, Nv, precision):
     ca, cb = a.counters(), b.counters()
     assert ca["transport_flags"] == cb["transport_flags"]
     assert ca["positivity_fixes"] == cb["positivity_fixes"]
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("name,Nx,Nv", [("cavity2d", 9, 6), ("cavity2d", 64, 6), ("cavity2d", 65, 6),
+                                        ("cavity3d", 16, 4), ("cavity3d", 17, 4), ("cavity3d", 27, 4)])
+def test_merged_end_of_step_equals_separate_launches(gpu, name, Nx, Nv, precision):
+    """Up to 4 096 particles and above: bitwise the chain of single kernels (timed steps)."""
+    c = ab.Case(name, Nx, Nv, -1.0, 2)
+    a, b = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision)
+    if name == "cavity2d":
+        a.set_launch(256, 0), b.set_launch(256, 0)
+    a.cudaStep(4)
+    ms = (ctypes.c_float * _abi.NSTAGES)()
+    ab._check(b.lib.alebgk_profile_steps(b.ctx, 4, ms), b.ctx)
+    (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
+    np.testing.assert_array_equal(ga, gb)
+    np.testing.assert_array_equal(ma, mb)
+    ca, cb = a.counters(), b.counters()
+    for k in ("mass_before", "mass_after_transport", "mass_scale", "mass_end", "transport_flags"):
+        assert ca[k] == cb[k], k
 
 
 def test_forward_rows_do_not_depend_on_the_call(gpu):
