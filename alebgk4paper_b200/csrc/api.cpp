@@ -927,7 +927,7 @@ int alebgk_step(alebgk_ctx *c, int nsteps)
         {
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t le = launchStep(c, from);
+            cudaError_t le = launchStep(c, from, nullptr, true);
             cudaError_t ee = cudaStreamEndCapture(c->stream, &g);
             if (le != cudaSuccess || ee != cudaSuccess)
             {

@@ -138,6 +138,7 @@ struct alebgk_ctx
     int cur = 0;                 // buffer holding the current h and macros
     bool uploaded = false;
     int ncls = 0;
+    int sms = 0;                 // multiprocessors of the device
     bool tiled = false;          // the gather transport runs by tiles (tiles.cu)
     int degenerateParticles = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -191,7 +192,7 @@ cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st);
 
 // Launch wrappers (step.cu).
 cudaError_t prepareKernels(alebgk_ctx *c);
-cudaError_t launchStep(alebgk_ctx *c, int from, cudaEvent_t *ev = nullptr);
+cudaError_t launchStep(alebgk_ctx *c, int from, cudaEvent_t *ev = nullptr, bool alone = false);
 cudaError_t launchMassInit(alebgk_ctx *c);
 // Slab groups (slab.cpp): one segment of the split step (0..3) on stream st,
 // the cross-slab combine of a segment's partial sums (phase 0..3, 4 = set-up

@@ -131,8 +131,10 @@ __host__ __device__ __forceinline__ int transportChunks(int V)
 }
 
 // Accumulates the slots of one chunk of a row: nodes k0 + 32 q for q < qn
-// (k0 = first node of the chunk + lane), both Chu layers when L = 2.
-template <typename T, int L>
+// (k0 = first node of the chunk + lane), both Chu layers when L = 2.  The
+// loads of U slots are in flight at once; every node still sums its slots one
+// after the other, so U changes no bit.
+template <typename T, int L, int U = 1>
 __device__ __forceinline__ void gatherChunk(const T *__restrict__ f, const T *__restrict__ cc,
                                             const int *__restrict__ sl, int ns, int V, int ldf,
                                             int k0, int qn, T (&a0)[kTransportQ],
@@ -142,7 +144,36 @@ __device__ __forceinline__ void gatherChunk(const T *__restrict__ f, const T *__
     for (int q = 0; q < kTransportQ; ++q) { a0[q] = T(0); a1[q] = T(0); }
     // the lanes past V in the last group neither load nor store
     const bool tail = k0 + 32 * (qn - 1) >= V;
-    for (int s = 0; s < ns; ++s)
+    int s = 0;
+    if constexpr (U > 1)
+        for (; s + U <= ns; s += U)
+        {
+            T w[U][kTransportQ], x0[U][kTransportQ], x1[U][L == 2 ? kTransportQ : 1];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+            {
+                const T *cs = cc + (size_t)(s + u) * V;
+                const T *fr = f + (size_t)__ldg(sl + s + u) * ldf + k0;
+#pragma unroll
+                for (int q = 0; q < kTransportQ; ++q)
+                    if (q < qn && (!tail || k0 + 32 * q < V))
+                    {
+                        w[u][q] = __ldg(cs + 32 * q);
+                        x0[u][q] = __ldg(fr + 32 * q);
+                        if constexpr (L == 2) x1[u][q] = __ldg(fr + V + 32 * q);
+                    }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < kTransportQ; ++q)
+                    if (q < qn && (!tail || k0 + 32 * q < V))
+                    {
+                        a0[q] = fma(w[u][q], x0[u][q], a0[q]);
+                        if constexpr (L == 2) a1[q] = fma(w[u][q], x1[u][q], a1[q]);
+                    }
+        }
+    for (; s < ns; ++s)
     {
         const T *cs = cc + (size_t)s * V;
         const T *fr = f + (size_t)__ldg(sl + s) * ldf + k0;
@@ -191,7 +222,7 @@ __device__ __forceinline__ void transportRow(const T *__restrict__ f, T *__restr
 // Particle i's whole transported row into a warp's shared-memory row copy
 // (the fused transport of the particle kernel): the same sums as
 // transportRow, chunk by chunk.
-template <typename T, int L>
+template <typename T, int L, int U>
 __device__ __forceinline__ void transportRowShared(const T *__restrict__ f, T *__restrict__ buf,
             const T *__restrict__ coef, const int *__restrict__ cls,
             const int *__restrict__ nslot, const int *__restrict__ slots,
@@ -208,7 +239,7 @@ __device__ __forceinline__ void transportRowShared(const T *__restrict__ f, T *_
         const int qn = min(per, groups - g0);
         const int k0 = g0 * 32 + lane;
         T a0[kTransportQ], a1[kTransportQ];
-        gatherChunk<T, L>(f, cc + k0, sl, ns, V, ldf, k0, qn, a0, a1);
+        gatherChunk<T, L, U>(f, cc + k0, sl, ns, V, ldf, k0, qn, a0, a1);
 #pragma unroll
         for (int q = 0; q < kTransportQ; ++q)
         {
@@ -590,7 +621,7 @@ __device__ int screen(const ParticleArgs<T> &a, const StepParams &p, int i, int 
 // g; a flagged particle's row is then not stored (k_redo rebuilds it), a
 // deferred one's is.
 // ---------------------------------------------------------------------------
-template <typename T, int L, bool Fused = false>
+template <typename T, int L, bool Fused = false, int U = 1>
 __device__ __forceinline__ void k_particle_body(const ParticleArgs<T> &a, const StepParams &p,
                                                 int warpsPerBlock, int bx)
 {
@@ -602,7 +633,7 @@ __device__ __forceinline__ void k_particle_body(const ParticleArgs<T> &a, const 
     if (i >= p.N) return;                        // warp-uniform
     T *buf = reinterpret_cast<T *>(rowSmem) + (size_t)warp * L * p.V;
     if (Fused)
-        transportRowShared<T, L>(a.fold, buf, a.coef, a.cls, a.nslot, a.slots, p.S, p.V, p.ldf,
+        transportRowShared<T, L, U>(a.fold, buf, a.coef, a.cls, a.nslot, a.slots, p.S, p.V, p.ldf,
                                  T(a.sc->scale), i, lane);
     RowRegs<T, L> r = Fused ? RowRegs<T, L>(a.g + (size_t)i * p.ldf, buf, p, lane, true)
                             : RowRegs<T, L>(a.g + (size_t)i * p.ldf, buf, p, lane);
@@ -628,6 +659,17 @@ __global__ void __launch_bounds__(kNT)
 k_particle(ParticleArgs<T> a, StepParams p, int warpsPerBlock)
 {
     k_particle_body<T, L, Fused>(a, p, warpsPerBlock, blockIdx.x);
+}
+
+// The fused form of a small 2-D cloud, all of whose particles are resident at
+// once: registers are free then and what counts is the latency of the gather's
+// dependent loads, so the loads of U slots are in flight (the same bits).
+// W particles (warps) per block, B blocks an SM.
+template <typename T, int W, int B, int U>
+__global__ void __launch_bounds__(32 * W, B)
+k_particle_small(ParticleArgs<T> a, StepParams p)
+{
+    k_particle_body<T, 2, true, U>(a, p, W, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1889,8 +1931,8 @@ k_mass_end(const double *__restrict__ massEnd, int N, double *partial, StepScala
 //   k_late        k_recollide, then k_mass_end by its last block
 // Measured, a step alone: cavity2d Nx 20 Nv 16 FP64 50.6 -> 49.2 us, cavity3d
 // Nx 27 Nv 12 FP32 778 -> 771 us for two.  Merging the whole chain into the
-// redo's last block was slower: 296 blocks' fences in every step, and sums on one SM (96 cavities:
-// 18.9 ms a 10 steps against 16.2).
+// redo's last block was slower: 296 blocks' fences in every step, and sums on
+// one SM (96 cavities: 18.9 ms a 10 steps against 16.2).
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __noinline__ void lateFixup(const ParticleArgs<T> &a, const StepParams &p)
@@ -2409,12 +2451,29 @@ static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
     return cudaGetLastError();
 }
 
+// The small 2-D form that holds the whole cloud in one wave, the one with the
+// most slots in flight first; sw = its particles per block.  Measured, SMALLFIGS
+template <typename T>
+static auto smallKernel(const alebgk_ctx *c, int &sw) -> void (*)(ParticleArgs<T>, StepParams)
+{
+    const int N = c->sp.N;
+    const size_t rowBytes = (size_t)c->sp.L * c->sp.V * sizeof(T);
+    if (8 * rowBytes > 100u * 1024u) return nullptr;
+    if constexpr (sizeof(T) == 4)
+    {
+        if (N <= c->sms * 12) { sw = 4; return k_particle_small<T, 4, 3, 4>; }
+    }
+    else if (N <= c->sms * 8) { sw = 4; return k_particle_small<T, 4, 2, 2>; }
+    return nullptr;
+}
+
 // Launches one step.  With ev != nullptr an event is recorded before each
 // launch and after the last one (ev[0..ALEBGK_NSTAGES]), in launch order:
 // step_begin, transport, particle, redo, sigma, fixup, mass_sum, scale_mood,
 // recollide, mass_end.
+// With alone the step has the device to itself (no batch graph around it).
 template <typename T>
-static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
+static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev, bool alone)
 {
     const StepParams &p = c->sp;
     DeviceBuffers &d = c->d;
@@ -2482,7 +2541,12 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev)
         launchParticleStream<T>(c, pa, p, st);
     else if (fused)
     {
-        if (p.L == 2) k_particle<T, 2, true><<<ppBlocks, kNT, wpb * rowBytes, st>>>(pa, p, wpb);
+        int sw = 0;
+        // (not where a launch shape was asked for)
+        const auto small = p.L == 2 && alone && c->tune.particleWarps == 0 ? smallKernel<T>(c, sw)
+                                                                           : nullptr;
+        if (small) small<<<(p.N + sw - 1) / sw, 32 * sw, sw * rowBytes, st>>>(pa, p);
+        else if (p.L == 2) k_particle<T, 2, true><<<ppBlocks, kNT, wpb * rowBytes, st>>>(pa, p, wpb);
         else k_particle<T, 1, true><<<ppBlocks, kNT, wpb * rowBytes, st>>>(pa, p, wpb);
     }
     else if (p.L == 2) k_particle<T, 2, false><<<ppBlocks, kNT, wpb * rowBytes, st>>>(pa, p, wpb);
@@ -2535,6 +2599,7 @@ static cudaError_t prepareT(alebgk_ctx *c)
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
     auto set = [&](const void *fn, size_t bytes) {
         cudaFuncAttributes fa{};
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
@@ -2547,6 +2612,9 @@ static cudaError_t prepareT(alebgk_ctx *c)
     set((const void *)k_particle<T, 2, false>, wpb * rowBytes);
     set((const void *)k_particle<T, 1, true>, wpb * rowBytes);
     set((const void *)k_particle<T, 2, true>, wpb * rowBytes);
+    int sw = 0;
+    if (p.L == 2)
+        if (const auto small = smallKernel<T>(c, sw)) set((const void *)small, sw * rowBytes);
     set((const void *)k_redo<T, 1>, rowBytes);
     set((const void *)k_redo<T, 2>, rowBytes);
 
@@ -2622,10 +2690,10 @@ cudaError_t prepareKernels(alebgk_ctx *c)
     return (c->cfg.precision == 64) ? prepareT<double>(c) : prepareT<float>(c);
 }
 
-cudaError_t launchStep(alebgk_ctx *c, int from, cudaEvent_t *ev)
+cudaError_t launchStep(alebgk_ctx *c, int from, cudaEvent_t *ev, bool alone)
 {
-    return (c->cfg.precision == 64) ? stepT<double>(c, from, ev)
-                                    : stepT<float>(c, from, ev);
+    return (c->cfg.precision == 64) ? stepT<double>(c, from, ev, alone)
+                                    : stepT<float>(c, from, ev, alone);
 }
 
 // ---------------------------------------------------------------------------

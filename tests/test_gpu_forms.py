@@ -81,6 +81,20 @@ def test_merged_end_of_step_equals_separate_launches(gpu, name, Nx, Nv, precisio
         assert ca[k] == cb[k], k
 
 
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("Nx,Nv", [(5, 6), (12, 15), (34, 6), (35, 6), (42, 8), (43, 8), (20, 28)])
+def test_small_2d_form_equals_plain_form(gpu, Nx, Nv, precision):
+    """Up to eight (FP64) and twelve (FP32) particles an SM and above: bitwise the plain fused form."""
+    c = ab.Case("cavity2d", Nx, Nv, -1.0, 2)
+    a, b = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision)
+    b.set_launch(0, 8)
+    a.cudaStep(4), b.cudaStep(4)
+    (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
+    np.testing.assert_array_equal(ga, gb)
+    np.testing.assert_array_equal(ma, mb)
+    assert a.counters() == b.counters()
+
+
 def test_forward_rows_do_not_depend_on_the_call(gpu):
     """One to three tiles in flight a block, full and ragged last tiles: a point's outputs are the same bits."""
     from alebgk4paper_b200 import warmstart as ws
