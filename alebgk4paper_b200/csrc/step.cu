@@ -2451,8 +2451,11 @@ static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
     return cudaGetLastError();
 }
 
-// The small 2-D form that holds the whole cloud in one wave, the one with the
-// most slots in flight first; sw = its particles per block.  Measured, SMALLFIGS
+// The small 2-D form where one wave holds the whole cloud, else none; sw = its
+// particles per block.  Measured, a step inside the line: FP64 Nx 20 Nv 16
+// 39.9 -> 30.7 us, Nx 33 Nv 20 57.8 -> 45.1; FP32 Nx 20 Nv 16 27.1 -> 25.6,
+// Nx 37 Nv 18 40.0 -> 36.9.  Above it the second wave costs more: FP64 Nx 48
+// Nv 16 45.1 -> 52.7, FP32 Nx 48 Nv 24 52.2 -> 67.4.
 template <typename T>
 static auto smallKernel(const alebgk_ctx *c, int &sw) -> void (*)(ParticleArgs<T>, StepParams)
 {
