@@ -125,8 +125,8 @@ void freeBuffers(alebgk_ctx *c)
                     d.boundary, d.bodyId, d.cls, d.nslot, d.slots, d.macro[0],
                     d.macro[1], d.mood, d.flag, d.flagList, d.degList, d.massPos, d.massEnd, d.minG, d.nad, d.redPartial,
                     d.dpx, d.bodyTmp, d.bodyOut, d.stage, d.surfList, d.bodyIO, d.rankAll, d.sc,
-                    d.rowOrder, d.tiles, d.tileRest, d.tileCount, d.tileFlag,
-                    d.tileCovered};
+                    d.rowOrder, d.tiles, d.strips, d.tileRest, d.tileCount, d.tileFlag,
+                    d.stripFlag, d.tileCovered};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     d = DeviceBuffers();
@@ -323,9 +323,11 @@ static int setupTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb
     if (!d.tiles)
     {
         CK(dalloc(&d.tiles, tileInts((int)N)));
+        CK(dalloc(&d.strips, stripInts((int)N)));
         CK(dalloc(&d.tileRest, N));
-        CK(dalloc(&d.tileCount, 2));
+        CK(dalloc(&d.tileCount, 3));
         CK(dalloc(&d.tileFlag, N));
+        CK(dalloc(&d.stripFlag, N));
         CK(dalloc(&d.tileCovered, N));
     }
     CK(buildTiles(c, in, tb));

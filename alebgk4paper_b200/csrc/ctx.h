@@ -74,10 +74,10 @@ struct DeviceBuffers
     int *surfList = nullptr;           // body-surface particles (boundary, bodyId >= 0)
     int *rowOrder = nullptr;           // the row kernel's visiting order: interior
                                        // particles, then wall particles
-    // Tiles of the gather transport (tiles.cu): tiles, particles outside them,
-    // the counts of both, and the plan's two per-particle arrays.
-    int *tiles = nullptr, *tileRest = nullptr, *tileCount = nullptr;
-    int *tileFlag = nullptr, *tileCovered = nullptr;
+    // Tiles of the gather transport (tiles.cu): tiles, strips, particles outside
+    // both, the three counts, and the plan's per-particle arrays.
+    int *tiles = nullptr, *strips = nullptr, *tileRest = nullptr, *tileCount = nullptr;
+    int *tileFlag = nullptr, *stripFlag = nullptr, *tileCovered = nullptr;
     double *bodyIO = nullptr;          // body-step staging: kBodyIOHead + 13 per surface particle
     double *rankAll = nullptr;         // multi-process slab: every rank's 4 combine words
     int rankAllCap = 0;                // ranks rankAll holds
@@ -183,11 +183,13 @@ struct alebgk_ctx
 namespace alebgk {
 
 // Tiles of the gather transport (tiles.cu): the plan of the uploaded cloud,
-// the int words of the tile list of N particles, and the transport of the tiles.
+// the int words of the lists of N particles, and the transport of the tiles and
+// strips.
 struct CoeffInput;
 struct CoeffTables;
 cudaError_t buildTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb);
 size_t tileInts(int N);
+size_t stripInts(int N);
 cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st);
 
 // Launch wrappers (step.cu).

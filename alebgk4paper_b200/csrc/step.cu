@@ -2428,8 +2428,8 @@ static void launchParticleStream(alebgk_ctx *c, const ParticleArgs<T> &pa, const
     k_particle_stream<T><<<c->pStreamBlocks, kNT, c->pStreamSmem, st>>>(pa, p, c->pStreamWpb);
 }
 
-// The gather transport as its own kernel: by tiles and the particles outside
-// them where the cloud has tiles, else every particle alone.
+// The gather transport as its own kernel: by tiles and strips and the particles
+// outside both where the cloud is tiled, else every particle alone.
 template <typename T>
 static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
 {
@@ -2447,7 +2447,7 @@ static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
     k_transport<T><<<gt, tt, 0, st>>>(fa, fb, static_cast<const T *>(d.coef), d.cls, d.nslot,
                                       d.slots, p.S, p.N, p.V, p.L, p.ldf, d.sc,
                                       c->tiled ? d.tileRest : nullptr,
-                                      c->tiled ? d.tileCount + 1 : nullptr);
+                                      c->tiled ? d.tileCount + 2 : nullptr);
     return cudaGetLastError();
 }
 

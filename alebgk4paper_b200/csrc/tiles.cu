@@ -1,23 +1,26 @@
 // tiles.cu -- coefficient-gather transport of a 3-D cloud that is a lattice
 // for the most part (a cavity with bodies in it): the particles inside it go
-// in tiles of 4 x 2 lattice neighbours, the rest through the plain gather.
+// in tiles of 4 x 2 lattice neighbours, those of the layers along its walls in
+// strips of four, the rest through the plain gather.
 //
 // A tile is eight particles of one full stencil class (80 neighbours at the
 // lattice offsets |o|^2 <= 6) whose neighbours, by their own slot lists, lie
 // in rows of consecutive particle indices: row (dz, y), y = -2..3, holds the
 // x = -2..5 around the tile.  The plan checks every slot of every member on
 // the device, so holes, surfaces and cut rows need no rules: a tile that does
-// not hold leaves its particles to the gather.
+// not hold leaves its particles to the strips and the gather.  A strip is four
+// particles along x of one class whose slots are whole rows of the template
+// (a wall layer's: some rows are missing, none in part), checked the same way.
 //
-// Transport: one warp per tile and chunk of velocities.  Each neighbour value
-// is loaded once for the tile and each coefficient once per row pair, 180 +
-// 160 loads for the 640 FMAs of eight particles (the gather loads a value and
-// a coefficient for every FMA and is bound by L1 throughput).  Every particle
-// sums its slots in slot order, as the gather does; the full class has no
-// coefficient of its own value.
+// Transport: one warp per tile (or strip) and chunk of velocities.  Each
+// neighbour value is loaded once for the tile and each coefficient once per
+// row pair, 180 + 160 loads for the 640 FMAs of eight particles, 144 + 80 for
+// a strip's 320 (the gather loads a value and a coefficient for every FMA and
+// is bound by L1 throughput).  Every particle sums its slots in slot order,
+// as the gather does; the full class has no coefficient of its own value.
 // Measured, cavity3d-cube Nx 40 Nv 10 FP32: transport 1.53 ms by the gather
-// alone, 0.756 ms with tiles; the particles outside them (walls, the layers
-// beside them, around the body) take about half of that.
+// alone; 0.756 ms with tiles (0.307 for 70 % of the particles, 0.456 for the
+// gather of the rest).  The strips take the step there from 985 to 909 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,6 +38,10 @@ namespace {
 // A tile: class, its two first members, then the index of x = 0 of each row
 // (dz + 2) * 6 + y + 2 (rows outside every member's stencil unused).
 constexpr int kTileInts = 33;
+
+// A strip: class, its first member, then for each row (dz + 2) * 5 + dy + 2
+// the index of x = 0 (-1: no such row) and the slot of its first offset.
+constexpr int kStripInts = 52;
 
 __host__ __device__ constexpr int off3(int dx, int dy, int dz)
 {
@@ -136,52 +143,113 @@ __global__ void k_tile_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__r
     if (ok && lane < 8) covered[lane >> 2 ? j + (lane & 3) : i + (lane & 3)] = 1;
 }
 
-// One block: places of the tiles and of the particles outside them, in
-// particle order, and their counts.
-__global__ void __launch_bounds__(1024)
-k_tile_scan(int N, int *flag, int *covered, int *count)
+// The same for strips, of the particles that no tile covers.  first[c] is -1
+// for a class without the strips' form, else the class's row of rowFirst: per
+// template row the slot of its first offset, -1 where the row is missing.
+__global__ void k_strip_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__restrict__ pos,
+                             const int *__restrict__ cls, const int *__restrict__ nslot,
+                             const int *__restrict__ slots, const int *__restrict__ first,
+                             const signed char *__restrict__ rowFirst, int *__restrict__ strip,
+                             int *__restrict__ covered)
 {
-    __shared__ int sh[2][1024];
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= N) return;
+    const int c = cls[i];
+    bool ok = first[c] >= 0 && i + 3 < N && covered[i] == 0 && nslot[i] > 1;
+    if (ok)
+    {
+        const long long ix = llround((pos[3 * (size_t)i] - g.x0) / g.hx);
+        ok = ((ix + 2) & 3) == 0;
+    }
+    for (int m = 1; m < 4 && ok; ++m) ok = cls[i + m] == c && covered[i + m] == 0;
+    if (ok)
+    {
+        const signed char *rs = rowFirst + 25 * first[c];
+        const int ns = nslot[i];
+        for (int q = lane; q < 4 * 25; q += 32)
+        {
+            const int m = q / 25, r = q % 25, s0 = rs[r];
+            if (s0 < 0) continue;
+            const int dy = r % 5 - 2, dz = r / 5 - 2;
+            const int w = dy * dy + dz * dz <= 2 ? 2 : 1;     // offsets -w..w
+            // (the first offset of the row is x = -w)
+            const int base = slots[(size_t)i * S + s0] + w;
+            int s = s0;
+            for (int dx = -w; dx <= w; ++dx)
+            {
+                if (r == 12 && dx == 0) continue;             // the self
+                ok = ok && s < ns && slots[(size_t)(i + m) * S + s] == base + m + dx;
+                ++s;
+            }
+        }
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) strip[i] = ok;
+    if (ok && lane < 4) covered[i + lane] = 2;
+}
+
+// One block: places of the tiles, of the strips and of the particles outside
+// both, in particle order, and their counts.
+__global__ void __launch_bounds__(1024)
+k_tile_scan(int N, int *flag, int *strip, int *covered, int *count)
+{
+    __shared__ int sh[3][1024];
     const int t = threadIdx.x, per = (N + 1023) / 1024;
     const int a = min(t * per, N), b = min(a + per, N);
-    int nt = 0, nr = 0;
+    int n[3] = {0, 0, 0};
     for (int i = a; i < b; ++i)
     {
-        nt += flag[i];
-        nr += !covered[i];
+        n[0] += flag[i];
+        n[1] += strip[i];
+        n[2] += !covered[i];
     }
-    sh[0][t] = nt;
-    sh[1][t] = nr;
+    for (int q = 0; q < 3; ++q) sh[q][t] = n[q];
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1)
     {
-        const int x = t >= o ? sh[0][t - o] : 0, y = t >= o ? sh[1][t - o] : 0;
+        int x[3];
+        for (int q = 0; q < 3; ++q) x[q] = t >= o ? sh[q][t - o] : 0;
         __syncthreads();
-        sh[0][t] += x;
-        sh[1][t] += y;
+        for (int q = 0; q < 3; ++q) sh[q][t] += x[q];
         __syncthreads();
     }
-    int pt = sh[0][t] - nt, pr = sh[1][t] - nr;
+    for (int q = 0; q < 3; ++q) n[q] = sh[q][t] - n[q];
     for (int i = a; i < b; ++i)
     {
-        flag[i] = flag[i] ? pt++ : -1;
-        covered[i] = covered[i] ? -1 : pr++;
+        flag[i] = flag[i] ? n[0]++ : -1;
+        strip[i] = strip[i] ? n[1]++ : -1;
+        covered[i] = covered[i] ? -1 : n[2]++;
     }
     if (t == 1023)
-    {
-        count[0] = sh[0][1023];
-        count[1] = sh[1][1023];
-    }
+        for (int q = 0; q < 3; ++q) count[q] = sh[q][1023];
 }
 
 __global__ void k_tile_write(Tmpl3 t, int N, int S, const int *__restrict__ cls,
                              const int *__restrict__ slots, const int *__restrict__ flag,
-                             const int *__restrict__ covered, int *__restrict__ tiles,
-                             int *__restrict__ rest)
+                             const int *__restrict__ strip, const int *__restrict__ covered,
+                             const int *__restrict__ first,
+                             const signed char *__restrict__ rowFirst, int *__restrict__ tiles,
+                             int *__restrict__ strips, int *__restrict__ rest)
 {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= N) return;
     if (lane == 0 && covered[i] >= 0) rest[covered[i]] = i;
+    if (strip[i] >= 0)
+    {
+        int *o = strips + (size_t)strip[i] * kStripInts;
+        const int s0 = lane < 25 ? rowFirst[25 * first[cls[i]] + lane] : -1;
+        if (lane < 25)
+        {
+            const int dy = lane % 5 - 2, dz = lane / 5 - 2, w = dy * dy + dz * dz <= 2 ? 2 : 1;
+            o[2 + 2 * lane] = s0 >= 0 ? slots[(size_t)i * S + s0] + w : -1;
+            o[3 + 2 * lane] = s0;
+        }
+        if (lane == 0)
+        {
+            o[0] = cls[i];
+            o[1] = i;
+        }
+    }
     if (flag[i] < 0) return;
     int *o = tiles + (size_t)flag[i] * kTileInts;
     const int j = slots[(size_t)i * S + t.slot[2 * 25 + 3 * 5 + 2]];
@@ -289,96 +357,219 @@ k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restric
     }
 }
 
-}  // namespace
-
-// Classes whose slots are the whole template in order (full classes), by
-// their representatives; the lattice spacing comes from the first of them.
-static bool fullClasses(const CoeffInput &in, const CoeffTables &tb, std::vector<int> &full,
-                        TileGrid &g)
+// Grid (velocity chunks, blocks of eight strips).
+template <typename T, int VPL>
+__global__ void __launch_bounds__(256, 3)
+k_transport_strips(const T *__restrict__ f, T *__restrict__ g, const T *__restrict__ coef,
+                   const int *__restrict__ strips, const int *__restrict__ count, int S, int V,
+                   int ldf, const StepScalars *__restrict__ sc)
 {
-    static const Tmpl3 t = makeTmpl3();
-    full.assign(tb.ncls, 0);
-    bool any = false;
-    if (tb.S < 81) return false;
-    for (int c = 0; c < tb.ncls; ++c)
+    typedef Vel<T, VPL> L;
+    typedef typename L::V VT;
+    const int strip = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (strip >= __ldg(count)) return;
+    const int k = (blockIdx.x * 32 + lane) * VPL;
+    if (k >= V) return;
+    const int *st = strips + (size_t)strip * kStripInts;
+    const T *cc = coef + (size_t)__ldg(st) * S * V + k;
+    const int i = __ldg(st + 1);
+    const T *fk = f + k;
+    // the particles' own values first (slot 0)
+    VT acc[4];
     {
-        const int r = tb.rep[c];
-        const bool packed = tb.slots.empty();
-        const int ns = packed ? tb.repNslot[c] : tb.nslot[r];
-        if (ns != 81 || in.boundary[r]) continue;
-        const int *sl = packed ? &tb.repSlots[(size_t)c * tb.S] : &tb.slots[(size_t)r * tb.S];
-        const double *p = in.xyz + 3 * (size_t)r;
-        const double *px = in.xyz + 3 * (size_t)sl[slot3(1, 0, 0)];
-        const double *py = in.xyz + 3 * (size_t)sl[slot3(0, 1, 0)];
-        const double *pz = in.xyz + 3 * (size_t)sl[slot3(0, 0, 1)];
-        const double h[3] = {px[0] - p[0], py[1] - p[1], pz[2] - p[2]};
-        bool ok = h[0] > 0 && h[1] > 0 && h[2] > 0;
-        for (int s = 1; s < 81 && ok; ++s)
-        {
-            const double *q = in.xyz + 3 * (size_t)sl[s];
-            for (int a = 0; a < 3 && ok; ++a)
-                ok = std::fabs((q[a] - p[a]) / h[a] - t.d[s][a]) < 1e-6;
-        }
-        if (!ok) continue;
-        full[c] = 1;
-        if (!any) g = TileGrid{in.xyz[0], in.xyz[1], h[0], h[1]};
-        any = true;
+        const VT c0 = __ldg(reinterpret_cast<const VT *>(cc));
+        const T *own = fk + (size_t)i * ldf;
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            acc[m] = L::fma(c0, __ldg(reinterpret_cast<const VT *>(own + (size_t)m * ldf)), L::zero());
     }
-    return any;
+    unroll3<25>([&](auto Q) {
+        constexpr int q = decltype(Q)::value, dy = q % 5 - 2, dz = q / 5 - 2;
+        if constexpr (dy * dy + dz * dz <= 6 && slot3(0, dy, dz) >= 0)
+        {
+            const int base = __ldg(st + 2 + 2 * q);
+            if (base >= 0)
+            {
+                const T *cs = cc + (size_t)__ldg(st + 3 + 2 * q) * V;
+                const T *row = fk + (size_t)base * ldf;
+                VT v[8];
+                unroll3<8>([&](auto X) {
+                    constexpr int x = decltype(X)::value - 2, qq = decltype(Q)::value;
+                    if constexpr ((x > -2 && x < 5) || slot3(2, qq % 5 - 2, qq / 5 - 2) >= 0)
+                        v[x + 2] = __ldg(reinterpret_cast<const VT *>(row + (long long)x * ldf));
+                });
+                unroll3<5>([&](auto D) {
+                    constexpr int dx = decltype(D)::value - 2, qq = decltype(Q)::value;
+                    constexpr int s = slot3(dx, qq % 5 - 2, qq / 5 - 2);
+                    if constexpr (s > 0)
+                    {
+                        // the offset's place in its row (the self has none)
+                        constexpr int w = slot3(2, qq % 5 - 2, qq / 5 - 2) >= 0 ? 2 : 1;
+                        constexpr int at = dx + w - (qq == 12 && dx > 0 ? 1 : 0);
+                        const VT c = __ldg(reinterpret_cast<const VT *>(cs + (size_t)at * V));
+                        unroll3<4>([&](auto M) {
+                            constexpr int m = decltype(M)::value;
+                            acc[m] = L::fma(c, v[m + decltype(D)::value], acc[m]);
+                        });
+                    }
+                });
+            }
+        }
+    });
+    const T scale = T(sc->scale);
+    T *o = g + (size_t)i * ldf + k;
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        *reinterpret_cast<VT *>(o + (size_t)m * ldf) = L::mul(acc[m], scale);
 }
 
-// Plans the tiles of the uploaded cloud (classes and slot lists on the
-// device); c->d.tileCount holds their number and that of the rest.
+}  // namespace
+
+// The classes on the lattice, by their representatives (the spacing comes from
+// a particle of 80 neighbours): full ones, whose slots are the whole template
+// in order, and ones whose slots are whole rows of it in order, with the slot
+// of each row's first offset.  False where there is no full class.
+static bool latticeClasses(const CoeffInput &in, const CoeffTables &tb, const Tmpl3 &t,
+                           std::vector<int> &full, std::vector<int> &first,
+                           std::vector<signed char> &rowFirst, TileGrid &g)
+{
+    full.assign(tb.ncls, 0);
+    first.assign(tb.ncls, -1);
+    rowFirst.clear();
+    if (tb.S < 81) return false;
+    const bool packed = tb.slots.empty();
+    auto slotsOf = [&](int c, int &ns) -> const int * {
+        const int r = tb.rep[c];
+        ns = packed ? tb.repNslot[c] : tb.nslot[r];
+        return packed ? &tb.repSlots[(size_t)c * tb.S] : &tb.slots[(size_t)r * tb.S];
+    };
+    double h[3] = {0, 0, 0};
+    auto onLattice = [&](const double *p, const double *q, int a, int d) {
+        return std::fabs((q[a] - p[a]) / h[a] - d) < 1e-6;
+    };
+    bool any = false;
+    for (int c = 0; c < tb.ncls; ++c)
+    {
+        int ns;
+        const int *sl = slotsOf(c, ns);
+        if (ns != 81 || in.boundary[tb.rep[c]]) continue;
+        const double *p = in.xyz + 3 * (size_t)tb.rep[c];
+        if (!any)
+        {
+            h[0] = in.xyz[3 * (size_t)sl[slot3(1, 0, 0)]] - p[0];
+            h[1] = in.xyz[3 * (size_t)sl[slot3(0, 1, 0)] + 1] - p[1];
+            h[2] = in.xyz[3 * (size_t)sl[slot3(0, 0, 1)] + 2] - p[2];
+        }
+        bool ok = h[0] > 0 && h[1] > 0 && h[2] > 0;
+        for (int s = 1; s < 81 && ok; ++s)
+            for (int a = 0; a < 3 && ok; ++a)
+                ok = onLattice(p, in.xyz + 3 * (size_t)sl[s], a, t.d[s][a]);
+        full[c] = ok;
+        any = any || ok;
+    }
+    if (!any) return false;
+    g = TileGrid{in.xyz[0], in.xyz[1], h[0], h[1]};
+    for (int c = 0; c < tb.ncls; ++c)
+    {
+        int ns;
+        const int *sl = slotsOf(c, ns);
+        const double *p = in.xyz + 3 * (size_t)tb.rep[c];
+        signed char rs[25];
+        std::fill(rs, rs + 25, (signed char)-1);
+        bool ok = ns <= 81;
+        int s = 1;
+        for (int r = 0; r < 25 && ok; ++r)
+        {
+            const int dy = r % 5 - 2, dz = r / 5 - 2;
+            if (slot3(0, dy, dz) < 0) continue;
+            const int w = slot3(2, dy, dz) >= 0 ? 2 : 1;
+            auto at = [&](int q, int dx) {
+                const double *x = in.xyz + 3 * (size_t)sl[q];
+                return onLattice(p, x, 0, dx) && onLattice(p, x, 1, dy) && onLattice(p, x, 2, dz);
+            };
+            if (s >= ns || !at(s, -w)) continue;      // the row is missing
+            rs[r] = (signed char)s;
+            for (int dx = -w; dx <= w && ok; ++dx)
+            {
+                if (r == 12 && dx == 0) continue;
+                ok = s < ns && at(s, dx);
+                ++s;
+            }
+        }
+        if (!ok || s != ns) continue;                 // other slots, or part of a row
+        first[c] = (int)(rowFirst.size() / 25);
+        rowFirst.insert(rowFirst.end(), rs, rs + 25);
+    }
+    return true;
+}
+
+// Plans the tiles and strips of the uploaded cloud (classes and slot lists on
+// the device); c->d.tileCount holds their numbers and that of the rest.
 cudaError_t buildTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb)
 {
     static const Tmpl3 t = makeTmpl3();
     DeviceBuffers &d = c->d;
     const int N = c->sp.N;
-    std::vector<int> full;
+    std::vector<int> full, first;
+    std::vector<signed char> rowFirst;
     TileGrid g{0, 0, 1, 1};
-    fullClasses(in, tb, full, g);
-    int *dFull = nullptr;
-    cudaError_t e = cudaMalloc(&dFull, 4 * std::max<size_t>(full.size(), 1));
+    latticeClasses(in, tb, t, full, first, rowFirst, g);
+    const size_t n = std::max<size_t>(full.size(), 1);
+    rowFirst.resize(std::max<size_t>(rowFirst.size(), 25), -1);
+    int *dCls = nullptr;              // full, first, then rowFirst
+    cudaError_t e = cudaMalloc(&dCls, 8 * n + rowFirst.size());
+    signed char *dRow = reinterpret_cast<signed char *>(dCls + 2 * n);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dFull, full.data(), 4 * full.size(), cudaMemcpyHostToDevice, c->stream);
+        e = cudaMemcpyAsync(dCls, full.data(), 4 * full.size(), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(dCls + n, first.data(), 4 * first.size(), cudaMemcpyHostToDevice,
+                            c->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(dRow, rowFirst.data(), rowFirst.size(), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d.tileCovered, 0, 4 * (size_t)N, c->stream);
     if (e == cudaSuccess)
     {
         const int blocks = (int)(((long long)N * 32 + 255) / 256);
-        k_tile_mark<<<blocks, 256, 0, c->stream>>>(t, g, N, tb.S, d.pos, d.cls, d.slots, dFull,
+        k_tile_mark<<<blocks, 256, 0, c->stream>>>(t, g, N, tb.S, d.pos, d.cls, d.slots, dCls,
                                                    d.tileFlag, d.tileCovered);
-        k_tile_scan<<<1, 1024, 0, c->stream>>>(N, d.tileFlag, d.tileCovered, d.tileCount);
+        k_strip_mark<<<blocks, 256, 0, c->stream>>>(t, g, N, tb.S, d.pos, d.cls, d.nslot, d.slots,
+                                                    dCls + n, dRow, d.stripFlag, d.tileCovered);
+        k_tile_scan<<<1, 1024, 0, c->stream>>>(N, d.tileFlag, d.stripFlag, d.tileCovered,
+                                               d.tileCount);
         k_tile_write<<<blocks, 256, 0, c->stream>>>(t, N, tb.S, d.cls, d.slots, d.tileFlag,
-                                                    d.tileCovered, d.tiles, d.tileRest);
+                                                    d.stripFlag, d.tileCovered, dCls + n, dRow,
+                                                    d.tiles, d.strips, d.tileRest);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (dFull) cudaFree(dFull);
+    if (dCls) cudaFree(dCls);
     return e;
 }
 
 size_t tileInts(int N) { return (size_t)(N / 8 + 1) * kTileInts; }
+size_t stripInts(int N) { return (size_t)(N / 4 + 1) * kStripInts; }
 
-cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st)
+template <typename T, int VPL>
+static void launchTilesT(alebgk_ctx *c, const void *f, void *g, cudaStream_t st)
 {
     const StepParams &p = c->sp;
     const DeviceBuffers &d = c->d;
-    // as many blocks as there could be tiles: the plan's counts stay on the
-    // device, and a refresh of the geometry changes no launch
-    const int by = (p.N / 8 + 7) / 8;
-    if (by == 0) return cudaSuccess;
-    if (c->cfg.precision == 64)
-        k_transport_tiles<double, 1><<<dim3((p.V + 31) / 32, by), 256, 0, st>>>(
-            static_cast<const double *>(f), static_cast<double *>(g),
-            static_cast<const double *>(d.coef), d.tiles, d.tileCount, p.S, p.V, p.ldf, d.sc);
-    else if (p.V % 2 == 0)
-        k_transport_tiles<float, 2><<<dim3((p.V + 63) / 64, by), 256, 0, st>>>(
-            static_cast<const float *>(f), static_cast<float *>(g),
-            static_cast<const float *>(d.coef), d.tiles, d.tileCount, p.S, p.V, p.ldf, d.sc);
-    else
-        k_transport_tiles<float, 1><<<dim3((p.V + 31) / 32, by), 256, 0, st>>>(
-            static_cast<const float *>(f), static_cast<float *>(g),
-            static_cast<const float *>(d.coef), d.tiles, d.tileCount, p.S, p.V, p.ldf, d.sc);
+    // as many blocks as there could be tiles and strips: the plan's counts
+    // stay on the device, and a refresh of the geometry changes no launch
+    const int chunks = (p.V + 32 * VPL - 1) / (32 * VPL);
+    k_transport_tiles<T, VPL><<<dim3(chunks, (p.N / 8 + 8) / 8), 256, 0, st>>>(
+        static_cast<const T *>(f), static_cast<T *>(g), static_cast<const T *>(d.coef), d.tiles,
+        d.tileCount, p.S, p.V, p.ldf, d.sc);
+    k_transport_strips<T, VPL><<<dim3(chunks, (p.N / 4 + 8) / 8), 256, 0, st>>>(
+        static_cast<const T *>(f), static_cast<T *>(g), static_cast<const T *>(d.coef), d.strips,
+        d.tileCount + 1, p.S, p.V, p.ldf, d.sc);
+}
+
+cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st)
+{
+    if (c->cfg.precision == 64) launchTilesT<double, 1>(c, f, g, st);
+    else if (c->sp.V % 2 == 0) launchTilesT<float, 2>(c, f, g, st);
+    else launchTilesT<float, 1>(c, f, g, st);
     return cudaGetLastError();
 }
 

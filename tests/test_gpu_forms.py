@@ -31,8 +31,9 @@ def test_fp64_march_equals_gather(gpu, Nx, Nv):
 @pytest.mark.parametrize("name,Nx,Nv", [("cavity3d-cube", 12, 5), ("cavity3d-cube", 17, 6), ("cavity3d-sphere", 21, 4),
                                         ("cavity3d-cube", 24, 8)])
 def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
-    """Odd rows (one velocity a lane), partial chunks, lattices with partial tiles, bodies in the middle: every
-    particle sums its slots in the same order, so the states are the same bits."""
+    """Odd rows (one velocity a lane), partial chunks, lattices with partial tiles, wall layers in strips and
+    remainders, bodies in the middle: every particle sums its slots in the same order, so the states are
+    the same bits."""
     c = ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True)
     a, b = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision, transport=1)
     a.cudaStep(3), b.cudaStep(3)
