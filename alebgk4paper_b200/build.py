@@ -23,7 +23,8 @@ SOURCES = ["step.cu", "march.cu", "body_noalloc.cu", "body_step.cu", "warm.cu", 
 # The device MLS table builder must round as the host builder (compiled
 # without contraction) does.
 FILE_FLAGS = {"coeffs_dev.cu": ["-fmad=false"]}
-HEADERS = ["ctx.h", "coeffs.h", "cases.h", "march.h", "mbar.cuh", "umma.cuh", "particle3d.cuh"]
+HEADERS = ["ctx.h", "coeffs.h", "cases.h", "march.h", "mbar.cuh", "umma.cuh", "particle3d.cuh",
+           "vel.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -29,6 +29,7 @@
 
 #include "ctx.h"
 #include "mbar.cuh"
+#include "vel.cuh"
 
 namespace alebgk {
 
@@ -113,64 +114,73 @@ __device__ __forceinline__ double minImage(double d, double L)
 
 // ---------------------------------------------------------------------------
 // Transport: coefficient gather.  Warp = one particle and one chunk of its
-// velocity nodes; lane = nodes k = k0 + lane + 32 q for q < qn <= kTransportQ,
-// so one slot's row index and coefficient row serve qn nodes per lane and
+// velocity nodes; lane = VPL consecutive nodes from k0 + 32 VPL q for q < qn,
+// so one slot's row index and coefficient row serve VPL qn nodes per lane and
 // qn (or 2 qn in 2-D) independent loads are in flight per slot.  The node's
 // coefficients are shared by both Chu layers in 2-D.  Every node sums its
 // slots in slot order, whatever the chunking.  The output is scaled by the
 // stored-state scale so that gt carries the true magnitude.
+// FP32 rows of an even length go by pairs of nodes (8-byte loads, packed FMAs:
+// half the instructions, twice the bytes in flight per load) in the 3-D kernel
+// and the small 2-D form: cavity3d-cube Nx 40 Nv 10 912 -> 877 us a step,
+// cavity2d Nx 37 Nv 18 17.5 -> 16.2.  The plain fused 2-D form keeps single
+// nodes: by pairs, cavity2d Nx 48 Nv 24 took 657 us for ten steps against 568
+// and 96 cavities 18.4 ms against 16.3.
 // ---------------------------------------------------------------------------
-constexpr int kTransportQ = 8;
+constexpr int kTransportQ = 8;    // nodes per lane and chunk at most
 
-// Chunks of a row: the 32-node groups of V split as evenly as possible into
-// chunks of at most kTransportQ groups.
+// Chunks of a row: the groups of 32 VPL nodes of V split as evenly as possible
+// into chunks of at most kTransportQ / VPL groups (the same for VPL 1 and 2).
 __host__ __device__ __forceinline__ int transportChunks(int V)
 {
-    const int groups = (V + 31) / 32;
-    return (groups + kTransportQ - 1) / kTransportQ;
+    return (V + 32 * kTransportQ - 1) / (32 * kTransportQ);
 }
 
-// Accumulates the slots of one chunk of a row: nodes k0 + 32 q for q < qn
-// (k0 = first node of the chunk + lane), both Chu layers when L = 2.  The
+// Accumulates the slots of one chunk of a row: nodes k0 + 32 VPL q for q < qn
+// (k0 = first node of the chunk + VPL lane), both Chu layers when L = 2.  The
 // loads of U slots are in flight at once; every node still sums its slots one
-// after the other, so U changes no bit.
-template <typename T, int L, int U = 1>
-__device__ __forceinline__ void gatherChunk(const T *__restrict__ f, const T *__restrict__ cc,
-                                            const int *__restrict__ sl, int ns, int V, int ldf,
-                                            int k0, int qn, T (&a0)[kTransportQ],
-                                            T (&a1)[kTransportQ])
+// after the other, so neither U nor VPL changes a bit.
+template <typename T, int L, int U, int VPL>
+__device__ __forceinline__ void
+gatherChunk(const T *__restrict__ f, const T *__restrict__ cc, const int *__restrict__ sl, int ns,
+            int V, int ldf, int k0, int qn, typename Vel<T, VPL>::V (&a0)[kTransportQ / VPL],
+            typename Vel<T, VPL>::V (&a1)[kTransportQ / VPL])
 {
+    typedef Vel<T, VPL> L1;
+    typedef typename L1::V VT;
+    constexpr int Q = kTransportQ / VPL, step = 32 * VPL;
+    auto at = [](const T *x) { return __ldg(reinterpret_cast<const VT *>(x)); };
 #pragma unroll
-    for (int q = 0; q < kTransportQ; ++q) { a0[q] = T(0); a1[q] = T(0); }
+    for (int q = 0; q < Q; ++q) { a0[q] = L1::zero(); a1[q] = L1::zero(); }
     // the lanes past V in the last group neither load nor store
-    const bool tail = k0 + 32 * (qn - 1) >= V;
+    const bool tail = k0 + step * (qn - 1) >= V;
     int s = 0;
     if constexpr (U > 1)
         for (; s + U <= ns; s += U)
         {
-            T w[U][kTransportQ], x0[U][kTransportQ], x1[U][L == 2 ? kTransportQ : 1];
+            VT w[U][Q], x0[U][Q], x1[U][L == 2 ? Q : 1];
 #pragma unroll
             for (int u = 0; u < U; ++u)
             {
                 const T *cs = cc + (size_t)(s + u) * V;
                 const T *fr = f + (size_t)__ldg(sl + s + u) * ldf + k0;
 #pragma unroll
-                for (int q = 0; q < kTransportQ; ++q)
-                    if (q < qn && (!tail || k0 + 32 * q < V))
+                for (int q = 0; q < Q; ++q)
+                    if (q < qn && (!tail || k0 + step * q < V))
                     {
-                        w[u][q] = __ldg(cs + 32 * q);
-                        x0[u][q] = __ldg(fr + 32 * q);
-                        if constexpr (L == 2) x1[u][q] = __ldg(fr + V + 32 * q);
+                        w[u][q] = at(cs + step * q);
+                        x0[u][q] = at(fr + step * q);
+                        if constexpr (L == 2) x1[u][q] = at(fr + V + step * q);
                     }
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
-                for (int q = 0; q < kTransportQ; ++q)
-                    if (q < qn && (!tail || k0 + 32 * q < V))
+                for (int q = 0; q < Q; ++q)
+                    if (q < qn && (!tail || k0 + step * q < V))
                     {
-                        a0[q] = fma(w[u][q], x0[u][q], a0[q]);
-                        if constexpr (L == 2) a1[q] = fma(w[u][q], x1[u][q], a1[q]);
+                        a0[q] = L1::fma(w[u][q], x0[u][q], a0[q]);
+                        if constexpr (L == 2) a1[q] = L1::fma(w[u][q], x1[u][q], a1[q]);
                     }
         }
     for (; s < ns; ++s)
@@ -178,79 +188,71 @@ __device__ __forceinline__ void gatherChunk(const T *__restrict__ f, const T *__
         const T *cs = cc + (size_t)s * V;
         const T *fr = f + (size_t)__ldg(sl + s) * ldf + k0;
 #pragma unroll
-        for (int q = 0; q < kTransportQ; ++q)
+        for (int q = 0; q < Q; ++q)
         {
-            if (q < qn && (!tail || k0 + 32 * q < V))
+            if (q < qn && (!tail || k0 + step * q < V))
             {
-                const T w = __ldg(cs + 32 * q);
-                a0[q] = fma(w, __ldg(fr + 32 * q), a0[q]);
-                if (L == 2) a1[q] = fma(w, __ldg(fr + V + 32 * q), a1[q]);
+                const VT w = at(cs + step * q);
+                a0[q] = L1::fma(w, at(fr + step * q), a0[q]);
+                if (L == 2) a1[q] = L1::fma(w, at(fr + V + step * q), a1[q]);
             }
         }
     }
 }
 
-// One chunk of particle i's transported row, stored to out = row of g.
-template <typename T, int L>
-__device__ __forceinline__ void transportRow(const T *__restrict__ f, T *__restrict__ g,
-            const T *__restrict__ coef, const int *__restrict__ cls,
-            const int *__restrict__ nslot, const int *__restrict__ slots,
-            int S, int V, int ldf, T scale, int i, int chunk, int nch, int lane)
+// One chunk of a transported row (qn groups from node group g0), stored to out,
+// the row in g or its copy in shared memory.
+template <typename T, int L, int U, int VPL>
+__device__ __forceinline__ void transportChunk(const T *__restrict__ f, T *__restrict__ out,
+            const T *__restrict__ cc, const int *__restrict__ sl, int ns,
+            int V, int ldf, T scale, int g0, int qn, int lane)
 {
-    const int groups = (V + 31) / 32;
-    const int per = (groups + nch - 1) / nch;
-    const int g0 = chunk * per;
-    const int qn = min(per, groups - g0);        // warp-uniform
-    if (qn <= 0) return;
-    const int k0 = g0 * 32 + lane;
-    const int c = __ldg(cls + i), ns = __ldg(nslot + i);
-    T a0[kTransportQ], a1[kTransportQ];
-    gatherChunk<T, L>(f, coef + (size_t)c * S * V + k0, slots + (size_t)i * S, ns, V, ldf, k0,
-                      qn, a0, a1);
-    T *out = g + (size_t)i * ldf + k0;
+    typedef Vel<T, VPL> L1;
+    typedef typename L1::V VT;
+    constexpr int Q = kTransportQ / VPL, step = 32 * VPL;
+    const int k0 = g0 * step + VPL * lane;
+    VT a0[Q], a1[Q];
+    gatherChunk<T, L, U, VPL>(f, cc + k0, sl, ns, V, ldf, k0, qn, a0, a1);
 #pragma unroll
-    for (int q = 0; q < kTransportQ; ++q)
+    for (int q = 0; q < Q; ++q)
     {
-        if (q < qn && k0 + 32 * q < V)
+        if (q < qn && k0 + step * q < V)
         {
-            out[32 * q] = a0[q] * scale;
-            if (L == 2) out[V + 32 * q] = a1[q] * scale;
+            *reinterpret_cast<VT *>(out + k0 + step * q) = L1::mul(a0[q], scale);
+            if (L == 2) *reinterpret_cast<VT *>(out + V + k0 + step * q) = L1::mul(a1[q], scale);
         }
     }
 }
 
-// Particle i's whole transported row into a warp's shared-memory row copy
-// (the fused transport of the particle kernel): the same sums as
-// transportRow, chunk by chunk.
-template <typename T, int L, int U>
-__device__ __forceinline__ void transportRowShared(const T *__restrict__ f, T *__restrict__ buf,
+// Particle i's row, one chunk of it (chunk >= 0) or all chunk by chunk.
+template <typename T, int L, int U, int VPL>
+__device__ __forceinline__ void transportRow(const T *__restrict__ f, T *__restrict__ out,
             const T *__restrict__ coef, const int *__restrict__ cls,
             const int *__restrict__ nslot, const int *__restrict__ slots,
-            int S, int V, int ldf, T scale, int i, int lane)
+            int S, int V, int ldf, T scale, int i, int chunk, int lane)
 {
-    const int groups = (V + 31) / 32;
+    const int groups = (V + 32 * VPL - 1) / (32 * VPL);
     const int nch = transportChunks(V);
     const int per = (groups + nch - 1) / nch;
     const int c = __ldg(cls + i), ns = __ldg(nslot + i);
     const T *cc = coef + (size_t)c * S * V;
     const int *sl = slots + (size_t)i * S;
-    for (int g0 = 0; g0 < groups; g0 += per)
+    if (chunk >= 0)
     {
-        const int qn = min(per, groups - g0);
-        const int k0 = g0 * 32 + lane;
-        T a0[kTransportQ], a1[kTransportQ];
-        gatherChunk<T, L, U>(f, cc + k0, sl, ns, V, ldf, k0, qn, a0, a1);
-#pragma unroll
-        for (int q = 0; q < kTransportQ; ++q)
-        {
-            if (q < qn && k0 + 32 * q < V)
-            {
-                buf[k0 + 32 * q] = a0[q] * scale;
-                if (L == 2) buf[V + k0 + 32 * q] = a1[q] * scale;
-            }
-        }
+        const int g0 = chunk * per, qn = min(per, groups - g0);      // warp-uniform
+        if (qn > 0) transportChunk<T, L, U, VPL>(f, out, cc, sl, ns, V, ldf, scale, g0, qn, lane);
+        return;
     }
-    __syncwarp();
+    for (int g0 = 0; g0 < groups; g0 += per)
+        transportChunk<T, L, U, VPL>(f, out, cc, sl, ns, V, ldf, scale, g0, min(per, groups - g0),
+                                     lane);
+}
+
+// Pairs of nodes: FP32 and V even (rows and coefficient rows then start on
+// whole pairs).
+template <typename T> __device__ __forceinline__ bool pairs(int V)
+{
+    return sizeof(T) == 4 && V % 2 == 0;
 }
 
 // Block = consecutive particles, one per warp, at one velocity chunk: the
@@ -268,13 +270,15 @@ __device__ __forceinline__ void k_transport_body(const T *__restrict__ f, T *__r
     if (i >= (list ? __ldg(count) : N)) return;
     if (list) i = __ldg(list + i);
     const T scale = T(sc->scale);
-    const int nch = transportChunks(V);
+    T *out = g + (size_t)i * ldf;
+    const int lane = threadIdx.x & 31;
+    constexpr int P = sizeof(T) == 4 ? 2 : 1;
     if (L == 2)
-        transportRow<T, 2>(f, g, coef, cls, nslot, slots, S, V, ldf, scale, i, chunk, nch,
-                           threadIdx.x & 31);
+        transportRow<T, 2, 1, 1>(f, out, coef, cls, nslot, slots, S, V, ldf, scale, i, chunk, lane);
+    else if (pairs<T>(V))
+        transportRow<T, 1, 1, P>(f, out, coef, cls, nslot, slots, S, V, ldf, scale, i, chunk, lane);
     else
-        transportRow<T, 1>(f, g, coef, cls, nslot, slots, S, V, ldf, scale, i, chunk, nch,
-                           threadIdx.x & 31);
+        transportRow<T, 1, 1, 1>(f, out, coef, cls, nslot, slots, S, V, ldf, scale, i, chunk, lane);
 }
 
 // Grid (velocity chunks, particle tiles of blockDim.x / 32); with a list,
@@ -617,11 +621,11 @@ __device__ int screen(const ParticleArgs<T> &a, const StepParams &p, int i, int 
 // Positivity + MOOD screen + finish, one warp per particle.  A particle the
 // screen flags is listed for k_redo and left as is.  Fused: the warp first
 // builds the particle's transported row in its shared-memory copy
-// (transportRowShared, the sums of k_transport) instead of loading it from
+// (transportRow, the sums of k_transport) instead of loading it from
 // g; a flagged particle's row is then not stored (k_redo rebuilds it), a
 // deferred one's is.
 // ---------------------------------------------------------------------------
-template <typename T, int L, bool Fused = false, int U = 1>
+template <typename T, int L, bool Fused = false, int U = 1, bool Pairs = false>
 __device__ __forceinline__ void k_particle_body(const ParticleArgs<T> &a, const StepParams &p,
                                                 int warpsPerBlock, int bx)
 {
@@ -633,8 +637,16 @@ __device__ __forceinline__ void k_particle_body(const ParticleArgs<T> &a, const 
     if (i >= p.N) return;                        // warp-uniform
     T *buf = reinterpret_cast<T *>(rowSmem) + (size_t)warp * L * p.V;
     if (Fused)
-        transportRowShared<T, L, U>(a.fold, buf, a.coef, a.cls, a.nslot, a.slots, p.S, p.V, p.ldf,
-                                 T(a.sc->scale), i, lane);
+    {
+        constexpr int P = Pairs && sizeof(T) == 4 ? 2 : 1;
+        if (P == 2 && pairs<T>(p.V))
+            transportRow<T, L, U, P>(a.fold, buf, a.coef, a.cls, a.nslot, a.slots, p.S, p.V, p.ldf,
+                                     T(a.sc->scale), i, -1, lane);
+        else
+            transportRow<T, L, U, 1>(a.fold, buf, a.coef, a.cls, a.nslot, a.slots, p.S, p.V, p.ldf,
+                                     T(a.sc->scale), i, -1, lane);
+        __syncwarp();
+    }
     RowRegs<T, L> r = Fused ? RowRegs<T, L>(a.g + (size_t)i * p.ldf, buf, p, lane, true)
                             : RowRegs<T, L>(a.g + (size_t)i * p.ldf, buf, p, lane);
     double pos, neg;
@@ -669,7 +681,7 @@ template <typename T, int W, int B, int U>
 __global__ void __launch_bounds__(32 * W, B)
 k_particle_small(ParticleArgs<T> a, StepParams p)
 {
-    k_particle_body<T, 2, true, U>(a, p, W, blockIdx.x);
+    k_particle_body<T, 2, true, U, true>(a, p, W, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------

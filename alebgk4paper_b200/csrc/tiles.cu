@@ -20,7 +20,7 @@
 // as the gather does; the full class has no coefficient of its own value.
 // Measured, cavity3d-cube Nx 40 Nv 10 FP32: transport 1.53 ms by the gather
 // alone; 0.756 ms with tiles (0.307 for 70 % of the particles, 0.456 for the
-// gather of the rest).  The strips take the step there from 985 to 909 us.
+// gather of the rest).  The strips take the step there from 985 to 909 us (877 with the rest by pairs).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,6 +30,7 @@
 
 #include "coeffs.h"
 #include "ctx.h"
+#include "vel.cuh"
 
 namespace alebgk {
 
@@ -276,23 +277,6 @@ __device__ __forceinline__ void unroll3(F &&f)
 {
     unroll3Impl(std::make_integer_sequence<int, M>{}, f);
 }
-
-// The velocities of one lane: two of FP32 (packed FMAs), or one.
-template <typename T, int VPL> struct Vel;
-template <> struct Vel<float, 2>
-{
-    typedef float2 V;
-    static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
-    static __device__ __forceinline__ V fma(V a, V b, V c) { return __ffma2_rn(a, b, c); }
-    static __device__ __forceinline__ V mul(V a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
-};
-template <typename T> struct Vel<T, 1>
-{
-    typedef T V;
-    static __device__ __forceinline__ V zero() { return T(0); }
-    static __device__ __forceinline__ V fma(V a, V b, V c) { return ::fma(a, b, c); }
-    static __device__ __forceinline__ V mul(V a, T s) { return a * s; }
-};
 
 // Grid (velocity chunks, blocks of eight tiles).
 template <typename T, int VPL>
