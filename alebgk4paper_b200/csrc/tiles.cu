@@ -20,7 +20,8 @@
 // as the gather does; the full class has no coefficient of its own value.
 // Measured, cavity3d-cube Nx 40 Nv 10 FP32: transport 1.53 ms by the gather
 // alone; 0.756 ms with tiles (0.307 for 70 % of the particles, 0.456 for the
-// gather of the rest).  The strips take the step there from 985 to 909 us (877 with the rest by pairs).
+// gather of the rest).  The strips take the step there from 985 to 909 us, the
+// pairs of nodes in the gather of the rest to 877.
 #include <cuda_runtime.h>
 
 #include <algorithm>
