@@ -48,6 +48,21 @@ def test_forward_matches_oracle(n):
     net.close()
 
 
+def test_forward_keeps_the_relative_accuracy_of_small_activations():
+    """Pre-activations of about 1e-6 in every layer: what the hidden values lose is their BF16 rounding (2^-9 relative
+    a layer, four layers), nothing absolute."""
+    _torch()
+    from alebgk4paper_b200.warmstart import WarmStartNet, init_params
+    p = init_params(4)
+    p[:W.W_OFF[1]] *= 1e-6
+    q = _inputs(700, seed=12)
+    net = WarmStartNet(p)
+    out = net.forward(q).cpu().numpy()[:, :W.N_USED]
+    ref = W.forward(p, W.features(q))[0][:, :W.N_USED]
+    assert np.linalg.norm(out - ref) <= 4 * 2.0 ** -9 * np.linalg.norm(ref)
+    net.close()
+
+
 def test_forward_gathers_rows_by_index():
     _torch()
     from alebgk4paper_b200.warmstart import WarmStartNet
