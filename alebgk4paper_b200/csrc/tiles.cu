@@ -16,8 +16,10 @@
 // neighbour value is loaded once for the tile and each coefficient once per
 // row pair, 180 + 160 loads for the 640 FMAs of eight particles, 144 + 80 for
 // a strip's 320 (the gather loads a value and a coefficient for every FMA and
-// is bound by L1 throughput).  Every particle sums its slots in slot order,
-// as the gather does; the full class has no coefficient of its own value.
+// is bound by L1 throughput), beside slot 0: the particle's own value, whose
+// coefficient is 1 for a node whose foot point has no neighbour in the support
+// (a step of more than the support's reach) and 0 for every other.  Every
+// particle sums its slots in slot order, as the gather does.
 // Measured, cavity3d-cube Nx 40 Nv 10 FP32: transport 1.53 ms by the gather
 // alone; 0.756 ms with tiles (0.307 for 70 % of the particles, 0.456 for the
 // gather of the rest).  The strips take the step there from 985 to 909 us, the
@@ -296,11 +298,18 @@ k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restric
     const T *cc = coef + (size_t)__ldg(tl) * S * V + k;
     const T *fk = f + k;
     auto coefAt = [&](int s) { return __ldg(reinterpret_cast<const VT *>(cc + (size_t)s * V)); };
+    // the particles' own values first (slot 0)
     VT acc[2][4];
+    const VT c0 = coefAt(0);
 #pragma unroll
     for (int b = 0; b < 2; ++b)
+    {
+        const T *own = fk + (size_t)__ldg(tl + 1 + b) * ldf;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) acc[b][x] = L::zero();
+        for (int x = 0; x < 4; ++x)
+            acc[b][x] = L::fma(c0, __ldg(reinterpret_cast<const VT *>(own + (size_t)x * ldf)),
+                               L::zero());
+    }
     unroll3<30>([&](auto R) {
         constexpr int r = decltype(R)::value, dz = r / 6 - 2, y = r % 6 - 2;
         // member row 0 meets this row at offset dy = y, member row 1 at y - 1

@@ -43,6 +43,25 @@ def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
 
 
 @pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("cells", [2.75, 3.0, 5.0])
+def test_gather_by_tiles_equals_plain_gather_at_a_large_step(gpu, cells, precision):
+    """Steps of more cells than the support reaches (2.5): nodes whose foot point has no neighbour keep the particle's
+    own value.  Bitwise, as at an ordinary step; the fastest node along an axis moves `cells` cells."""
+    c = ab.Case("cavity3d-cube", 17, 6, -1.0, 2, fixed_body=True)
+    c.dt = cells * c.params["dx"] / max(abs(c.params["vmin"]), c.params["vmin"] + (c.Nv - 1) * c.params["dv"])
+    out = []
+    for transport in (0, 1):
+        cfg = c.config(precision, 0, transport)
+        cfg.limiter = 0
+        s = ab.Solver(c, config=cfg)
+        s.cudaStep(1)
+        out.append(s.cudaDownloadFull())
+        s.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("precision", [32, 64])
 @pytest.mark.parametrize("Nx,Nv", [(6, 7), (6, 9), (7, 12), (5, 14), (5, 16), (4, 20), (4, 27)])
 def test_row_groups_equal_general_particle_kernel(gpu, Nx, Nv, precision):
     """Groups of four, two and one rows, the last group of a kind partly filled, rows below and above one round of
