@@ -380,6 +380,12 @@ class Solver:
         _check(self.lib.alebgk_get_counters(self.ctx, ctypes.byref(c)), self.ctx)
         return {k: getattr(c, k) for k, _ in _abi.Counters._fields_}
 
+    def gather_counts(self) -> tuple:
+        """Tiles of eight, strips of four and single particles of the coefficient gather."""
+        n = np.zeros(3, np.int32)
+        _check(self.lib.alebgk_gather_counts(self.ctx, _ip(n)), self.ctx)
+        return tuple(int(x) for x in n)
+
     def cudaLimiterCounts(self):
         c = self.counters()
         return c["positivity_fixes"], c["transport_flags"]

@@ -1089,6 +1089,19 @@ int alebgk_get_counters(alebgk_ctx *c, alebgk_counters *out)
     return ALEBGK_OK;
 }
 
+int alebgk_gather_counts(alebgk_ctx *c, int *counts)
+{
+    if (!c || !counts) return fail(c, ALEBGK_EINVAL, "null argument");
+    if (!c->uploaded) return fail(c, ALEBGK_ESTATE, "upload the cloud first");
+    counts[0] = counts[1] = 0;
+    counts[2] = c->sp.N;
+    if (!c->tiled) return ALEBGK_OK;
+    CK(cudaSetDevice(c->cfg.device));
+    CK(cudaMemcpyAsync(counts, c->d.tileCount, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return ALEBGK_OK;
+}
+
 int alebgk_total_mass(alebgk_ctx *c, double *mass)
 {
     if (!c || !mass) return fail(c, ALEBGK_EINVAL, "null argument");

@@ -88,9 +88,19 @@ Tmpl3 makeTmpl3()
     return t;
 }
 
+// The lattice's columns: spacing, and a particle of a full class as the origin
+// (any other particle may lie off the lattice, a wall point between two columns).
 struct TileGrid
 {
     double x0, y0, hx, hy;
+    __device__ long long col(const double *pos, int i) const
+    {
+        return llround((pos[3 * (size_t)i] - x0) / hx);
+    }
+    __device__ long long row(const double *pos, int i) const
+    {
+        return llround((pos[3 * (size_t)i + 1] - y0) / hy);
+    }
 };
 
 __device__ __forceinline__ int rowSlot(const Tmpl3 &t, int dy, int dz)
@@ -110,6 +120,11 @@ __device__ __forceinline__ int tileRow(const Tmpl3 &t, const int *slots, int S, 
 }
 
 // One warp per particle: whether a tile starts there; marks its members.
+// Tiles start on every fourth column and every second row, and each member's own
+// column and row must be the start's plus its place in the tile.  So no two
+// tiles share a particle, whatever the cloud, and N / 8 places are enough: as a
+// member of a first row a particle has one start, i = itself - (column mod 4);
+// as one of a second row (odd rows) likewise one j, and j's slots name one i.
 __global__ void k_tile_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__restrict__ pos,
                             const int *__restrict__ cls, const int *__restrict__ slots,
                             const int *__restrict__ full, int *__restrict__ flag,
@@ -120,17 +135,18 @@ __global__ void k_tile_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__r
     const int c = cls[i];
     bool ok = full[c] != 0 && i + 3 < N;
     int j = 0;
-    if (ok)
-    {
-        const long long ix = llround((pos[3 * (size_t)i] - g.x0) / g.hx);
-        const long long iy = llround((pos[3 * (size_t)i + 1] - g.y0) / g.hy);
-        ok = ((ix + 2) & 3) == 0 && (iy & 1) == 0;
-    }
+    const long long ix = ok ? g.col(pos, i) : 0, iy = ok ? g.row(pos, i) : 0;
+    ok = ok && (ix & 3) == 0 && (iy & 1) == 0;
     if (ok)
     {
         j = slots[(size_t)i * S + t.slot[2 * 25 + 3 * 5 + 2]];      // (0, 1, 0)
         ok = j + 3 < N;
         for (int m = 0; m < 4 && ok; ++m) ok = cls[i + m] == c && cls[j + m] == c;
+    }
+    if (ok && lane < 8)
+    {
+        const int mem = lane >> 2 ? j + (lane & 3) : i + (lane & 3);
+        ok = g.col(pos, mem) == ix + (lane & 3) && g.row(pos, mem) == iy + (lane >> 2);
     }
     if (ok)
         for (int q = lane; q < 8 * 80; q += 32)
@@ -147,7 +163,9 @@ __global__ void k_tile_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__r
     if (ok && lane < 8) covered[lane >> 2 ? j + (lane & 3) : i + (lane & 3)] = 1;
 }
 
-// The same for strips, of the particles that no tile covers.  first[c] is -1
+// The same for strips, of the particles that no tile covers (covered is 1 for
+// those; strips write 2 for their own members, which no other strip has, by
+// their columns).  first[c] is -1
 // for a class without the strips' form, else the class's row of rowFirst: per
 // template row the slot of its first offset, -1 where the row is missing.
 __global__ void k_strip_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__restrict__ pos,
@@ -159,13 +177,11 @@ __global__ void k_strip_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= N) return;
     const int c = cls[i];
-    bool ok = first[c] >= 0 && i + 3 < N && covered[i] == 0 && nslot[i] > 1;
-    if (ok)
-    {
-        const long long ix = llround((pos[3 * (size_t)i] - g.x0) / g.hx);
-        ok = ((ix + 2) & 3) == 0;
-    }
-    for (int m = 1; m < 4 && ok; ++m) ok = cls[i + m] == c && covered[i + m] == 0;
+    bool ok = first[c] >= 0 && i + 3 < N && covered[i] != 1 && nslot[i] > 1;
+    const long long ix = ok ? g.col(pos, i) : 0;
+    ok = ok && (ix & 3) == 0;
+    for (int m = 1; m < 4 && ok; ++m)
+        ok = cls[i + m] == c && covered[i + m] != 1 && g.col(pos, i + m) == ix + m;
     if (ok)
     {
         const signed char *rs = rowFirst + 25 * first[c];
@@ -458,11 +474,11 @@ static bool latticeClasses(const CoeffInput &in, const CoeffTables &tb, const Tm
         for (int s = 1; s < 81 && ok; ++s)
             for (int a = 0; a < 3 && ok; ++a)
                 ok = onLattice(p, in.xyz + 3 * (size_t)sl[s], a, t.d[s][a]);
+        if (ok && !any) g = TileGrid{p[0], p[1], h[0], h[1]};
         full[c] = ok;
         any = any || ok;
     }
     if (!any) return false;
-    g = TileGrid{in.xyz[0], in.xyz[1], h[0], h[1]};
     for (int c = 0; c < tb.ncls; ++c)
     {
         int ns;

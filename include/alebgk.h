@@ -197,6 +197,13 @@ int alebgk_profile_steps(alebgk_ctx *ctx, int nsteps, float *ms_per_stage);
  * (Solver/CudaBackend.cu:1986-2030). */
 int alebgk_get_counters(alebgk_ctx *ctx, alebgk_counters *out);
 
+/* How the coefficient gather divides the uploaded cloud: tiles of eight
+ * particles, strips of four, and particles gathered one by one (counts[0..2]).
+ * The three cover every particle once: 8 counts[0] + 4 counts[1] + counts[2] =
+ * N.  A cloud that marches or is gathered plainly has {0, 0, N}.  No reference
+ * counterpart. */
+int alebgk_gather_counts(alebgk_ctx *ctx, int *counts);
+
 /* Total gas mass sum(g dv^d) on the device.
  * Replaces cudaTotalMass (Solver/CudaBackend.cu:2018-2024). */
 int alebgk_total_mass(alebgk_ctx *ctx, double *mass);

@@ -1,4 +1,5 @@
 """The forms that a step and the network choose by size against the general ones, at the edges of their ranges."""
+import copy
 import ctypes
 
 import numpy as np
@@ -59,6 +60,71 @@ def test_gather_by_tiles_equals_plain_gather_at_a_large_step(gpu, cells, precisi
         s.close()
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+def _own_cloud(xyz, h, Nv, wall_first, box=None):
+    """A case of these positions at spacing h: neighbours within 2.5 h (over the box's edges where it is given), the
+    density varying from particle to particle.  With wall_first particle 0 is a wall particle."""
+    from scipy.spatial import cKDTree
+    c = copy.copy(ab.Case("cavity3d", 6, Nv, -1.0, 2))
+    N = len(xyz)
+    scale = c.params["radius"] / (2.5 * h)
+    near = cKDTree(xyz, boxsize=box).query_ball_point(xyz, 2.5 * h)
+    c.N, c.xyz, c.meshv = N, np.ascontiguousarray(xyz * scale), np.zeros((N, 3))
+    c.nnb, c.nbr = np.zeros(N, np.int32), np.zeros((N, _abi.MAX_NEIGH), np.int32)
+    for i, js in enumerate(near):
+        js = [j for j in js if j != i]
+        c.nnb[i] = len(js)
+        c.nbr[i, :len(js)] = js
+    c.boundary, c.body_id = np.zeros(N, np.int32), np.full(N, -1, np.int32)
+    c.wall = np.tile(c.wall[0], (N, 1))
+    c.boundary[0] = int(wall_first)
+    f = 1.0 + 0.01 * np.cos(np.arange(N))[:, None]
+    c.g, c.macro = c.g[:1] * f, np.tile(c.macro[0], (N, 1))
+    c.macro[:, 0] *= f[:, 0]
+    return c, scale
+
+
+def _assert_tiled_equals_plain(c, precision, box=0.0, tiles=True):
+    out = []
+    for transport in (0, 1):
+        cfg = c.config(precision, 0, transport)
+        for a in range(3):
+            cfg.periodic[a], cfg.L[a] = int(box > 0), box
+        s = ab.Solver(c, config=cfg)
+        if transport == 0:
+            n = s.gather_counts()
+            assert 8 * n[0] + 4 * n[1] + n[2] == c.N
+            assert (n[0] > 0) == tiles, n
+        s.cudaStep(2)
+        out.append(s.cudaDownloadFull())
+        s.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n", [13, 33])
+def test_tiles_of_a_lattice_that_does_not_hold_the_first_particle(gpu, n, precision):
+    """Cell centres and one wall point, half a cell off them in every axis: the particles' distances from it are k + 1/2
+    cells to an ulp, to either side.  At n = 33 columns rounded from there give 4 437 tiles over the 18 792
+    particles of 2 349.  Every particle is in one tile, one strip or neither."""
+    ax = (np.arange(n) + 0.5) / n
+    z, y, x = np.meshgrid(ax, ax, ax, indexing="ij")
+    xyz = np.concatenate([np.zeros((1, 3)), np.column_stack([x.ravel(), y.ravel(), z.ravel()])])
+    c, _ = _own_cloud(xyz, 1.0 / n, 4, True)
+    _assert_tiled_equals_plain(c, precision)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n,roll", [(13, 0), (13, 2), (14, 3)])
+def test_tiles_of_a_periodic_lattice(gpu, n, roll, precision):
+    """Stencils that reach over the box's edges, of one class with those that do not: no tile reaches over an edge, and
+    with an odd number of rows none overlaps another.  Rolled, the class's first particle lies inside."""
+    ax = np.roll((np.arange(n) + 0.5) / n, -roll)
+    z, y, x = np.meshgrid(ax, ax, ax, indexing="ij")
+    c, scale = _own_cloud(np.column_stack([x.ravel(), y.ravel(), z.ravel()]), 1.0 / n, 4, False, box=1.0)
+    _assert_tiled_equals_plain(c, precision, scale, tiles=roll > 0)
 
 
 @pytest.mark.parametrize("precision", [32, 64])
