@@ -297,7 +297,7 @@ __device__ __forceinline__ void unroll3(F &&f)
     unroll3Impl(std::make_integer_sequence<int, M>{}, f);
 }
 
-// Grid (velocity chunks, blocks of eight tiles).
+// Blocks of eight tiles, the chunks of velocities of a block one after the other.
 template <typename T, int VPL>
 __global__ void __launch_bounds__(256, 2)
 k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restrict__ coef,
@@ -306,9 +306,10 @@ k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restric
 {
     typedef Vel<T, VPL> L;
     typedef typename L::V VT;
-    const int tile = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const unsigned chunks = (V + 32 * VPL - 1) / (32 * VPL);
+    const int tile = blockIdx.x / chunks * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (tile >= __ldg(count)) return;
-    const int k = (blockIdx.x * 32 + lane) * VPL;
+    const int k = (blockIdx.x % chunks * 32 + lane) * VPL;
     if (k >= V) return;
     const int *tl = tiles + (size_t)tile * kTileInts;
     const T *cc = coef + (size_t)__ldg(tl) * S * V + k;
@@ -367,7 +368,7 @@ k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restric
     }
 }
 
-// Grid (velocity chunks, blocks of eight strips).
+// Blocks of eight strips, the chunks of velocities of a block one after the other.
 template <typename T, int VPL>
 __global__ void __launch_bounds__(256, 3)
 k_transport_strips(const T *__restrict__ f, T *__restrict__ g, const T *__restrict__ coef,
@@ -376,9 +377,10 @@ k_transport_strips(const T *__restrict__ f, T *__restrict__ g, const T *__restri
 {
     typedef Vel<T, VPL> L;
     typedef typename L::V VT;
-    const int strip = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const unsigned chunks = (V + 32 * VPL - 1) / (32 * VPL);
+    const int strip = blockIdx.x / chunks * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (strip >= __ldg(count)) return;
-    const int k = (blockIdx.x * 32 + lane) * VPL;
+    const int k = (blockIdx.x % chunks * 32 + lane) * VPL;
     if (k >= V) return;
     const int *st = strips + (size_t)strip * kStripInts;
     const T *cc = coef + (size_t)__ldg(st) * S * V + k;
@@ -566,11 +568,11 @@ static void launchTilesT(alebgk_ctx *c, const void *f, void *g, cudaStream_t st)
     const DeviceBuffers &d = c->d;
     // as many blocks as there could be tiles and strips: the plan's counts
     // stay on the device, and a refresh of the geometry changes no launch
-    const int chunks = (p.V + 32 * VPL - 1) / (32 * VPL);
-    k_transport_tiles<T, VPL><<<dim3(chunks, (p.N / 8 + 8) / 8), 256, 0, st>>>(
+    const unsigned chunks = (p.V + 32 * VPL - 1) / (32 * VPL);
+    k_transport_tiles<T, VPL><<<chunks * ((p.N / 8 + 8) / 8), 256, 0, st>>>(
         static_cast<const T *>(f), static_cast<T *>(g), static_cast<const T *>(d.coef), d.tiles,
         d.tileCount, p.S, p.V, p.ldf, d.sc);
-    k_transport_strips<T, VPL><<<dim3(chunks, (p.N / 4 + 8) / 8), 256, 0, st>>>(
+    k_transport_strips<T, VPL><<<chunks * ((p.N / 4 + 8) / 8), 256, 0, st>>>(
         static_cast<const T *>(f), static_cast<T *>(g), static_cast<const T *>(d.coef), d.strips,
         d.tileCount + 1, p.S, p.V, p.ldf, d.sc);
 }

@@ -62,6 +62,23 @@ def test_gather_by_tiles_equals_plain_gather_at_a_large_step(gpu, cells, precisi
     np.testing.assert_array_equal(out[0][1], out[1][1])
 
 
+def test_gather_beyond_524280_particles(gpu):
+    """The gather as its own kernel above 65 535 blocks of eight particles, against the march (the FP32 sums in
+    another order: as far apart as test_lattice_march_matches_gather allows)."""
+    c = ab.LatticeCase("cavity3d", 82, 4)
+    assert c.N > 8 * 65535
+    out = []
+    for transport in (1, 2):
+        cfg = c.config(32, 0, transport)
+        cfg.limiter = 0
+        s = ab.Solver(c, config=cfg)
+        s.cudaStep(1)
+        s.sync()
+        out.append(s.cudaDownloadFull()[0])
+        s.close()
+    assert _rel(out[0], out[1]) < 1e-5
+
+
 def _own_cloud(xyz, h, Nv, wall_first, box=None):
     """A case of these positions at spacing h: neighbours within 2.5 h (over the box's edges where it is given), the
     density varying from particle to particle.  With wall_first particle 0 is a wall particle."""
