@@ -217,7 +217,8 @@ __device__ __forceinline__ void classNode(const ClassArgs &a, int c, int n, doub
 
 // Per class: rep position (3), mesh velocity (3), wall state (7), then the
 // positions of slots 1..nsl-1 (3 each) at [c][S][3].  A block is of one
-// class, so its threads take one basis size.
+// class, so its threads take one basis size; a class's blocks follow one
+// another.
 // Bound: FP64 issue (about 280 operations a slot in the support and 4 000 for
 // the elimination, uncontracted).  Measured, cavity3d-cube Nx 40 Nv 10
 // (1 099 classes x 1 000 nodes, FP32 tables): quadratic 14.2 ms with both
@@ -229,8 +230,9 @@ k_class_tables(ClassArgs a, int order0, const int *__restrict__ boundary,
                const int *__restrict__ nsl, const double *__restrict__ rep,
                const double *__restrict__ slotPos, T *__restrict__ table, int *__restrict__ degen)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
+    const unsigned chunks = (a.V + blockDim.x - 1) / blockDim.x;
+    const int k = blockIdx.x % chunks * blockDim.x + threadIdx.x;
+    const int c = blockIdx.x / chunks;
     if (k >= a.V) return;
     const int ndim = a.dim, Nv = a.Nv, V = a.V;
     const bool bnd = boundary[c] != 0;
@@ -309,7 +311,8 @@ cudaError_t buildTablesDevice(const CoeffInput &in, const CoeffTables &cls, int 
         e = cudaMemsetAsync(table, 0, (size_t)ncls * S * V * (f64 ? 8 : 4), st);
     if (e == cudaSuccess)
     {
-        dim3 grid((V + 127) / 128, ncls);
+        // (classes in grid x: y would hold 65 535)
+        const unsigned grid = (unsigned)((V + 127) / 128) * ncls;
         if (f64)
             k_class_tables<double><<<grid, 128, 0, st>>>(a, order, dBnd, dNsl, dRep, dPos,
                                                          static_cast<double *>(table), dDeg);

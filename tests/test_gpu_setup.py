@@ -182,6 +182,25 @@ def test_device_mls_tables_equal_host_tables(name, kw, precision):
     b.cudaFreeCloud()
 
 
+def test_device_mls_tables_of_more_than_65535_classes(gpu):
+    """Every particle a class of its own, by its mesh velocity: bitwise the state that the host's tables give."""
+    from alebgk4paper_b200 import _abi
+    c = Case("cavity2d", 260, 4, -1.0, 1)
+    c.meshv[:, 0] = 1e-3 * np.arange(c.N) / c.N
+    out = []
+    for builder in (0, 1):
+        _abi.load().alebgk_set_coeff_builder(builder)
+        try:
+            s = Solver(c, precision=32)
+            s.cudaStep(1)
+            out.append(s.cudaDownloadFull()[0])
+            s.close()
+        finally:
+            _abi.load().alebgk_set_coeff_builder(0)
+    assert c.N > 65535
+    np.testing.assert_array_equal(out[0], out[1])
+
+
 def test_bad_neighbour_lists_are_refused_at_the_first_bad_particle(gpu):
     """The upload and the in-place geometry refresh check every neighbour
     list (counts within 0..ALEBGK_MAX_NEIGH, indices of other particles) and
