@@ -1082,10 +1082,7 @@ int alebgk_get_counters(alebgk_ctx *c, alebgk_counters *out)
     out->mass_before = s.sigma * s.massNew;
     out->error_word = s.err;
     out->transport_kernel = c->march.enabled ? 2 : 1;
-    // 3: the register rows of the FP32 grids up to Nv 10; the other forms of
-    // the row stage count as the streamed one
-    out->particle_kernel =
-        c->pStream ? (c->pRows && c->cfg.precision != 64 && c->sp.Nv <= 10 ? 3 : 2) : 1;
+    out->particle_kernel = c->pRows ? 3 : (c->pGroup ? 4 : (c->pStream ? 2 : 1));
     return ALEBGK_OK;
 }
 

@@ -153,7 +153,7 @@ struct alebgk_ctx
     bool pStream = false;
     int pStreamWpb = 0, pStreamBlocks = 0;
     size_t pStreamSmem = 0;
-    // Register-row form of the streamed stages (FP32, Nv <= 10): on, blocks.
+    // Register-row form of the streamed stages (Nv of an instance): on, blocks.
     bool pRows = false;
     int pRowsBlocks = 0;
     // Groups of rows (the other 3-D clouds); interior rows lead rowOrder.

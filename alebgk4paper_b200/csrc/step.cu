@@ -2662,12 +2662,14 @@ static cudaError_t prepareT(alebgk_ctx *c)
             }
         }
         // The register-row form of the same stages (Nv of an instance): the
-        // default, unless the shared-memory form is asked for.
+        // default, unless the shared-memory form is asked for (in FP64 by
+        // particle 2 too: its streamed rows are one warp per particle).
         c->pRows = false;
+        const bool streamAsked = c->cfg.particle == 3 || (sizeof(T) == 8 && c->cfg.particle == 2);
         // (Its staged rows are whole 16-byte units, the row stride.)
         const auto rk = rowsKernel<T>(p.Nv);
         const int pad = 16 / (int)sizeof(T);
-        if (e == cudaSuccess && c->pStream && c->cfg.particle != 3 && rk && p.dim == 3 &&
+        if (e == cudaSuccess && c->pStream && !streamAsked && rk && p.dim == 3 &&
             p.ldf == (p.V + pad - 1) / pad * pad)
         {
             const size_t smem = rowsSmem<T>(p.Nv);
@@ -2691,7 +2693,7 @@ static cudaError_t prepareT(alebgk_ctx *c)
         // and 168 us.)
         const int rows = groupRows(p, sizeof(T));
         if (e == cudaSuccess && !c->pRows && (sizeof(T) == 8 || !c->pStream) &&
-            c->cfg.particle != 3 && rows > 0)
+            !streamAsked && rows > 0)
         {
             set((const void *)k_particle_group<T>, (size_t)rows * p.ldf * sizeof(T));
             c->pGroup = e == cudaSuccess;

@@ -337,7 +337,7 @@ def run_ours(args):
     cnt0 = s.counters()
     kernels = {"transport": "k_march" if cnt0["transport_kernel"] == 2 else "k_transport",
                "particle": {1: "k_particle", 2: "k_particle_stream",
-                            3: "k_particle_rows"}[cnt0["particle_kernel"]]}
+                            3: "k_particle_rows", 4: "k_particle_group"}[cnt0["particle_kernel"]]}
     # Algorithmic bytes per update: the transport reads f once and writes it
     # once (FP32: 4 + 4 bytes); so does the particle stage.  The roofline is
     # the transport's, the step's single largest kernel.

@@ -67,11 +67,12 @@ typedef struct alebgk_config
     int transport;    /* 0 auto (lattice march when the cloud is a complete
                          lattice without bodies, else coefficient gather),
                          1 always gather, 2 require the march (FP32 only)    */
-    int particle;     /* 0 auto (streamed rows for a 3-D cloud whose rows fit,
-                         in FP32 as three row kernels; else one warp per
-                         particle), 1 always the general kernel, 2 require
-                         streamed rows (three row kernels in FP32), 3
-                         require streamed rows with one warp per particle     */
+    int particle;     /* 0 auto (3-D: rows in registers where they fit, else
+                         streamed rows or groups of rows in shared memory;
+                         else one warp per particle), 1 always the general
+                         kernel, 2 require streamed rows (in FP32 in
+                         registers where they fit), 3 require streamed rows
+                         in shared memory, one warp per particle              */
 } alebgk_config;
 
 /* The host cloud in SoA form.  Inputs for alebgk_upload; the download calls
@@ -110,8 +111,9 @@ typedef struct alebgk_counters
     int transport_kernel;     /* transport in use: 1 coefficient gather,
                                  2 lattice march                              */
     int particle_kernel;      /* particle stage in use: 1 warp per particle,
-                                 2 streamed rows, one warp per particle,
-                                 3 streamed rows, three row kernels           */
+                                 2 streamed rows in shared memory, one warp
+                                 per particle, 3 streamed rows in registers,
+                                 4 groups of rows in shared memory            */
 } alebgk_counters;
 
 /* ---- context --------------------------------------------------------- */
