@@ -546,15 +546,13 @@ namespace {
 // geometry arrays, stencil classes and slot lists (built on the device from
 // the uploaded geometry) and MLS tables (solved on the device) are written
 // over the old ones, and only buffers that must grow are reallocated; a
-// lattice's march is set up again.  Returns 1 (nothing done) where it does
-// not apply: tables the host builds.
-int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
+// lattice's march is set up again.  On a failure the context holds parts of
+// both geometries (refreshGeometryInPlace drops it).
+int refreshGeometry(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
 {
     StepParams &p = c->sp;
     const int N = p.N;
-    if (gCoeffBuilder == 1) return 1;
     const bool f64 = c->cfg.precision == 64;
-    if (const int r = checkNeighbours(c, cl, N)) return r;
     p.dt = dt;
     p.lam = dt / p.tau;
     p.c1 = 1.0 / (1.0 + p.lam);
@@ -663,6 +661,26 @@ int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
     c->geometryDirty = false;
     ++c->epoch;
     return ALEBGK_OK;
+}
+
+// refreshGeometry after its checks.  Returns 1 (nothing done) where it does
+// not apply: tables the host builds.  A refresh that fails midway (a buffer
+// that does not fit the memory) leaves the context as a failed full upload
+// does, not uploaded and without buffers: its step graphs, and those of a
+// batch by the epoch, would launch over what was freed.
+int refreshGeometryInPlace(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
+{
+    if (gCoeffBuilder == 1) return 1;
+    if (const int r = checkNeighbours(c, cl, c->sp.N)) return r;
+    const int r = refreshGeometry(c, cl, dt);
+    if (r != ALEBGK_OK)
+    {
+        cudaStreamSynchronize(c->stream);
+        freeBuffers(c);
+        ++c->epoch;
+        cudaGetLastError();      // (a failed allocation is no launch's error)
+    }
+    return r;
 }
 
 }  // namespace

@@ -205,7 +205,8 @@ int alebgk_slab_step(alebgk_slab *g, int nsteps)
     alebgk_ctx *c = g->ctx[0];
     const int n = (int)g->ctx.size();
     for (alebgk_ctx *x : g->ctx)
-        if (x->cur != c->cur) return failS(c, ALEBGK_ESTATE, "a slab left the lockstep");
+        if (!x->uploaded || x->cur != c->cur)
+            return failS(c, ALEBGK_ESTATE, "a slab left the lockstep");
     for (int s = 0; s < nsteps; ++s)
     {
         const int from = c->cur;

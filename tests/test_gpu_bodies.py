@@ -2,6 +2,8 @@
 Newton-Euler update (RigidBody/BodyDynamics.cpp:17-97, 352-638), against the
 compiled reference's own free-body step and against the rigid-motion
 formulas."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -232,3 +234,35 @@ def test_geometry_refresh_in_place_equals_full_upload(gpu, precision, case, Nx, 
         np.testing.assert_array_equal(g0, g1)
         np.testing.assert_array_equal(m0, m1)
         np.testing.assert_array_equal(st0, st1)
+
+
+@pytest.mark.parametrize("name,transport,left", [("cavity3d", 0, 256), ("cavity3d", 0, 1450), ("cavity3d", 1, 256),
+                                                 ("cavity3d-cube", 0, 256)])
+def test_refresh_that_does_not_fit_the_memory_drops_the_cloud(gpu, name, transport, left):
+    """A refresh that needs larger tables (every particle a class of its own, by its mesh velocity: 1 728 and more
+    classes x 81 slots x 1 000 nodes, 560 MB a table) than the device has memory for (`left` MB; at 1 450 both tables
+    fit and the march's own does not), after graphs of the old geometry ran: it fails, no step runs over what it
+    freed, and a new upload starts afresh."""
+    import torch
+    c = ab.Case(name, 12, 10, -1.0, 2, fixed_body=True)
+    s = ab.Solver(c, precision=32, transport=transport)
+    s.cudaStep(2)
+    s.sync()
+    still, c.meshv = c.meshv, 1e-3 * np.arange(3 * c.N).reshape(c.N, 3) / c.N
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (left << 20), dtype=torch.uint8, device="cuda")
+    with pytest.raises(ab.AlebgkError):
+        cl = c.cloud()
+        ab._check(s.lib.alebgk_upload_geometry(s.ctx, ctypes.byref(cl), s.dt), s.ctx)
+    with pytest.raises(ab.AlebgkError) as e:
+        s.cudaStep(1)
+    assert e.value.code == ab._abi.ESTATE
+    del hold
+    torch.cuda.empty_cache()
+    c.meshv = still
+    s.cudaUploadCloud(c)
+    s.cudaStep(2)
+    f = ab.Solver(c, precision=32, transport=transport)
+    f.cudaStep(2)
+    np.testing.assert_array_equal(s.cudaDownloadFull()[0], f.cudaDownloadFull()[0])
+    s.close(), f.close()
