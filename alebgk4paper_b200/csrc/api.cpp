@@ -553,6 +553,14 @@ int refreshGeometry(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
     StepParams &p = c->sp;
     const int N = p.N;
     const bool f64 = c->cfg.precision == 64;
+    DeviceBuffers &d = c->d;
+    // What the captured step graphs hold: the step parameters (by value, the
+    // time step among them) and the buffers the refresh may reallocate.  When
+    // none of them changes, the graphs stay valid and are kept.
+    unsigned char spBefore[sizeof(StepParams)];
+    std::memcpy(spBefore, &p, sizeof p);
+    const int interiorBefore = c->interiorRows;
+    const void *bufBefore[] = {d.coef, d.coefLin, d.slots, d.surfList, d.bodyIO};
     p.dt = dt;
     p.lam = dt / p.tau;
     p.c1 = 1.0 / (1.0 + p.lam);
@@ -565,15 +573,7 @@ int refreshGeometry(alebgk_ctx *c, const alebgk_cloud *cl, double dt)
     in.maxNeigh = ALEBGK_MAX_NEIGH;
     CoeffTables tb;
     std::string err;
-    DeviceBuffers &d = c->d;
     const size_t es = f64 ? 8 : 4;
-    // What the captured step graphs hold: the step parameters (by value) and
-    // the buffers the refresh may reallocate.  When none of them changes,
-    // the graphs stay valid and are kept.
-    unsigned char spBefore[sizeof(StepParams)];
-    std::memcpy(spBefore, &p, sizeof p);
-    const int interiorBefore = c->interiorRows;
-    const void *bufBefore[] = {d.coef, d.coefLin, d.slots, d.surfList, d.bodyIO};
     // Geometry first: the class keys are computed from the device copy.
     CK(cudaMemcpy(d.pos, cl->xyz, 24 * (size_t)N, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d.meshv, cl->meshv, 24 * (size_t)N, cudaMemcpyHostToDevice));

@@ -266,3 +266,21 @@ def test_refresh_that_does_not_fit_the_memory_drops_the_cloud(gpu, name, transpo
     f.cudaStep(2)
     np.testing.assert_array_equal(s.cudaDownloadFull()[0], f.cudaDownloadFull()[0])
     s.close(), f.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("name,Nx,Nv", [("cavity3d-cube", 12, 4), ("cavity2d", 12, 8), ("cavity3d", 9, 6)])
+def test_refresh_with_another_time_step(gpu, name, Nx, Nv, precision):
+    """The same geometry refreshed for half the time step after graphs of the whole one ran: bitwise the state of a
+    solver that was set up for half the step."""
+    c = ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True)
+    s, h = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision, dt=0.5 * c.dt)
+    s.cudaStep(2)
+    cl = c.cloud()
+    ab._check(s.lib.alebgk_upload_geometry(s.ctx, ctypes.byref(cl), 0.5 * c.dt), s.ctx)
+    g, m = np.ascontiguousarray(c.g), np.ascontiguousarray(c.macro)
+    for x in (s, h):
+        ab._check(x.lib.alebgk_upload_state(x.ctx, ab._dp(g), ab._dp(m)), x.ctx)
+        x.cudaStep(2)
+    np.testing.assert_array_equal(s.cudaDownloadFull()[0], h.cudaDownloadFull()[0])
+    s.close(), h.close()
