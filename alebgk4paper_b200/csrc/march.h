@@ -53,7 +53,8 @@ struct MarchPlan
 };
 
 // Detects the lattice and builds the plan; plan.ok is false when the cloud
-// is not a complete lattice with two-step stencils.
+// is not a complete lattice with two-step stencils, the same for all members of
+// a class.
 void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb,
                     const int *nbr, int maxNeigh, const CoeffTables &tb, MarchPlan &plan);
 

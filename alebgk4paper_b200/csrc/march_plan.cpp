@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <cstdint>
 #include <map>
 
 namespace alebgk {
@@ -74,6 +75,12 @@ void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb, const int
     auto coord = [&](int i, int &x, int &y, int &z) {
         x = i % nx; y = (i / nx) % ny; z = i / (nx * ny);
     };
+    // Every particle's set of offsets.  The table goes by the offsets of each
+    // class's representative, so a class with members that differ in them (a
+    // periodic lattice of three planes: a neighbour over the edge is two planes
+    // back, the same neighbour inside one on) or a list that names a neighbour
+    // twice is left to the gather.
+    std::vector<std::array<uint64_t, 2>> sets(N, {0, 0});
     int outside = 0;
 #pragma omp parallel for schedule(static) reduction(| : outside)
     for (int i = 0; i < N; ++i)
@@ -84,9 +91,14 @@ void buildMarchPlan(const double *xyz, int N, int dim, const int *nnb, const int
         {
             int xj, yj, zj;
             coord(nbr[(size_t)i * maxNeigh + s], xj, yj, zj);
-            outside |= templateIndex(xj - xi, yj - yi, zj - zi) < 0;
+            const int o = templateIndex(xj - xi, yj - yi, zj - zi);
+            const uint64_t bit = o < 0 ? 0 : uint64_t(1) << (o & 63);
+            uint64_t &set = sets[i][o >= 64];
+            outside |= o < 0 || (set & bit);
+            set |= bit;
         }
     }
+    for (int i = 0; i < N && !outside; ++i) outside = sets[i] != sets[tb.rep[tb.cls[i]]];
     if (outside) return;
 
     // Template offset -> slot of each class, from its representative.

@@ -79,14 +79,15 @@ def test_gather_beyond_524280_particles(gpu):
     assert _rel(out[0], out[1]) < 1e-5
 
 
-def _own_cloud(xyz, h, Nv, wall_first, box=None):
-    """A case of these positions at spacing h: neighbours within 2.5 h (over the box's edges where it is given), the
-    density varying from particle to particle.  With wall_first particle 0 is a wall particle."""
+def _own_cloud(xyz, h, Nv, wall_first=False, box=(0, 0, 0), reach=2.5):
+    """A case of these positions at spacing h: neighbours within reach h (over the box's edges where it has a length), the
+    density varying from particle to particle.  With wall_first particle 0 is a wall particle.  Returns the box's
+    lengths at the case's scale too."""
     from scipy.spatial import cKDTree
     c = copy.copy(ab.Case("cavity3d", 6, Nv, -1.0, 2))
     N = len(xyz)
     scale = c.params["radius"] / (2.5 * h)
-    near = cKDTree(xyz, boxsize=box).query_ball_point(xyz, 2.5 * h)
+    near = cKDTree(xyz, boxsize=box).query_ball_point(xyz, reach * h)
     c.N, c.xyz, c.meshv = N, np.ascontiguousarray(xyz * scale), np.zeros((N, 3))
     c.nnb, c.nbr = np.zeros(N, np.int32), np.zeros((N, _abi.MAX_NEIGH), np.int32)
     for i, js in enumerate(near):
@@ -99,16 +100,17 @@ def _own_cloud(xyz, h, Nv, wall_first, box=None):
     f = 1.0 + 0.01 * np.cos(np.arange(N))[:, None]
     c.g, c.macro = c.g[:1] * f, np.tile(c.macro[0], (N, 1))
     c.macro[:, 0] *= f[:, 0]
-    return c, scale
+    return c, [scale * b for b in box]
 
 
-def _assert_tiled_equals_plain(c, precision, box=0.0, tiles=True):
+def _assert_auto_equals_plain(c, precision, box=(0, 0, 0), tiles=True):
     out = []
     for transport in (0, 1):
         cfg = c.config(precision, 0, transport)
         for a in range(3):
-            cfg.periodic[a], cfg.L[a] = int(box > 0), box
+            cfg.periodic[a], cfg.L[a] = int(box[a] > 0), box[a]
         s = ab.Solver(c, config=cfg)
+        assert s.counters()["transport_kernel"] == 1
         if transport == 0:
             n = s.gather_counts()
             assert 8 * n[0] + 4 * n[1] + n[2] == c.N
@@ -130,7 +132,7 @@ def test_tiles_of_a_lattice_that_does_not_hold_the_first_particle(gpu, n, precis
     z, y, x = np.meshgrid(ax, ax, ax, indexing="ij")
     xyz = np.concatenate([np.zeros((1, 3)), np.column_stack([x.ravel(), y.ravel(), z.ravel()])])
     c, _ = _own_cloud(xyz, 1.0 / n, 4, True)
-    _assert_tiled_equals_plain(c, precision)
+    _assert_auto_equals_plain(c, precision)
 
 
 @pytest.mark.parametrize("precision", [32, 64])
@@ -140,8 +142,31 @@ def test_tiles_of_a_periodic_lattice(gpu, n, roll, precision):
     with an odd number of rows none overlaps another.  Rolled, the class's first particle lies inside."""
     ax = np.roll((np.arange(n) + 0.5) / n, -roll)
     z, y, x = np.meshgrid(ax, ax, ax, indexing="ij")
-    c, scale = _own_cloud(np.column_stack([x.ravel(), y.ravel(), z.ravel()]), 1.0 / n, 4, False, box=1.0)
-    _assert_tiled_equals_plain(c, precision, scale, tiles=roll > 0)
+    c, box = _own_cloud(np.column_stack([x.ravel(), y.ravel(), z.ravel()]), 1.0 / n, 4, box=(1, 1, 1))
+    _assert_auto_equals_plain(c, precision, box, tiles=roll > 0)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("shape", [(7, 6, 3), (3, 6, 7), (7, 3, 3)])
+def test_lattice_of_three_periodic_planes_is_gathered(gpu, shape, precision):
+    """In an axis of three periodic planes the neighbour over the edge is two planes back: particles of one class, whose
+    offsets differ from member to member (lists of the 26 next neighbours, whose offsets all lie in the march's
+    template)."""
+    axes = [(np.arange(k) + 0.5) / 10 for k in shape]
+    z, y, x = np.meshgrid(axes[2], axes[1], axes[0], indexing="ij")
+    c, box = _own_cloud(np.column_stack([x.ravel(), y.ravel(), z.ravel()]), 0.1, 4,
+                        box=[0.3 if k == 3 else 0 for k in shape], reach=1.8)
+    _assert_auto_equals_plain(c, precision, box, tiles=False)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_lattice_with_a_neighbour_listed_twice_is_gathered(gpu, precision):
+    """Both entries count, as in any other cloud."""
+    c = ab.Case("cavity3d", 9, 4, -1.0, 2)
+    i = int(np.nonzero(c.boundary == 0)[0][100])
+    c.nbr[i, c.nnb[i]] = c.nbr[i, 7]
+    c.nnb[i] += 1
+    _assert_auto_equals_plain(c, precision)
 
 
 @pytest.mark.parametrize("precision", [32, 64])
