@@ -341,6 +341,10 @@ static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool wi
         !cl->nnb || !cl->nbr || (withState && (!cl->g || !cl->macro)))
         return fail(c, ALEBGK_EINVAL, "alebgk_upload needs every cloud member");
     if (!(dt > 0)) return fail(c, ALEBGK_EINVAL, "dt must be > 0");
+    if (c->cfg.transport == 2 && c->cfg.precision == 64)
+        return fail(c, ALEBGK_EINVAL,
+                    "transport 2 requires the FP32 lattice march; an FP64 lattice marches by "
+                    "transport 0");
     CK(cudaSetDevice(c->cfg.device));
     CK(cudaStreamSynchronize(c->stream));
     freeBuffers(c);
@@ -511,7 +515,7 @@ static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool wi
                     "shared memory");
     if (const int r = setupMarch(c, cl, tb)) return r;
     if (const int r = setupTiles(c, in, tb)) return r;
-    if (c->cfg.transport == 2 && (!c->march.enabled || f64))
+    if (c->cfg.transport == 2 && !c->march.enabled)
         return fail(c, ALEBGK_EINVAL,
                     "the lattice march needs FP32 and a complete 3-D lattice cloud");
     c->bodyIdHost.assign(cl->body_id, cl->body_id + N);

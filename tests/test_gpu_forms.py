@@ -28,6 +28,14 @@ def test_fp64_march_equals_gather(gpu, Nx, Nv):
     assert _rel(ma[:, 0], mb[:, 0]) < 3 * 5 * 9 * 1.2e-16
 
 
+def test_required_march_is_refused_in_fp64(gpu):
+    """Transport 2 is the FP32 march: an FP64 context is refused by what it asks for, a cloud that is no lattice by what
+    it is."""
+    for name, precision, says in (("cavity3d", 64, "transport 0"), ("cavity3d-cube", 32, "complete 3-D lattice")):
+        with pytest.raises(ab.AlebgkError, match=says):
+            ab.Solver(ab.Case(name, 12, 4, -1.0, 2, fixed_body=True), precision=precision, transport=2)
+
+
 @pytest.mark.parametrize("precision", [32, 64])
 @pytest.mark.parametrize("name,Nx,Nv", [("cavity3d-cube", 12, 5), ("cavity3d-cube", 17, 6), ("cavity3d-sphere", 21, 4),
                                         ("cavity3d-cube", 24, 8)])
