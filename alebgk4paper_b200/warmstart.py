@@ -220,37 +220,34 @@ class WarmStartNet:
         def draw():
             return rng.permutation(n).astype(np.int32)
 
+        # The steps read the rows and indices on the network's own stream, which
+        # torch's allocator does not know: an epoch's indices, and at the end
+        # all of them, are released only once the steps are done.
+        perm, pos, log = None, n, []
         with ThreadPoolExecutor(1) as pool:
             ahead = pool.submit(draw) if left > 0 else None
-            log = self._fit_steps(x, y, n, steps, batch, lr, lr_final, log_every, wp, pool, draw,
-                                  ahead, left)
-        self._ok(self.lib.alebgk_net_sync(self.h))
-        return log
-
-    def _fit_steps(self, x, y, n, steps, batch, lr, lr_final, log_every, wp, pool, draw, ahead,
-                   left):
-        t = self.torch
-        perm, pos, log = None, n, []
-        for s in range(steps):
-            if pos + batch > n:
-                perm, left = ahead.result(), left - 1
-                ahead = pool.submit(draw) if left > 0 else None
-                # the steps read the indices on the network's own stream: the
-                # last epoch's are freed only once they are done
-                if s:
-                    self._ok(self.lib.alebgk_net_sync(self.h))
-                perm = self._dev(perm, t.int32)
-                pos = 0
-            ix = perm[pos:pos + batch]
-            pos += batch
-            cur = lr_final + 0.5 * (lr - lr_final) * (1 + math.cos(math.pi * s / max(1, steps)))
-            want = bool(log_every) and (s % log_every == 0 or s == steps - 1)
-            loss = ctypes.c_float()
-            self._ok(self.lib.alebgk_net_train_step(
-                self.h, x.data_ptr(), y.data_ptr(), ix.data_ptr(), int(ix.shape[0]), wp,
-                float(cur), 0.9, 0.999, 1e-8, ctypes.byref(loss) if want else None))
-            if want:
-                log.append((s, loss.value / ix.shape[0]))
+            try:
+                for s in range(steps):
+                    if pos + batch > n:
+                        drawn, left = ahead.result(), left - 1
+                        ahead = pool.submit(draw) if left > 0 else None
+                        if perm is not None:
+                            self._ok(self.lib.alebgk_net_sync(self.h))
+                        perm = self._dev(drawn, t.int32)
+                        pos = 0
+                    ix = perm[pos:pos + batch]
+                    pos += batch
+                    cur = lr_final + 0.5 * (lr - lr_final) * (1 + math.cos(math.pi * s / max(1, steps)))
+                    want = bool(log_every) and (s % log_every == 0 or s == steps - 1)
+                    loss = ctypes.c_float()
+                    self._ok(self.lib.alebgk_net_train_step(
+                        self.h, x.data_ptr(), y.data_ptr(), ix.data_ptr(), int(ix.shape[0]), wp,
+                        float(cur), 0.9, 0.999, 1e-8, ctypes.byref(loss) if want else None))
+                    if want:
+                        log.append((s, loss.value / ix.shape[0]))
+            finally:
+                done = self.lib.alebgk_net_sync(self.h)
+        self._ok(done)
         return log
 
     def close(self):

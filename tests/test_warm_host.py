@@ -108,3 +108,57 @@ def test_case_scalings_round_trip():
     scale, shift = ws.denormalise(c, mu, sd)
     back = shift + scale * ((t.astype(np.float64) - mu) / sd)
     assert np.allclose(back, mom, rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("n,batch,steps,fail_at", [(100, 32, 10, None), (64, 64, 3, None), (40, 64, 2, None),
+                                                   (100, 32, 10, 7)])
+def test_fit_keeps_its_indices_until_the_network_has_read_them(n, batch, steps, fail_at):
+    """The training steps run on the network's own stream: no index or row array of fit is released between a step that
+    reads it and the next synchronisation, on the way out and when a step fails too."""
+    import weakref
+
+    import torch
+    from alebgk4paper_b200.warmstart import WarmStartNet
+
+    pending, early, seen = set(), [], []
+
+    class Lib:
+        def alebgk_net_train_step(self, h, x, y, ix, rows, *rest):
+            seen.append((ix, rows))
+            pending.update(a for a, (lo, hi) in spans.items() if any(lo <= p < hi for p in (x, y, ix)))
+            return -2 if len(seen) - 1 == fail_at else 0
+
+        def alebgk_net_sync(self, h):
+            pending.clear()
+            return 0
+
+        def alebgk_net_last_error(self, h):
+            return b"planted"
+
+    spans = {}
+
+    def dev(a, dtype):
+        a = np.array(a, copy=True)
+        key = len(spans)
+        spans[key] = (a.ctypes.data, a.ctypes.data + a.nbytes)
+
+        def released():
+            if key in pending:
+                early.append(key)
+        weakref.finalize(a, released)
+        return torch.from_numpy(a)
+
+    net = WarmStartNet.__new__(WarmStartNet)
+    net.torch, net.lib, net.h, net._dev = torch, Lib(), None, dev
+    X, T = np.zeros((n, 4), np.float32), np.zeros((n, W.N_OUT), np.float32)
+    if fail_at is None:
+        net.fit(X, T, steps=steps, batch=batch, log_every=0)
+        assert len(seen) == steps and all(r == min(batch, n) for _, r in seen)
+    else:
+        try:
+            net.fit(X, T, steps=steps, batch=batch, log_every=0)
+        except RuntimeError as e:
+            assert "planted" in str(e)
+        else:
+            raise AssertionError("the failed step went unnoticed")
+    assert not early and not pending
