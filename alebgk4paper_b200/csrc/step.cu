@@ -1801,18 +1801,20 @@ k_sigma(const double *__restrict__ massPos, int N, double *partial, StepScalars 
 
 // Mass at the end of the step (the next step's massOld); the stored state
 // now carries the scale sigma.
+__device__ __forceinline__ void endStepMass(StepScalars *sc, double m)
+{
+    const double sigma = sc->sigma;
+    sc->massEnd = sigma * m;
+    sc->massOld = sc->massEnd;
+    sc->scale = sigma;
+    sc->steps += 1;
+}
+
 __global__ void __launch_bounds__(kRedThreads)
 k_mass_sum(const double *__restrict__ massEnd, int N, double *partial, StepScalars *sc)
 {
     double m;
-    if (gridSumLast(massEnd, N, partial, sc, &m))
-    {
-        const double sigma = sc->sigma;
-        sc->massEnd = sigma * m;
-        sc->massOld = sc->massEnd;
-        sc->scale = sigma;
-        sc->steps += 1;
-    }
+    if (gridSumLast(massEnd, N, partial, sc, &m)) endStepMass(sc, m);
 }
 
 // Applies sigma to the macros and runs moodCheck (Conservation.cpp:16-38,
@@ -1939,15 +1941,22 @@ k_mass_end(const double *__restrict__ massEnd, int N, double *partial, StepScala
 // arrays of N values): k_fixup and k_mass_end find nothing to do in nearly
 // every step, so their work goes to the last block of the kernel before them
 // (a ticket, as in gridSumLast).  Same operations and orders, same bits.
-//   k_sigma_fix   k_sigma, then k_fixup by its last block (lists of the few
-//                 rows without positive mass; with tau(rho, T) every row is
-//                 listed and k_fixup keeps its own launch)
+//   k_sigma_fix   k_sigma, then k_fixup by its last block when few rows are
+//                 listed
+//   k_fix_mass    k_mass_sum; when more are, k_fixup over the whole grid
+//                 before it, and the sum by the last block
 //   k_late        k_recollide, then k_mass_end by its last block
+// (With tau(rho, T) every row is listed and k_fixup keeps its own launch.)
 // Measured, a step alone: cavity2d Nx 20 Nv 16 FP64 50.6 -> 49.2 us, cavity3d
 // Nx 27 Nv 12 FP32 778 -> 771 us for two.  Merging the whole chain into the
 // redo's last block was slower: 296 blocks' fences in every step, and sums on
 // one SM (96 cavities: 18.9 ms a 10 steps against 16.2).
 // ---------------------------------------------------------------------------
+// Rows that k_sigma_fix's last block takes: one round of its warps, as long as
+// k_fixup itself would take.  More go over the grid: a step of an empty cavity3d
+// Nx 40 Nv 10 (54 872 rows) takes 158 ms by one block, 1.2 this way.
+constexpr int kFixupRows = kNT / 32;
+
 template <typename T>
 __device__ __noinline__ void lateFixup(const ParticleArgs<T> &a, const StepParams &p)
 {
@@ -1967,60 +1976,99 @@ k_sigma_fix(ParticleArgs<T> a, StepParams p, double *partial)
     {
         sc->massNew = m;
         sc->sigma = (m > 1.0e-30) ? sc->massOld / m : 1.0;
-        mine = sc->ndeg > 0;
+        mine = sc->ndeg > 0 && sc->ndeg <= kFixupRows;
     }
     __syncthreads();
     if (mine) lateFixup<T>(a, p);
 }
 
-// The sum of a[0..N) by one block, in the order of gridSumLast over
-// kRedBlocks blocks; every thread receives it.
-__device__ double blockGridSum(const double *a, int N, double *sh)
+// The sum of a[0..N) by one block, in the order of gridSumLast over kRedBlocks
+// blocks.  A warp stands in for every eighth of them, its lanes for those of
+// all the block's warps at once, so that their loads overlap.  Complete in
+// thread 0.
+__device__ __noinline__ double blockGridSum(const double *a, int N, double *sh)
 {
-    constexpr int stride = kRedBlocks * kRedThreads;
-    double total = 0.0;
-    for (int b = 0; b < kRedBlocks; ++b)
+    constexpr int stride = kRedBlocks * kRedThreads, W = kRedThreads / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int b = warp; b < kRedBlocks; b += W)
     {
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        int i = b * kRedThreads + threadIdx.x;
-        for (; i + 3 * stride < N; i += 4 * stride)
-        {
-            s0 += __ldcg(a + i);
-            s1 += __ldcg(a + i + stride);
-            s2 += __ldcg(a + i + 2 * stride);
-            s3 += __ldcg(a + i + 3 * stride);
-        }
-        for (; i < N; i += stride) s0 += __ldcg(a + i);
-        double v[1] = {(s0 + s1) + (s2 + s3)};
-        blockSums<1>(v, sh);
-        total += v[0];
+        double v[W][4];
+#pragma unroll
+        for (int w = 0; w < W; ++w) v[w][0] = v[w][1] = v[w][2] = v[w][3] = 0.0;
+        // four interleaved partial sums; an incomplete round of four goes to the first
+        for (int i0 = b * kRedThreads + lane; i0 < N; i0 += 4 * stride)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int w = 0; w < W; ++w)
+                {
+                    const int i = i0 + 32 * w;
+                    const double x = i + q * stride < N ? __ldcg(a + i + q * stride) : 0.0;
+                    if (q == 0 || i + 3 * stride < N) v[w][q] += x;
+                    else v[w][0] += x;
+                }
+        double total = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) total += warpSum((v[w][0] + v[w][1]) + (v[w][2] + v[w][3]));
+        if (lane == 0) sh[b] = total;
     }
+    __syncthreads();
+    double total = 0.0;
+    if (threadIdx.x == 0)
+        for (int b = 0; b < kRedBlocks; ++b) total += sh[b];
     return total;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kNT)
-k_late(T *__restrict__ g, StepParams p, const int *__restrict__ boundary,
-       double *__restrict__ macNew, double *massEnd, StepScalars *sc)
+// Ticket of a grid whose blocks have done their part: true in every thread of
+// the last one, which sees what the others wrote (and sets redCount back).
+__device__ bool lastBlock(StepScalars *sc)
 {
-    static_assert(kRedThreads == kNT, "one block size");
-    if (sc->moodfail == 0) return;
-    __shared__ double sh[32];
     __shared__ bool last;
-    k_recollide_body(g, p, boundary, macNew, massEnd, sc, blockIdx.x, gridDim.x);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0)
     {
         last = atomicAdd(&sc->redCount, 1u) == gridDim.x - 1;
         __threadfence();
+        if (last) sc->redCount = 0;
     }
     __syncthreads();
-    if (!last) return;
+    return last;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads)
+k_fix_mass(ParticleArgs<T> a, StepParams p, double *partial)
+{
+    StepScalars *sc = a.sc;
+    double m;
+    if (sc->ndeg <= kFixupRows)
+    {
+        if (blockIdx.x < kRedBlocks &&
+            gridSumLast(a.massEnd, p.N, partial, sc, &m, blockIdx.x, kRedBlocks))
+            endStepMass(sc, m);
+        return;
+    }
+    __shared__ double sh[kRedBlocks];
+    k_fixup_body<T>(a, p, blockIdx.x, gridDim.x);
+    if (!lastBlock(sc)) return;
+    m = blockGridSum(a.massEnd, p.N, sh);
+    if (threadIdx.x == 0) endStepMass(sc, m);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kNT, 3)
+k_late(T *__restrict__ g, StepParams p, const int *__restrict__ boundary,
+       double *__restrict__ macNew, double *massEnd, StepScalars *sc)
+{
+    static_assert(kRedThreads == kNT, "one block size");
+    if (sc->moodfail == 0) return;
+    __shared__ double sh[kRedBlocks];
+    k_recollide_body(g, p, boundary, macNew, massEnd, sc, blockIdx.x, gridDim.x);
+    if (!lastBlock(sc)) return;
     const double m = blockGridSum(massEnd, p.N, sh);
     if (threadIdx.x == 0)
     {
-        sc->redCount = 0;
         sc->massEnd = sc->sigma * m;
         sc->massOld = sc->massEnd;
     }
@@ -2573,7 +2621,8 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev, bool alone)
     else k_redo<T, 1><<<listBlocks, kNT, rowBytes, st>>>(pa, p);
     mark();
     const bool merged = !ev;      // (timed stages need launches of their own)
-    if (merged && !p.tauVar)
+    const bool mergedFix = merged && !p.tauVar;
+    if (mergedFix)
         k_sigma_fix<T><<<kRedBlocks, kRedThreads, 0, st>>>(pa, p, d.redPartial);
     else
     {
@@ -2582,7 +2631,11 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev, bool alone)
         k_fixup<T><<<min(pBlocks, 296), kNT, 0, st>>>(pa, p);
     }
     mark();
-    k_mass_sum<<<kRedBlocks, kRedThreads, 0, st>>>(d.massEnd, p.N, d.redPartial, d.sc);
+    if (mergedFix)
+        k_fix_mass<T><<<max(kRedBlocks, min(pBlocks, 296)), kRedThreads, 0, st>>>(pa, p,
+                                                                                  d.redPartial);
+    else
+        k_mass_sum<<<kRedBlocks, kRedThreads, 0, st>>>(d.massEnd, p.N, d.redPartial, d.sc);
     mark();
     k_scale_mood<<<(p.N + 255) / 256, 256, 0, st>>>(p, d.boundary, macB, d.minG, d.mood, d.sc);
     mark();

@@ -252,6 +252,60 @@ def test_merged_end_of_step_equals_separate_launches(gpu, name, Nx, Nv, precisio
         assert ca[k] == cb[k], k
 
 
+def _merged_and_separate_steps(c, precision, limiter, steps):
+    """The state and counters after steps of the merged chain; bitwise those of the single kernels."""
+    cfg = c.config(precision)
+    cfg.limiter = limiter
+    a, b = ab.Solver(c, config=cfg), ab.Solver(c, config=cfg)
+    if c.dim == 2:
+        a.set_launch(256, 0), b.set_launch(256, 0)
+    a.cudaStep(steps)
+    ms = (ctypes.c_float * _abi.NSTAGES)()
+    ab._check(b.lib.alebgk_profile_steps(b.ctx, steps, ms), b.ctx)
+    (ga, ma), (gb, mb), ca = a.cudaDownloadFull(), b.cudaDownloadFull(), a.counters()
+    np.testing.assert_array_equal(ga, gb)
+    np.testing.assert_array_equal(ma, mb)
+    assert ca == b.counters()
+    a.close(), b.close()
+    return ga, ma, ca
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("limiter", [0, 2])
+@pytest.mark.parametrize("name,Nx,Nv,radius", [("cavity2d", 16, 8, 1.5), ("cavity2d", 16, 8, 99.0),
+                                               ("cavity3d", 12, 6, 2.1), ("cavity3d", 12, 6, 5.0)])
+def test_merged_end_of_step_finishes_rows_without_mass(gpu, name, Nx, Nv, radius, limiter, precision):
+    """A ball of empty rows, of which one to eight rows come out of the first transport without positive mass (the mass
+    sum's last block finishes them), or more (the whole grid does): like the single kernels, and like the oracle."""
+    from oracle.oracle import Oracle
+    from test_mls_tables import _tables
+    c = ab.Case(name, Nx, Nv, -1.0, 2)
+    inner = np.nonzero(c.boundary == 0)[0]
+    c.g[np.linalg.norm(c.xyz - c.xyz[inner[len(inner) // 2]], axis=1) < radius * c.params["dx"]] = 0
+    cls, nslot, slots, coef, V = _tables(c)
+    empty = sum(not (coef[cls[i], :nslot[i]] * c.g[slots[i, :nslot[i]], :V]).sum() > 0 for i in inner)
+    assert 1 <= empty <= 8 if radius < 3 else empty > 8
+    g, m, _ = _merged_and_separate_steps(c, precision, limiter, 1)
+    if precision == 64:
+        o = Oracle.from_case(c, limiter=limiter)
+        o.step(1)
+        assert np.abs(g - o.g).max() <= 1e-10 * np.abs(o.g).max()
+        assert np.abs(m[:, 0] - o.macro[:, 0]).max() <= 1e-10 * np.abs(o.macro[:, 0]).max()
+    _merged_and_separate_steps(c, precision, limiter, 3)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("name,Nx,Nv", [("cavity2d", 12, 8), ("cavity2d", 65, 6), ("cavity3d", 12, 6),
+                                        ("cavity3d", 27, 4)])
+def test_merged_end_of_step_after_a_failed_moodcheck(gpu, name, Nx, Nv, precision):
+    """The second collision and the end mass by its last block: like the single kernels."""
+    c = ab.Case(name, Nx, Nv, -1.0, 2)
+    i = int(np.nonzero(c.boundary == 0)[0][20])
+    c.g[i] = -50.0 * np.abs(c.g[i])
+    assert _merged_and_separate_steps(c, precision, 2, 1)[2]["mood_fail"] == 1
+    _merged_and_separate_steps(c, precision, 2, 3)
+
+
 @pytest.mark.parametrize("precision", [32, 64])
 @pytest.mark.parametrize("Nx,Nv", [(5, 6), (12, 15), (34, 6), (35, 6), (42, 8), (43, 8), (20, 28)])
 def test_small_2d_form_equals_plain_form(gpu, Nx, Nv, precision):
