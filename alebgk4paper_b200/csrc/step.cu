@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "ctx.h"
 #include "mbar.cuh"
@@ -1353,29 +1354,39 @@ k_particle_rows(ParticleArgs<T> a, StepParams p)
             bulkLoad(b ? rowBuf[0] : rowBuf[1], a.g + (size_t)inext * p.ldf, kRowBytes,
                      &rowBar[warp][b ^ 1]);
         }
-        T s0 = T(0), sn = T(0), sx = T(0), sy = T(0), sz = T(0), se = T(0);
+        // FP32 rows of up to 10^3 sum a lane's lines in FP32, and their negative
+        // part in one chain.  Longer ones (five and seven lines a lane) combine
+        // the lines in FP64: the relative error (rms) of a sum of 60 values is
+        // 2.4e-8 this way, 3.1e-8 in the streamed rows' four chains, 4.6e-8 line
+        // by line in FP32, 1.2e-7 in one chain.
+        constexpr bool inT = NV <= 10;
+        typedef std::conditional_t<inT, T, double> A;
+        A s0 = A(0), sn = A(0), sx = A(0), sy = A(0), sz = A(0), se = A(0);
 #pragma unroll
         for (int j = 0; j < LPL; ++j)
         {
             const int L = lane + 32 * j;
-            T ls = T(0), lx = T(0), le = T(0);
+            T ls = T(0), ln = T(0), lx = T(0), le = T(0);
 #pragma unroll
             for (int q = 0; q < NV; ++q)
             {
                 const T xp = fmax(x[j][q], T(0));
+                const T xn = x[j][q] - xp;   // the negative part; not finite if x is not
                 ls += xp;
-                sn += x[j][q] - xp;      // the negative part; not finite if x is not
+                if constexpr (inT) sn += xn;
+                else ln += xn;
                 lx = fma(vx[q], xp, lx);
                 le = fma(vx[q] * vx[q], xp, le);
             }
+            if constexpr (!inT) sn += ln;
             if (L < LINES)
             {
                 const T vy = velT[L % NV], vz = velT[L / NV];
                 s0 += ls;
                 sx += lx;
-                sy = fma(vy, ls, sy);
-                sz = fma(vz, ls, sz);
-                se += le + (vy * vy + vz * vz) * ls;
+                sy = fma(A(vy), A(ls), sy);
+                sz = fma(A(vz), A(ls), sz);
+                se += le + A(vy * vy + vz * vz) * A(ls);
             }
         }
         double r6[6] = {(double)s0, (double)sn, (double)sx, (double)sy, (double)sz, (double)se};
