@@ -23,7 +23,7 @@ namespace {
 
 struct ClassArgs
 {
-    int dim, Nv, V, S, mlsOrder;
+    int dim, Nv, V, S, ncls, mlsOrder;
     double dt, h, vmin, dv;
     int periodic[3];
     double L[3];
@@ -217,8 +217,7 @@ __device__ __forceinline__ void classNode(const ClassArgs &a, int c, int n, doub
 
 // Per class: rep position (3), mesh velocity (3), wall state (7), then the
 // positions of slots 1..nsl-1 (3 each) at [c][S][3].  A block is of one
-// class, so its threads take one basis size; a class's blocks follow one
-// another.
+// class (grid y and z), so its threads take one basis size.
 // Bound: FP64 issue (about 280 operations a slot in the support and 4 000 for
 // the elimination, uncontracted).  Measured, cavity3d-cube Nx 40 Nv 10
 // (1 099 classes x 1 000 nodes, FP32 tables): quadratic 14.2 ms with both
@@ -230,10 +229,9 @@ k_class_tables(ClassArgs a, int order0, const int *__restrict__ boundary,
                const int *__restrict__ nsl, const double *__restrict__ rep,
                const double *__restrict__ slotPos, T *__restrict__ table, int *__restrict__ degen)
 {
-    const unsigned chunks = (a.V + blockDim.x - 1) / blockDim.x;
-    const int k = blockIdx.x % chunks * blockDim.x + threadIdx.x;
-    const int c = blockIdx.x / chunks;
-    if (k >= a.V) return;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = blockIdx.z * gridDim.y + blockIdx.y;
+    if (k >= a.V || c >= a.ncls) return;
     const int ndim = a.dim, Nv = a.Nv, V = a.V;
     const bool bnd = boundary[c] != 0;
     const int order = bnd ? 1 : order0;
@@ -288,7 +286,7 @@ cudaError_t buildTablesDevice(const CoeffInput &in, const CoeffTables &cls, int 
             for (int q = 0; q < 3; ++q) pos[((size_t)c * S + s) * 3 + q] = in.xyz[3 * (size_t)sl[s] + q];
     }
     ClassArgs a{};
-    a.dim = in.dim; a.Nv = in.Nv; a.V = V; a.S = S; a.mlsOrder = order;
+    a.dim = in.dim; a.Nv = in.Nv; a.V = V; a.S = S; a.ncls = ncls; a.mlsOrder = order;
     a.dt = in.dt; a.h = in.h; a.vmin = in.vmin; a.dv = in.dv;
     for (int q = 0; q < 3; ++q) { a.periodic[q] = in.periodic[q] ? 1 : 0; a.L[q] = in.L[q]; }
     int *dBnd = nullptr, *dNsl = nullptr, *dDeg = nullptr;
@@ -311,8 +309,7 @@ cudaError_t buildTablesDevice(const CoeffInput &in, const CoeffTables &cls, int 
         e = cudaMemsetAsync(table, 0, (size_t)ncls * S * V * (f64 ? 8 : 4), st);
     if (e == cudaSuccess)
     {
-        // (classes in grid x: y would hold 65 535)
-        const unsigned grid = (unsigned)((V + 127) / 128) * ncls;
+        const dim3 grid = yzGrid((V + 127) / 128, ncls);
         if (f64)
             k_class_tables<double><<<grid, 128, 0, st>>>(a, order, dBnd, dNsl, dRep, dPos,
                                                          static_cast<double *>(table), dDeg);

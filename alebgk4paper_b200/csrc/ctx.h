@@ -182,6 +182,15 @@ struct alebgk_ctx
 
 namespace alebgk {
 
+// Grid of nx blocks in x and any number n >= 1 of rows of them: in y, which holds
+// 65 535, and z; a kernel's row is blockIdx.z * gridDim.y + blockIdx.y (the last
+// ones may lie past n).
+inline dim3 yzGrid(unsigned nx, unsigned n)
+{
+    const unsigned y = n < 65535u ? n : 65535u;
+    return dim3(nx, y, (n + y - 1) / y);
+}
+
 // Tiles of the gather transport (tiles.cu): the plan of the uploaded cloud,
 // the int words of the lists of N particles, and the transport of the tiles and
 // strips.

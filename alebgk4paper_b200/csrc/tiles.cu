@@ -297,7 +297,7 @@ __device__ __forceinline__ void unroll3(F &&f)
     unroll3Impl(std::make_integer_sequence<int, M>{}, f);
 }
 
-// Blocks of eight tiles, the chunks of velocities of a block one after the other.
+// Grid (velocity chunks, blocks of eight tiles in y and z).
 template <typename T, int VPL>
 __global__ void __launch_bounds__(256, 2)
 k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restrict__ coef,
@@ -306,10 +306,10 @@ k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restric
 {
     typedef Vel<T, VPL> L;
     typedef typename L::V VT;
-    const unsigned chunks = (V + 32 * VPL - 1) / (32 * VPL);
-    const int tile = blockIdx.x / chunks * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int tile = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (tile >= __ldg(count)) return;
-    const int k = (blockIdx.x % chunks * 32 + lane) * VPL;
+    const int k = (blockIdx.x * 32 + lane) * VPL;
     if (k >= V) return;
     const int *tl = tiles + (size_t)tile * kTileInts;
     const T *cc = coef + (size_t)__ldg(tl) * S * V + k;
@@ -368,7 +368,7 @@ k_transport_tiles(const T *__restrict__ f, T *__restrict__ g, const T *__restric
     }
 }
 
-// Blocks of eight strips, the chunks of velocities of a block one after the other.
+// Grid (velocity chunks, blocks of eight strips in y and z).
 template <typename T, int VPL>
 __global__ void __launch_bounds__(256, 3)
 k_transport_strips(const T *__restrict__ f, T *__restrict__ g, const T *__restrict__ coef,
@@ -377,10 +377,10 @@ k_transport_strips(const T *__restrict__ f, T *__restrict__ g, const T *__restri
 {
     typedef Vel<T, VPL> L;
     typedef typename L::V VT;
-    const unsigned chunks = (V + 32 * VPL - 1) / (32 * VPL);
-    const int strip = blockIdx.x / chunks * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int strip = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (strip >= __ldg(count)) return;
-    const int k = (blockIdx.x % chunks * 32 + lane) * VPL;
+    const int k = (blockIdx.x * 32 + lane) * VPL;
     if (k >= V) return;
     const int *st = strips + (size_t)strip * kStripInts;
     const T *cc = coef + (size_t)__ldg(st) * S * V + k;
@@ -569,10 +569,10 @@ static void launchTilesT(alebgk_ctx *c, const void *f, void *g, cudaStream_t st)
     // as many blocks as there could be tiles and strips: the plan's counts
     // stay on the device, and a refresh of the geometry changes no launch
     const unsigned chunks = (p.V + 32 * VPL - 1) / (32 * VPL);
-    k_transport_tiles<T, VPL><<<chunks * ((p.N / 8 + 8) / 8), 256, 0, st>>>(
+    k_transport_tiles<T, VPL><<<yzGrid(chunks, (p.N / 8 + 8) / 8), 256, 0, st>>>(
         static_cast<const T *>(f), static_cast<T *>(g), static_cast<const T *>(d.coef), d.tiles,
         d.tileCount, p.S, p.V, p.ldf, d.sc);
-    k_transport_strips<T, VPL><<<chunks * ((p.N / 4 + 8) / 8), 256, 0, st>>>(
+    k_transport_strips<T, VPL><<<yzGrid(chunks, (p.N / 4 + 8) / 8), 256, 0, st>>>(
         static_cast<const T *>(f), static_cast<T *>(g), static_cast<const T *>(d.coef), d.strips,
         d.tileCount + 1, p.S, p.V, p.ldf, d.sc);
 }
