@@ -158,8 +158,8 @@ int alebgk_create(const alebgk_config *cfg, alebgk_ctx **out)
         return fail(nullptr, ALEBGK_EINVAL, "mls_order must be 1 or 2");
     if (cfg->limiter != 0 && cfg->limiter != 2)
         return fail(nullptr, ALEBGK_EINVAL, "limiter must be 0 (none) or 2 (MOOD)");
-    if (cfg->transport < 0 || cfg->transport > 2)
-        return fail(nullptr, ALEBGK_EINVAL, "the transport selector is 0, 1 or 2");
+    if (cfg->transport < 0 || cfg->transport > 3)
+        return fail(nullptr, ALEBGK_EINVAL, "the transport selector is 0, 1, 2 or 3");
     if (cfg->particle < 0 || cfg->particle > 3)
         return fail(nullptr, ALEBGK_EINVAL, "the particle selector is 0, 1, 2 or 3");
     if (!(cfg->tau > 0) || !(cfg->R > 0) || !(cfg->dv > 0) || !(cfg->radius > 0))
@@ -262,7 +262,7 @@ static int setupMarch(alebgk_ctx *c, const alebgk_cloud *cl, const CoeffTables &
     std::string err;
     bool anyBody = false;
     for (int i = 0; i < N && !anyBody; ++i) anyBody = cl->body_id[i] >= 0;
-    if (c->cfg.transport != 1 && !anyBody)
+    if ((c->cfg.transport == 0 || c->cfg.transport == 2) && !anyBody)
     {
         MarchPlan plan;
         buildMarchPlan(cl->xyz, N, p.dim, cl->nnb, cl->nbr, ALEBGK_MAX_NEIGH, tb, plan);
@@ -312,14 +312,15 @@ static int setupMarch(alebgk_ctx *c, const alebgk_cloud *cl, const CoeffTables &
     return ALEBGK_OK;
 }
 
-// The gather transport's tiles of a 3-D cloud that does not march, unless the
-// plain gather is asked for.
+// The gather transport's tiles of a 3-D cloud that does not march, where they pay
+// (or wherever there are any, when asked for).
 static int setupTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb)
 {
     DeviceBuffers &d = c->d;
     const size_t N = c->sp.N;
-    c->tiled = c->sp.dim == 3 && !c->march.enabled && c->cfg.transport == 0;
-    if (!c->tiled) return ALEBGK_OK;
+    c->tiled = false;
+    if (c->sp.dim != 3 || c->march.enabled || (c->cfg.transport != 0 && c->cfg.transport != 3))
+        return ALEBGK_OK;
     if (!d.tiles)
     {
         CK(dalloc(&d.tiles, tileInts((int)N)));
@@ -331,6 +332,9 @@ static int setupTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb
         CK(dalloc(&d.tileCovered, N));
     }
     CK(buildTiles(c, in, tb));
+    int n[3];
+    CK(cudaMemcpy(n, d.tileCount, sizeof n, cudaMemcpyDeviceToHost));
+    c->tiled = c->cfg.transport == 3 ? n[0] + n[1] > 0 : tilesPay(c, n[0], n[1]);
     return ALEBGK_OK;
 }
 

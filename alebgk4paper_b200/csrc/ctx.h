@@ -139,6 +139,7 @@ struct alebgk_ctx
     bool uploaded = false;
     int ncls = 0;
     int sms = 0;                 // multiprocessors of the device
+    int gatherWave = 0;          // blocks of k_transport that the device holds at once
     bool tiled = false;          // the gather transport runs by tiles (tiles.cu)
     int degenerateParticles = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -200,6 +201,8 @@ cudaError_t buildTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &t
 size_t tileInts(int N);
 size_t stripInts(int N);
 cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st);
+// Whether a plan of so many tiles and strips is faster than the plain gather (step.cu).
+bool tilesPay(const alebgk_ctx *c, int tiles, int strips);
 
 // Launch wrappers (step.cu).
 cudaError_t prepareKernels(alebgk_ctx *c);

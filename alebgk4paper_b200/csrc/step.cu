@@ -2525,6 +2525,21 @@ static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
     return cudaGetLastError();
 }
 
+// Tiles and strips are launches of their own before the gather of the rest, each
+// at least as long as one wave of blocks.  So they pay where the plain gather
+// takes more than a wave, and they take at least half a wave off it.  Measured,
+// a step of cavity3d-cube by the plain gather and with tiles, FP32 (a wave is
+// 740 blocks of eight particles and a chunk) and FP64 (592): Nx 16 Nv 6 (523
+// blocks) 80 and 89 us, 164 and 184; Nx 16 Nv 8 (1 046) 147 and 133, 244 and 211;
+// Nx 8 Nv 16 (1 204, of them 224 in strips) 178 and 186, 328 and 329; Nx 12 Nv 10
+// (908, 396 in tiles and strips) 147 and 139, 255 and 217.
+bool tilesPay(const alebgk_ctx *c, int tiles, int strips)
+{
+    const long long nch = transportChunks(c->sp.V), per = kNT / 32;
+    return nch * (c->sp.N / per) > c->gatherWave &&
+           2 * nch * ((8LL * tiles + 4LL * strips) / per) > c->gatherWave;
+}
+
 // The small 2-D form where one wave holds the whole cloud, else none; sw = its
 // particles per block.  Measured, a step inside the line: FP64 Nx 20 Nv 16
 // 39.9 -> 30.7 us, Nx 33 Nv 20 57.8 -> 45.1; FP32 Nx 20 Nv 16 27.1 -> 25.6,
@@ -2682,6 +2697,10 @@ static cudaError_t prepareT(alebgk_ctx *c)
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
+    int gatherBlocks = 0;
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gatherBlocks, k_transport<T>, kNT, 0);
+    c->gatherWave = c->sms * gatherBlocks;
     auto set = [&](const void *fn, size_t bytes) {
         cudaFuncAttributes fa{};
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);

@@ -66,7 +66,9 @@ typedef struct alebgk_config
     double L[3];      /* periodic lengths                                     */
     int transport;    /* 0 auto (lattice march when the cloud is a complete
                          lattice without bodies, else coefficient gather),
-                         1 always gather, 2 require the march (FP32 only)    */
+                         1 always the plain gather, 2 require the march (FP32
+                         only), 3 always gather, by tiles wherever a 3-D cloud
+                         has any (0 takes them where they are faster)         */
     int particle;     /* 0 auto (3-D: rows in registers where they fit, else
                          streamed rows or groups of rows in shared memory;
                          else one warp per particle), 1 always the general

@@ -44,11 +44,23 @@ def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
     remainders, bodies in the middle: every particle sums its slots in the same order, so the states are
     the same bits."""
     c = ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True)
-    a, b = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision, transport=1)
+    a, b = ab.Solver(c, precision=precision, transport=3), ab.Solver(c, precision=precision, transport=1)
+    assert min(a.gather_counts()) > 0 and b.gather_counts() == (0, 0, c.N)
     a.cudaStep(3), b.cudaStep(3)
     (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
     np.testing.assert_array_equal(ga, gb)
     np.testing.assert_array_equal(ma, mb)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("name,Nx,Nv,tiled", [("cavity3d-cube", 12, 6, False), ("cavity3d-cube", 8, 16, False),
+                                              ("cavity3d-cube", 24, 6, True), ("cavity3d-sphere", 24, 4, True)])
+def test_tiles_are_taken_where_they_pay(gpu, name, Nx, Nv, tiled, precision):
+    """Not where one wave of the plain gather holds the cloud, or few particles are in tiles and strips; a cloud that
+    grows or shrinks past the line would change its graphs with it."""
+    s = ab.Solver(ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True), precision=precision)
+    assert (s.gather_counts()[0] > 0) == tiled
+    s.close()
 
 
 @pytest.mark.parametrize("precision", [32, 64])
@@ -59,10 +71,11 @@ def test_gather_by_tiles_equals_plain_gather_at_a_large_step(gpu, cells, precisi
     c = ab.Case("cavity3d-cube", 17, 6, -1.0, 2, fixed_body=True)
     c.dt = cells * c.params["dx"] / max(abs(c.params["vmin"]), c.params["vmin"] + (c.Nv - 1) * c.params["dv"])
     out = []
-    for transport in (0, 1):
+    for transport in (3, 1):
         cfg = c.config(precision, 0, transport)
         cfg.limiter = 0
         s = ab.Solver(c, config=cfg)
+        assert transport == 1 or s.gather_counts()[0] > 0
         s.cudaStep(1)
         out.append(s.cudaDownloadFull())
         s.close()
@@ -113,21 +126,21 @@ def _own_cloud(xyz, h, Nv, wall_first=False, box=(0, 0, 0), reach=2.5):
 
 def _assert_auto_equals_plain(c, precision, box=(0, 0, 0), tiles=True):
     out = []
-    for transport in (0, 1):
+    for transport in (0, 3, 1):
         cfg = c.config(precision, 0, transport)
         for a in range(3):
             cfg.periodic[a], cfg.L[a] = int(box[a] > 0), box[a]
         s = ab.Solver(c, config=cfg)
         assert s.counters()["transport_kernel"] == 1
-        if transport == 0:
-            n = s.gather_counts()
-            assert 8 * n[0] + 4 * n[1] + n[2] == c.N
-            assert (n[0] > 0) == tiles, n
+        n = s.gather_counts()
+        assert 8 * n[0] + 4 * n[1] + n[2] == c.N
+        assert transport != 3 or (n[0] > 0) == tiles, n
         s.cudaStep(2)
         out.append(s.cudaDownloadFull())
         s.close()
-    np.testing.assert_array_equal(out[0][0], out[1][0])
-    np.testing.assert_array_equal(out[0][1], out[1][1])
+    for g, m in out[1:]:
+        np.testing.assert_array_equal(g, out[0][0])
+        np.testing.assert_array_equal(m, out[0][1])
 
 
 @pytest.mark.parametrize("precision", [32, 64])
