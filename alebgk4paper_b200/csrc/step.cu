@@ -15,8 +15,7 @@
 //   k_scale_mood      sigma on the macros, moodCheck
 //   k_recollide       second collision when moodCheck failed (else exits)
 //   k_mass_end        end-of-step mass after a second collision (else exits)
-// In a step graph k_fixup runs in k_sigma's last block (k_sigma_fix) and
-// k_mass_end in k_recollide's (k_late).
+// In a step graph k_mass_end runs in k_recollide's last block (k_late).
 // k_batch_* run the same stage bodies for a batch of clouds, one launch per
 // stage over all of them (a block finds its cloud from block offsets).
 // The stored state h is the true distribution divided by StepScalars::scale.
@@ -1813,20 +1812,18 @@ k_sigma(const double *__restrict__ massPos, int N, double *partial, StepScalars 
 
 // Mass at the end of the step (the next step's massOld); the stored state
 // now carries the scale sigma.
-__device__ __forceinline__ void endStepMass(StepScalars *sc, double m)
-{
-    const double sigma = sc->sigma;
-    sc->massEnd = sigma * m;
-    sc->massOld = sc->massEnd;
-    sc->scale = sigma;
-    sc->steps += 1;
-}
-
 __global__ void __launch_bounds__(kRedThreads)
 k_mass_sum(const double *__restrict__ massEnd, int N, double *partial, StepScalars *sc)
 {
     double m;
-    if (gridSumLast(massEnd, N, partial, sc, &m)) endStepMass(sc, m);
+    if (gridSumLast(massEnd, N, partial, sc, &m))
+    {
+        const double sigma = sc->sigma;
+        sc->massEnd = sigma * m;
+        sc->massOld = sc->massEnd;
+        sc->scale = sigma;
+        sc->steps += 1;
+    }
 }
 
 // Applies sigma to the macros and runs moodCheck (Conservation.cpp:16-38,
@@ -1948,52 +1945,17 @@ k_mass_end(const double *__restrict__ massEnd, int N, double *partial, StepScala
 }
 
 // ---------------------------------------------------------------------------
-// The rare-path launches of a step graph, merged.  A step ends in a chain of
-// short kernels that cost their launch (about 2 us each, beside sums of a few
-// arrays of N values): k_fixup and k_mass_end find nothing to do in nearly
-// every step, so their work goes to the last block of the kernel before them
-// (a ticket, as in gridSumLast).  Same operations and orders, same bits.
-//   k_sigma_fix   k_sigma, then k_fixup by its last block when few rows are
-//                 listed
-//   k_fix_mass    k_mass_sum; when more are, k_fixup over the whole grid
-//                 before it, and the sum by the last block
-//   k_late        k_recollide, then k_mass_end by its last block
-// (With tau(rho, T) every row is listed and k_fixup keeps its own launch.)
-// Measured, a step alone: cavity2d Nx 20 Nv 16 FP64 50.6 -> 49.2 us, cavity3d
-// Nx 27 Nv 12 FP32 778 -> 771 us for two.  Merging the whole chain into the
-// redo's last block was slower: 296 blocks' fences in every step, and sums on
-// one SM (96 cavities: 18.9 ms a 10 steps against 16.2).
+// The second collision with the end mass, in a step graph.  A step ends in a chain
+// of short kernels that cost their launch (about 2 us each), and k_mass_end finds
+// nothing to do in nearly every step: its sum goes to the last block of
+// k_recollide (a ticket, as in gridSumLast).  Same operations and orders, same
+// bits.  Measured, steps of cavity2d Nx 20 Nv 16 FP64 one after the other 13.6 ->
+// 13.0 us, a step alone 42 -> 40.  The other merges were slower: k_fixup in the last block of k_sigma and,
+// for more than a few rows, in the grid of k_mass_sum (cavity2d Nx 37 Nv 18 FP32
+// 16.0 -> 17.1 us, 96 cavities 16.1 -> 17.2 ms a 10 steps; all rows by one block,
+// 158 ms a step of an empty cavity3d Nx 40 Nv 10 for 1.2), and the whole chain in
+// the redo's last block (296 blocks' fences in every step, and sums on one SM).
 // ---------------------------------------------------------------------------
-// Rows that k_sigma_fix's last block takes: one round of its warps, as long as
-// k_fixup itself would take.  More go over the grid: a step of an empty cavity3d
-// Nx 40 Nv 10 (54 872 rows) takes 158 ms by one block, 1.2 this way.
-constexpr int kFixupRows = kNT / 32;
-
-template <typename T>
-__device__ __noinline__ void lateFixup(const ParticleArgs<T> &a, const StepParams &p)
-{
-    k_fixup_body<T>(a, p, 0, 1);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kRedThreads)
-k_sigma_fix(ParticleArgs<T> a, StepParams p, double *partial)
-{
-    static_assert(kRedThreads == kNT, "one block size");
-    __shared__ bool mine;
-    StepScalars *sc = a.sc;
-    double m = 0.0;
-    if (threadIdx.x == 0) mine = false;
-    if (gridSumLast(a.massPos, p.N, partial, sc, &m))
-    {
-        sc->massNew = m;
-        sc->sigma = (m > 1.0e-30) ? sc->massOld / m : 1.0;
-        mine = sc->ndeg > 0 && sc->ndeg <= kFixupRows;
-    }
-    __syncthreads();
-    if (mine) lateFixup<T>(a, p);
-}
-
 // The sum of a[0..N) by one block, in the order of gridSumLast over kRedBlocks
 // blocks.  A warp stands in for every eighth of them, its lanes for those of
 // all the block's warps at once, so that their loads overlap.  Complete in
@@ -2031,43 +1993,6 @@ __device__ __noinline__ double blockGridSum(const double *a, int N, double *sh)
     return total;
 }
 
-// Ticket of a grid whose blocks have done their part: true in every thread of
-// the last one, which sees what the others wrote (and sets redCount back).
-__device__ bool lastBlock(StepScalars *sc)
-{
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        last = atomicAdd(&sc->redCount, 1u) == gridDim.x - 1;
-        __threadfence();
-        if (last) sc->redCount = 0;
-    }
-    __syncthreads();
-    return last;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kRedThreads)
-k_fix_mass(ParticleArgs<T> a, StepParams p, double *partial)
-{
-    StepScalars *sc = a.sc;
-    double m;
-    if (sc->ndeg <= kFixupRows)
-    {
-        if (blockIdx.x < kRedBlocks &&
-            gridSumLast(a.massEnd, p.N, partial, sc, &m, blockIdx.x, kRedBlocks))
-            endStepMass(sc, m);
-        return;
-    }
-    __shared__ double sh[kRedBlocks];
-    k_fixup_body<T>(a, p, blockIdx.x, gridDim.x);
-    if (!lastBlock(sc)) return;
-    m = blockGridSum(a.massEnd, p.N, sh);
-    if (threadIdx.x == 0) endStepMass(sc, m);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kNT, 3)
 k_late(T *__restrict__ g, StepParams p, const int *__restrict__ boundary,
@@ -2076,11 +2001,21 @@ k_late(T *__restrict__ g, StepParams p, const int *__restrict__ boundary,
     static_assert(kRedThreads == kNT, "one block size");
     if (sc->moodfail == 0) return;
     __shared__ double sh[kRedBlocks];
+    __shared__ bool last;
     k_recollide_body(g, p, boundary, macNew, massEnd, sc, blockIdx.x, gridDim.x);
-    if (!lastBlock(sc)) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        last = atomicAdd(&sc->redCount, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
     const double m = blockGridSum(massEnd, p.N, sh);
     if (threadIdx.x == 0)
     {
+        sc->redCount = 0;
         sc->massEnd = sc->sigma * m;
         sc->massOld = sc->massEnd;
     }
@@ -2648,21 +2583,11 @@ static cudaError_t stepT(alebgk_ctx *c, int from, cudaEvent_t *ev, bool alone)
     else k_redo<T, 1><<<listBlocks, kNT, rowBytes, st>>>(pa, p);
     mark();
     const bool merged = !ev;      // (timed stages need launches of their own)
-    const bool mergedFix = merged && !p.tauVar;
-    if (mergedFix)
-        k_sigma_fix<T><<<kRedBlocks, kRedThreads, 0, st>>>(pa, p, d.redPartial);
-    else
-    {
-        k_sigma<<<kRedBlocks, kRedThreads, 0, st>>>(d.massPos, p.N, d.redPartial, d.sc);
-        mark();
-        k_fixup<T><<<min(pBlocks, 296), kNT, 0, st>>>(pa, p);
-    }
+    k_sigma<<<kRedBlocks, kRedThreads, 0, st>>>(d.massPos, p.N, d.redPartial, d.sc);
     mark();
-    if (mergedFix)
-        k_fix_mass<T><<<max(kRedBlocks, min(pBlocks, 296)), kRedThreads, 0, st>>>(pa, p,
-                                                                                  d.redPartial);
-    else
-        k_mass_sum<<<kRedBlocks, kRedThreads, 0, st>>>(d.massEnd, p.N, d.redPartial, d.sc);
+    k_fixup<T><<<min(pBlocks, 296), kNT, 0, st>>>(pa, p);
+    mark();
+    k_mass_sum<<<kRedBlocks, kRedThreads, 0, st>>>(d.massEnd, p.N, d.redPartial, d.sc);
     mark();
     k_scale_mood<<<(p.N + 255) / 256, 256, 0, st>>>(p, d.boundary, macB, d.minG, d.mood, d.sc);
     mark();

@@ -419,9 +419,9 @@ def run_ours(args):
                          "ping-pong, no flush needed"},
         # per step in the step graph: k_step_begin twice (the one-block
         # scalar reset, then the NAD ranges on the side stream beside the
-        # transport), then transport, particle, redo, sigma (with the fixup),
-        # mass_sum, scale_mood, late (recollide with the end mass)
-        "gpu_launches": 9 * args.steps,
+        # transport), then transport, particle, redo, sigma, fixup, mass_sum,
+        # scale_mood, late (recollide with the end mass)
+        "gpu_launches": 10 * args.steps,
         "kernels": kernels,
         "stage_ms": {k: round(v, 5) for k, v in stage_ms.items()},
         "roofline": {"bound": "hbm", "kernel": kern_name, "achieved": achieved,

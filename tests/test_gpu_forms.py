@@ -249,7 +249,8 @@ def test_row_forms_repair_negative_rows_like_the_oracle(gpu, Nx, Nv, precision, 
 @pytest.mark.parametrize("name,Nx,Nv", [("cavity2d", 9, 6), ("cavity2d", 64, 6), ("cavity2d", 65, 6),
                                         ("cavity3d", 16, 4), ("cavity3d", 17, 4), ("cavity3d", 27, 4)])
 def test_merged_end_of_step_equals_separate_launches(gpu, name, Nx, Nv, precision):
-    """Up to 4 096 particles and above: bitwise the chain of single kernels (timed steps)."""
+    """Clouds of a few blocks and of many: bitwise the chain of single kernels (timed steps).  (What the merged kernels
+    do when they have rows to finish is in the two tests below.)"""
     c = ab.Case(name, Nx, Nv, -1.0, 2)
     a, b = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision)
     if name == "cavity2d":
@@ -288,8 +289,8 @@ def _merged_and_separate_steps(c, precision, limiter, steps):
 @pytest.mark.parametrize("name,Nx,Nv,radius", [("cavity2d", 16, 8, 1.5), ("cavity2d", 16, 8, 99.0),
                                                ("cavity3d", 12, 6, 2.1), ("cavity3d", 12, 6, 5.0)])
 def test_merged_end_of_step_finishes_rows_without_mass(gpu, name, Nx, Nv, radius, limiter, precision):
-    """A ball of empty rows, of which one to eight rows come out of the first transport without positive mass (the mass
-    sum's last block finishes them), or more (the whole grid does): like the single kernels, and like the oracle."""
+    """A ball of empty rows, of which a few or many come out of the first transport without positive mass: finished like
+    by the single kernels, and like by the oracle."""
     from oracle.oracle import Oracle
     from test_mls_tables import _tables
     c = ab.Case(name, Nx, Nv, -1.0, 2)
