@@ -2,15 +2,12 @@
 //
 // Same quantity as alebgk_body_loads (computeBodyLoads,
 // RigidBody/BodyDynamics.cpp:17-97): per body the force and torque of the
-// surface stress -(P . n) dA summed over the body's wall particles.  The
-// allocating entry point stages the body geometry in a cudaMalloc'd buffer and
-// frees it after every call; cudaFree synchronises the whole device, so a
-// caller that advances several cavities on separate streams of one device
-// would stall all of them on every load query, and a caller that has reserved
-// the device memory for its own pools may see the allocation fail mid-run.
-// This variant allocates nothing: the body geometry travels as a by-value
+// surface stress -(P . n) dA summed over the body's wall particles.
+// alebgk_body_loads takes the context's body staging and waits for its stream;
+// this variant needs no staging: the body geometry travels as a by-value
 // kernel argument, and the per-block partial sums and the result live in one
-// file-scope device array of fixed size.
+// file-scope device array of fixed size.  (Made when alebgk_body_loads
+// allocated and freed on every call, which stalled the device's other streams.)
 //
 // The scratch is one per device and shared by every context on that device:
 // calls that overlap in time on the same device race on it and must be

@@ -61,8 +61,9 @@ __device__ __forceinline__ void basisOf(double sx, double sy, double sz, double 
 }
 
 // One (class, node): the coefficients of its slots into cc, with the basis
-// size fixed at compile time so that the normal matrix lives in registers
-// from its first term to the last back substitution.  The elimination
+// size fixed at compile time so that the normal matrix needs no indexed memory
+// from its first term to the last back substitution (registers; of the
+// quadratic 3-D one the compiler spills 372 bytes).  The elimination
 // (partial pivots, |pivot| < 1e-30 skipped, as solveSkipGE) keeps its
 // multipliers below the diagonal and its pivot rows in one word; the unit
 // right-hand sides, of which only the first unknown is needed, then go
@@ -218,8 +219,9 @@ __device__ __forceinline__ void classNode(const ClassArgs &a, int c, int n, doub
 // Per class: rep position (3), mesh velocity (3), wall state (7), then the
 // positions of slots 1..nsl-1 (3 each) at [c][S][3].  A block is of one
 // class (grid y and z), so its threads take one basis size.
-// Bound: FP64 issue (about 280 operations a slot in the support and 4 000 for
-// the elimination, uncontracted).  Measured, cavity3d-cube Nx 40 Nv 10
+// Bound: the chain of dependent FP64 operations of a node (about 280 a slot in
+// the support and 4 000 for the elimination, uncontracted) at two warps a
+// scheduler: the FP64 pipe is busy 39 % of the cycles.  Measured, cavity3d-cube Nx 40 Nv 10
 // (1 099 classes x 1 000 nodes, FP32 tables): quadratic 14.2 ms with both
 // matrices in local memory, read and written for every slot; 3.1 ms in
 // registers (255, two blocks an SM).  Linear 1.92 -> 1.87 ms.

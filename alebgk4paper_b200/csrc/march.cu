@@ -27,8 +27,9 @@
 // fma.rn.f32x2 is one fmaf), so both widths give the same bits.
 //
 // FP64 takes the kernel at one velocity a lane, in the registers and shared
-// memory of the two-velocity FP32 form: its bound is the FP64 pipe (4.8e9
-// FMAs at cavity3d Nx 40 Nv 10, 0.26 ms at 64 lanes an SM; HBM 0.16 ms).
+// memory of the two-velocity FP32 form: its floor is the FP64 pipe (4.8e9
+// FMAs at cavity3d Nx 40 Nv 10, 0.26 ms at 64 lanes an SM; HBM 0.16 ms), which
+// two warps a scheduler keep busy for 54 % of the cycles.
 // Measured there: 2.58 ms by the coefficient gather (L1-bound, a coefficient
 // and a value loaded per FMA), 0.685 ms marched.
 #include <cuda.h>

@@ -11,8 +11,9 @@
 //      distribution, and the macros by linearity (k_particle_stream).
 // The group shares the chain of barriers, divisions and exponentials that a
 // row needs between its two passes, which is what a warp or a block per row
-// waits for; the rest is about seven FP64-pipe operations a value beside the
-// HBM traffic of the row in and out.
+// waits for; the rest is about seven FP64-pipe operations a value, with their
+// conversions and indices (issue slots 76 % busy, the FP64 pipe 28 %), beside
+// the HBM traffic of the row in and out.
 // All arithmetic is FP64, as in the general kernel.
 // Measured, particle stage: cavity3d Nx 24 Nv 16 FP32 688 us by the general
 // kernel (a warp per row, its copy read and written in every pass), 240 us

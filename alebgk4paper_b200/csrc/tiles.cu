@@ -23,7 +23,8 @@
 // Measured, cavity3d-cube Nx 40 Nv 10 FP32: transport 1.53 ms by the gather
 // alone; 0.756 ms with tiles (0.307 for 70 % of the particles, 0.456 for the
 // gather of the rest).  The strips take the step there from 985 to 909 us, the
-// pairs of nodes in the gather of the rest to 877.
+// pairs of nodes in the gather of the rest to 877.  Tiles and rest run at 69 and
+// 75 % of L1's throughput.  (Which clouds take them: tilesPay in step.cu.)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -163,11 +164,11 @@ __global__ void k_tile_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__r
     if (ok && lane < 8) covered[lane >> 2 ? j + (lane & 3) : i + (lane & 3)] = 1;
 }
 
-// The same for strips, of the particles that no tile covers (covered is 1 for
-// those; strips write 2 for their own members, which no other strip has, by
-// their columns).  first[c] is -1
-// for a class without the strips' form, else the class's row of rowFirst: per
-// template row the slot of its first offset, -1 where the row is missing.
+// The same for strips, of the particles that no tile covers (a tile's have 1 in
+// covered; strips write 2 for their own members, which no other strip has, by
+// their columns).  first[c] is -1 for a class without the strips' form, else
+// the class's row of rowFirst: per template row the slot of its first offset,
+// -1 where the row is missing.
 __global__ void k_strip_mark(Tmpl3 t, TileGrid g, int N, int S, const double *__restrict__ pos,
                              const int *__restrict__ cls, const int *__restrict__ nslot,
                              const int *__restrict__ slots, const int *__restrict__ first,

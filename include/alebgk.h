@@ -233,11 +233,9 @@ int alebgk_body_loads(alebgk_ctx *ctx, int nbodies, const double *body_centre,
                       const double *body_area, double *out);
 
 /* The loads of alebgk_body_loads without any device allocation.  No
- * counterpart in the reference.  For callers that must not allocate: one
- * that advances several cavities on separate streams of a device (the
- * cudaFree of the allocating call synchronises the whole device and stalls
- * every other stream), and one that has reserved the device memory for its
- * own pools (an allocation could fail mid-run).  Sums run per block and then
+ * counterpart in the reference.  For callers that must not allocate (made
+ * when alebgk_body_loads did, on every call; it now uses the context's body
+ * staging).  Sums run per block and then
  * over blocks, so results match alebgk_body_loads to rounding, not bitwise.
  * Limits: 1..ALEBGK_NOALLOC_MAX_BODIES bodies; larger counts return
  * ALEBGK_EINVAL.  Scratch: one fixed 114,432-byte device array per device,
