@@ -636,6 +636,10 @@ class Solver:
         """Velocities per lane of the lattice march (2: packed FMAs, or 1)."""
         _check(self.lib.alebgk_set_march_width(self.ctx, int(velocities_per_lane)), self.ctx)
 
+    def set_gather_tiles(self, always: bool):
+        """The gather's tiles and strips wherever the cloud has any, or (default) where they are faster."""
+        _check(self.lib.alebgk_set_gather_tiles(self.ctx, int(bool(always))), self.ctx)
+
     def set_residual_speed(self, speed: float):
         """Speed scale of the residual's momentum terms (0: thermal speed)."""
         _check(self.lib.alebgk_set_residual_speed(self.ctx, float(speed)), self.ctx)

@@ -96,6 +96,7 @@ SIGNATURES = {
     "alebgk_coeff_free": (None, [ctypes.c_void_p]),
     "alebgk_get_counters": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Counters)]),
     "alebgk_gather_counts": (ctypes.c_int, [ctypes.c_void_p, c_int_p]),
+    "alebgk_set_gather_tiles": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "alebgk_total_mass": (ctypes.c_int, [ctypes.c_void_p, c_double_p]),
     "alebgk_wall_momentum": (ctypes.c_int, [ctypes.c_void_p, c_double_p]),
     "alebgk_device_state": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p),

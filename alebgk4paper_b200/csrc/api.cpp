@@ -158,8 +158,8 @@ int alebgk_create(const alebgk_config *cfg, alebgk_ctx **out)
         return fail(nullptr, ALEBGK_EINVAL, "mls_order must be 1 or 2");
     if (cfg->limiter != 0 && cfg->limiter != 2)
         return fail(nullptr, ALEBGK_EINVAL, "limiter must be 0 (none) or 2 (MOOD)");
-    if (cfg->transport < 0 || cfg->transport > 3)
-        return fail(nullptr, ALEBGK_EINVAL, "the transport selector is 0, 1, 2 or 3");
+    if (cfg->transport < 0 || cfg->transport > 2)
+        return fail(nullptr, ALEBGK_EINVAL, "the transport selector is 0, 1 or 2");
     if (cfg->particle < 0 || cfg->particle > 3)
         return fail(nullptr, ALEBGK_EINVAL, "the particle selector is 0, 1, 2 or 3");
     if (!(cfg->tau > 0) || !(cfg->R > 0) || !(cfg->dv > 0) || !(cfg->radius > 0))
@@ -262,7 +262,7 @@ static int setupMarch(alebgk_ctx *c, const alebgk_cloud *cl, const CoeffTables &
     std::string err;
     bool anyBody = false;
     for (int i = 0; i < N && !anyBody; ++i) anyBody = cl->body_id[i] >= 0;
-    if ((c->cfg.transport == 0 || c->cfg.transport == 2) && !anyBody)
+    if (c->cfg.transport != 1 && !anyBody)
     {
         MarchPlan plan;
         buildMarchPlan(cl->xyz, N, p.dim, cl->nnb, cl->nbr, ALEBGK_MAX_NEIGH, tb, plan);
@@ -319,8 +319,8 @@ static int setupTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb
     DeviceBuffers &d = c->d;
     const size_t N = c->sp.N;
     c->tiled = false;
-    if (c->sp.dim != 3 || c->march.enabled || (c->cfg.transport != 0 && c->cfg.transport != 3))
-        return ALEBGK_OK;
+    c->gatherTiles = c->gatherStrips = 0;
+    if (c->sp.dim != 3 || c->march.enabled || c->cfg.transport != 0) return ALEBGK_OK;
     if (!d.tiles)
     {
         CK(dalloc(&d.tiles, tileInts((int)N)));
@@ -334,7 +334,9 @@ static int setupTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb
     CK(buildTiles(c, in, tb));
     int n[3];
     CK(cudaMemcpy(n, d.tileCount, sizeof n, cudaMemcpyDeviceToHost));
-    c->tiled = c->cfg.transport == 3 ? n[0] + n[1] > 0 : tilesPay(c, n[0], n[1]);
+    c->gatherTiles = n[0];
+    c->gatherStrips = n[1];
+    c->tiled = takeTiles(c);
     return ALEBGK_OK;
 }
 
@@ -1119,9 +1121,10 @@ int alebgk_gather_counts(alebgk_ctx *c, int *counts)
     counts[0] = counts[1] = 0;
     counts[2] = c->sp.N;
     if (!c->tiled) return ALEBGK_OK;
+    int n[3];
     CK(cudaSetDevice(c->cfg.device));
-    CK(cudaMemcpyAsync(counts, c->d.tileCount, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    CK(cudaMemcpy(n, c->d.tileCount, sizeof n, cudaMemcpyDeviceToHost));
+    for (int q = 0; q < 3; ++q) counts[q] = n[q];
     return ALEBGK_OK;
 }
 

@@ -172,6 +172,18 @@ int alebgk_set_march_width(alebgk_ctx *c, int velocities_per_lane)
     return ALEBGK_OK;
 }
 
+int alebgk_set_gather_tiles(alebgk_ctx *c, int always)
+{
+    if (!c) return ALEBGK_EINVAL;
+    if (always != 0 && always != 1)
+        return failc(c, ALEBGK_EINVAL, "gather tiles: 0 (where they are faster) or 1 (always)");
+    c->tune.allTiles = always != 0;
+    const bool before = c->tiled;
+    if (c->uploaded) c->tiled = takeTiles(c);
+    if (c->tiled != before) dropGraphs(c);
+    return ALEBGK_OK;
+}
+
 int alebgk_set_nad_floor(alebgk_ctx *c, double rel)
 {
     if (!c) return ALEBGK_EINVAL;

@@ -140,6 +140,7 @@ struct alebgk_ctx
     int ncls = 0;
     int sms = 0;                 // multiprocessors of the device
     int gatherWave = 0;          // blocks of k_transport that the device holds at once
+    int gatherTiles = 0, gatherStrips = 0;   // of the cloud's plan (tiles.cu)
     bool tiled = false;          // the gather transport runs by tiles (tiles.cu)
     int degenerateParticles = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -149,6 +150,7 @@ struct alebgk_ctx
         int transportThreads = 0;     // coefficient-gather transport per block; 0 fused
         int particleWarps = 0;        // warp-per-particle kernel; 0 = as many as fit
         int marchVpl = 2;             // lattice march: velocities per lane (1 or 2)
+        bool allTiles = false;        // the gather's tiles wherever there are any
     } tune;
     // Streamed particle kernel: on, warps per block, blocks, dynamic smem.
     bool pStream = false;
@@ -201,8 +203,9 @@ cudaError_t buildTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &t
 size_t tileInts(int N);
 size_t stripInts(int N);
 cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st);
-// Whether a plan of so many tiles and strips is faster than the plain gather (step.cu).
-bool tilesPay(const alebgk_ctx *c, int tiles, int strips);
+// Whether the context takes its plan's tiles and strips: where they are faster
+// than the plain gather, or wherever there are any when asked for (step.cu).
+bool takeTiles(const alebgk_ctx *c);
 
 // Launch wrappers (step.cu).
 cudaError_t prepareKernels(alebgk_ctx *c);

@@ -2468,11 +2468,12 @@ static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
 // blocks) 80 and 89 us, 164 and 184; Nx 16 Nv 8 (1 046) 147 and 133, 244 and 211;
 // Nx 8 Nv 16 (1 204, of them 224 in strips) 178 and 186, 328 and 329; Nx 12 Nv 10
 // (908, 396 in tiles and strips) 147 and 139, 255 and 217.
-bool tilesPay(const alebgk_ctx *c, int tiles, int strips)
+bool takeTiles(const alebgk_ctx *c)
 {
     const long long nch = transportChunks(c->sp.V), per = kNT / 32;
-    return nch * (c->sp.N / per) > c->gatherWave &&
-           2 * nch * ((8LL * tiles + 4LL * strips) / per) > c->gatherWave;
+    const long long members = 8LL * c->gatherTiles + 4LL * c->gatherStrips;
+    if (c->tune.allTiles) return members > 0;
+    return nch * (c->sp.N / per) > c->gatherWave && 2 * nch * (members / per) > c->gatherWave;
 }
 
 // The small 2-D form where one wave holds the whole cloud, else none; sw = its

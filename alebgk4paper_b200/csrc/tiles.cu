@@ -24,7 +24,7 @@
 // alone; 0.756 ms with tiles (0.307 for 70 % of the particles, 0.456 for the
 // gather of the rest).  The strips take the step there from 985 to 909 us, the
 // pairs of nodes in the gather of the rest to 877.  Tiles and rest run at 69 and
-// 75 % of L1's throughput.  (Which clouds take them: tilesPay in step.cu.)
+// 75 % of L1's throughput.  (Which clouds take them: takeTiles in step.cu.)
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -67,8 +67,7 @@ typedef struct alebgk_config
     int transport;    /* 0 auto (lattice march when the cloud is a complete
                          lattice without bodies, else coefficient gather),
                          1 always the plain gather, 2 require the march (FP32
-                         only), 3 always gather, by tiles wherever a 3-D cloud
-                         has any (0 takes them where they are faster)         */
+                         only)                                                */
     int particle;     /* 0 auto (3-D: rows in registers where they fit, else
                          streamed rows or groups of rows in shared memory;
                          else one warp per particle), 1 always the general
@@ -207,6 +206,12 @@ int alebgk_get_counters(alebgk_ctx *ctx, alebgk_counters *out);
  * N.  A cloud that marches or is gathered plainly has {0, 0, N}.  No reference
  * counterpart. */
 int alebgk_gather_counts(alebgk_ctx *ctx, int *counts);
+
+/* Whether the coefficient gather of a transport-0 cloud takes its tiles and
+ * strips wherever there are any (always = 1), or where they are faster than
+ * the plain gather (0, the default).  Same bits.  Drops the captured step
+ * graphs.  No reference counterpart. */
+int alebgk_set_gather_tiles(alebgk_ctx *ctx, int always);
 
 /* Total gas mass sum(g dv^d) on the device.
  * Replaces cudaTotalMass (Solver/CudaBackend.cu:2018-2024). */

@@ -44,7 +44,8 @@ def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
     remainders, bodies in the middle: every particle sums its slots in the same order, so the states are
     the same bits."""
     c = ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True)
-    a, b = ab.Solver(c, precision=precision, transport=3), ab.Solver(c, precision=precision, transport=1)
+    a, b = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision, transport=1)
+    a.set_gather_tiles(True)
     assert min(a.gather_counts()) > 0 and b.gather_counts() == (0, 0, c.N)
     a.cudaStep(3), b.cudaStep(3)
     (ga, ma), (gb, mb) = a.cudaDownloadFull(), b.cudaDownloadFull()
@@ -56,11 +57,17 @@ def test_gather_by_tiles_equals_plain_gather(gpu, name, Nx, Nv, precision):
 @pytest.mark.parametrize("name,Nx,Nv,tiled", [("cavity3d-cube", 12, 6, False), ("cavity3d-cube", 8, 16, False),
                                               ("cavity3d-cube", 24, 6, True), ("cavity3d-sphere", 24, 4, True)])
 def test_tiles_are_taken_where_they_pay(gpu, name, Nx, Nv, tiled, precision):
-    """Not where one wave of the plain gather holds the cloud, or few particles are in tiles and strips; a cloud that
-    grows or shrinks past the line would change its graphs with it."""
-    s = ab.Solver(ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True), precision=precision)
+    """Not where one wave of the plain gather holds the cloud, or few particles are in tiles and strips.  Asked for
+    between steps, the same bits."""
+    c = ab.Case(name, Nx, Nv, -1.0, 2, fixed_body=True)
+    s, p = ab.Solver(c, precision=precision), ab.Solver(c, precision=precision, transport=1)
     assert (s.gather_counts()[0] > 0) == tiled
-    s.close()
+    for always in (False, True, False):
+        s.set_gather_tiles(always)
+        assert (sum(s.gather_counts()[:2]) > 0) == (tiled or always)
+        s.cudaStep(2), p.cudaStep(2)
+    np.testing.assert_array_equal(s.cudaDownloadFull()[0], p.cudaDownloadFull()[0])
+    s.close(), p.close()
 
 
 @pytest.mark.parametrize("precision", [32, 64])
@@ -71,10 +78,11 @@ def test_gather_by_tiles_equals_plain_gather_at_a_large_step(gpu, cells, precisi
     c = ab.Case("cavity3d-cube", 17, 6, -1.0, 2, fixed_body=True)
     c.dt = cells * c.params["dx"] / max(abs(c.params["vmin"]), c.params["vmin"] + (c.Nv - 1) * c.params["dv"])
     out = []
-    for transport in (3, 1):
+    for transport in (0, 1):
         cfg = c.config(precision, 0, transport)
         cfg.limiter = 0
         s = ab.Solver(c, config=cfg)
+        s.set_gather_tiles(True)
         assert transport == 1 or s.gather_counts()[0] > 0
         s.cudaStep(1)
         out.append(s.cudaDownloadFull())
@@ -126,15 +134,16 @@ def _own_cloud(xyz, h, Nv, wall_first=False, box=(0, 0, 0), reach=2.5):
 
 def _assert_auto_equals_plain(c, precision, box=(0, 0, 0), tiles=True):
     out = []
-    for transport in (0, 3, 1):
+    for transport, always in ((0, False), (0, True), (1, True)):
         cfg = c.config(precision, 0, transport)
         for a in range(3):
             cfg.periodic[a], cfg.L[a] = int(box[a] > 0), box[a]
         s = ab.Solver(c, config=cfg)
         assert s.counters()["transport_kernel"] == 1
+        s.set_gather_tiles(always)
         n = s.gather_counts()
         assert 8 * n[0] + 4 * n[1] + n[2] == c.N
-        assert transport != 3 or (n[0] > 0) == tiles, n
+        assert not always or (n[0] > 0) == (tiles and transport == 0), n
         s.cudaStep(2)
         out.append(s.cudaDownloadFull())
         s.close()
