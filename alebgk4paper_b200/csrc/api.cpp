@@ -246,8 +246,34 @@ int alebgk_last_error(const alebgk_ctx *c, char *buf, size_t len)
     return ALEBGK_OK;
 }
 
-// The geometry part of alebgk_upload (tables, march plan, buffers); with
-// withState also the state (g and macros) from the cloud.
+// Whether an FP64 lattice marches or is gathered, by the time of either.  The
+// march has one block an SM: a unit and chunk costs its block's start (7.2 us
+// over the SMs) and 0.7 us a plane.  A wave of the gather's blocks takes about 60
+// us, the first 40 at least; 68 and 55 are allowed, so that a lattice near the
+// line marches.  Small lattices with long rows are the gather's: they have few
+// columns a unit and a unit for every wall layer.  Measured, a step marched and
+// gathered: Nx 8 Nv 10 95 and 67 us, Nx 9 Nv 10 163 and 90, Nx 10 Nv 10 97 and 80,
+// Nx 10 Nv 12 150 and 137 (by tiles); Nx 8 Nv 6 47 and 60, Nx 12 Nv 10 119 and 133,
+// Nx 12 Nv 14 267 and 277, Nx 14 Nv 8 80 and 97.  Near the line: Nx 9 Nv 8, 80 and
+// 70, and Nx 13 Nv 10, 146 and 139, march.  FP32 lattices always march, as they
+// did before FP64 ones could.
+static bool marchPays(const alebgk_ctx *c, const MarchPlan &plan)
+{
+    if (c->cfg.precision != 64) return true;
+    long long planes = 0;
+    for (const std::vector<MarchUnit> *us : {&plan.units, &plan.unitsY})
+        for (const MarchUnit &u : *us)
+        {
+            const int len = u.yMarch ? plan.Ny : plan.Nz;
+            planes += u.zb - u.za > 4 ? u.zb - u.za + 4
+                                      : std::min(u.zb + 1, len - 1) - std::max(u.za - 2, 0) + 1;
+        }
+    const double chunks = (c->sp.V + kMarchChunk - 1) / kMarchChunk;
+    const double march =
+        chunks / c->sms * (7.2 * (plan.units.size() + plan.unitsY.size()) + 0.7 * planes);
+    return march <= std::max(55.0, 68.0 * gatherBlocks(c) / c->gatherWave);
+}
+
 // Sets up the lattice march where it applies (a complete 3-D lattice without
 // bodies): its plan, and its coefficient table laid out from the class table
 // that is already on the device.
@@ -266,7 +292,7 @@ static int setupMarch(alebgk_ctx *c, const alebgk_cloud *cl, const CoeffTables &
     {
         MarchPlan plan;
         buildMarchPlan(cl->xyz, N, p.dim, cl->nnb, cl->nbr, ALEBGK_MAX_NEIGH, tb, plan);
-        if (plan.ok)
+        if (plan.ok && marchPays(c, plan))
         {
             MarchState &m = c->march;
             m.f64 = f64;
@@ -340,6 +366,8 @@ static int setupTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &tb
     return ALEBGK_OK;
 }
 
+// The geometry part of alebgk_upload (tables, march plan, buffers); with
+// withState also the state (g and macros) from the cloud.
 static int uploadCloud(alebgk_ctx *c, const alebgk_cloud *cl, double dt, bool withState)
 {
     if (!c || !cl) return fail(c, ALEBGK_EINVAL, "null argument");

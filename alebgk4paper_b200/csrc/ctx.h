@@ -203,6 +203,8 @@ cudaError_t buildTiles(alebgk_ctx *c, const CoeffInput &in, const CoeffTables &t
 size_t tileInts(int N);
 size_t stripInts(int N);
 cudaError_t launchTiles(alebgk_ctx *c, const void *f, void *g, cudaStream_t st);
+// Blocks of the plain gather over the whole cloud (step.cu).
+long long gatherBlocks(const alebgk_ctx *c);
 // Whether the context takes its plan's tiles and strips: where they are faster
 // than the plain gather, or wherever there are any when asked for (step.cu).
 bool takeTiles(const alebgk_ctx *c);

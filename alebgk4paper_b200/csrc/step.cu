@@ -2460,6 +2460,11 @@ static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
     return cudaGetLastError();
 }
 
+long long gatherBlocks(const alebgk_ctx *c)
+{
+    return (long long)transportChunks(c->sp.V) * (c->sp.N / (kNT / 32));
+}
+
 // Tiles and strips are launches of their own before the gather of the rest, each
 // at least as long as one wave of blocks.  So they pay where the plain gather
 // takes more than a wave, and they take at least half a wave off it.  Measured,
@@ -2470,10 +2475,10 @@ static cudaError_t launchGather(alebgk_ctx *c, int from, cudaStream_t st)
 // (908, 396 in tiles and strips) 147 and 139, 255 and 217.
 bool takeTiles(const alebgk_ctx *c)
 {
-    const long long nch = transportChunks(c->sp.V), per = kNT / 32;
     const long long members = 8LL * c->gatherTiles + 4LL * c->gatherStrips;
     if (c->tune.allTiles) return members > 0;
-    return nch * (c->sp.N / per) > c->gatherWave && 2 * nch * (members / per) > c->gatherWave;
+    return gatherBlocks(c) > c->gatherWave &&
+           2 * transportChunks(c->sp.V) * (members / (kNT / 32)) > c->gatherWave;
 }
 
 // The small 2-D form where one wave holds the whole cloud, else none; sw = its

@@ -65,7 +65,8 @@ typedef struct alebgk_config
     int periodic[3];  /* per-axis periodicity (minimum-image stencils)        */
     double L[3];      /* periodic lengths                                     */
     int transport;    /* 0 auto (lattice march when the cloud is a complete
-                         lattice without bodies, else coefficient gather),
+                         lattice without bodies, in FP64 where it is faster;
+                         else coefficient gather),
                          1 always the plain gather, 2 require the march (FP32
                          only)                                                */
     int particle;     /* 0 auto (3-D: rows in registers where they fit, else

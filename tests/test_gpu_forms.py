@@ -28,6 +28,21 @@ def test_fp64_march_equals_gather(gpu, Nx, Nv):
     assert _rel(ma[:, 0], mb[:, 0]) < 3 * 5 * 9 * 1.2e-16
 
 
+@pytest.mark.parametrize("Nx,Nv,marches", [(6, 8, True), (8, 10, False), (9, 12, False), (10, 12, False), (11, 12, True),
+                                           (12, 10, True), (14, 8, True)])
+def test_fp64_lattices_march_where_it_is_faster(gpu, Nx, Nv, marches):
+    """Small lattices with long rows are gathered (bitwise the plain gather); FP32 ones march as they always did."""
+    c = ab.Case("cavity3d", Nx, Nv, -1.0, 2)
+    s, f = ab.Solver(c, precision=64), ab.Solver(c, precision=32)
+    assert (s.counters()["transport_kernel"], f.counters()["transport_kernel"]) == (2 if marches else 1, 2)
+    if not marches:
+        p = ab.Solver(c, precision=64, transport=1)
+        s.cudaStep(3), p.cudaStep(3)
+        np.testing.assert_array_equal(s.cudaDownloadFull()[0], p.cudaDownloadFull()[0])
+        p.close()
+    s.close(), f.close()
+
+
 def test_required_march_is_refused_in_fp64(gpu):
     """Transport 2 is the FP32 march: an FP64 context is refused by what it asks for, a cloud that is no lattice by what
     it is."""
