@@ -250,7 +250,10 @@ def test_refresh_that_does_not_fit_the_memory_drops_the_cloud(gpu, name, transpo
     s.sync()
     still, c.meshv = c.meshv, 1e-3 * np.arange(3 * c.N).reshape(c.N, 3) / c.N
     torch.cuda.empty_cache()
-    hold = torch.empty(torch.cuda.mem_get_info()[0] - (left << 20), dtype=torch.uint8, device="cuda")
+    try:
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (left << 20), dtype=torch.uint8, device="cuda")
+    except torch.cuda.OutOfMemoryError:
+        pytest.skip("another process holds device memory")
     with pytest.raises(ab.AlebgkError):
         cl = c.cloud()
         ab._check(s.lib.alebgk_upload_geometry(s.ctx, ctypes.byref(cl), s.dt), s.ctx)
